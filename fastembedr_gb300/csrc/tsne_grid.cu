@@ -873,29 +873,29 @@ rows_inverse_kernel(const float2* __restrict__ arow, const float2* __restrict__ 
 // (add_sparse_attractive_gradient_f, src/tsne_neighbors.cpp:1061-1088).
 // Rows are taken in storage (spatial) order: slot_rows[s] = (begin, end) of the CSR row of the
 // point in slot s (rebuilt at every reorder), so a row is one contiguous segment of P and
-// consecutive rows of a warp belong to neighbouring points, whose neighbour sets overlap: their
-// y gathers hit L1. Warp w first takes chunk w of `chunk` consecutive slots, then further
-// chunks from a counter (the last warp to finish resets it for the next launch), which keeps
-// every SM busy to the end whatever the row lengths of a region. The chunk size and the number of
-// resident blocks are launch parameters chosen at run time by timing (tsne_tune_attractive): the
-// result does not depend on them. A row is read with 128-bit loads: lane l takes entries
-// c0 + 4 l .. + 3 of each 128-entry round (c0 = the row's first entry rounded down to a multiple
-// of 4; entries outside the row are masked), kAttrRounds rounds loaded before their gathers.
-// Lane 0 keeps a bulk L2 prefetch (cp.async.bulk.prefetch) of the row kAttrAhead rows ahead.
-// Each lane sums its entries in a fixed order, the rounds of a row longer than one group are
-// added with Kahan compensation, and the warp sum is a fixed butterfly: the force depends only
-// on the row and its entries' positions modulo 4, not on the schedule.
+// neighbouring slots belong to neighbouring points, whose neighbour sets overlap.
+//
+// What bounds the pass is the rate at which 32-byte sectors reach the SMs from L2: a y gather that
+// misses L1 costs a whole sector, and the SMs take about one sector per clock each (measured: 2.07
+// random 8-byte gathers per ns and SM from L2, 6.1 from L1). So the slots are divided into one
+// contiguous range of chunks per SM and every warp takes its chunks from the counter of the SM it
+// runs on (%smid): the gathers of an SM then stay within one neighbourhood of the layout, which its
+// L1 holds, where one counter for all SMs spread every neighbourhood over all of them. The stream
+// of columns and values bypasses L1. A warp whose SM has no chunk left takes chunks from the
+// SM with the most left, so uneven row lengths, or an SM shared with the grid stage, cost nothing.
+//
+// With three quarters of the gathers served by L1 the pass is bound by instruction issue (75 % of
+// the issue slots at 400,000 points), so the rest of the kernel is about instructions. A row is read
+// in rounds of 128 entries from c0, its first entry rounded down to a multiple of 4, with 128-bit
+// loads (lane l takes entries 4 l .. + 3); entries outside the row are masked only in the rounds that
+// can hold some. Two rows share one reduction, and the two rows after them are prefetched into L2
+// (cp.async.bulk.prefetch), a lane each. Each lane sums its entries in a fixed order, rounds are
+// added with Kahan compensation, and the warp sum is a fixed butterfly: the force depends only on
+// the row and its entries' positions modulo 4, not on the schedule. The chunk size and the number
+// of resident blocks are launch parameters chosen at run time by timing (tsne_tune_attractive); the
+// result does not depend on them.
 constexpr int kAttrThreads = 256;
 constexpr int kAttrWarps = kAttrThreads / 32;
-constexpr int kAttrAhead = 2;
-// Compile-time shape of the pass (measured alternatives in the attractive-pass variants profile):
-// 128-entry rounds loaded together (1: 40 registers) and the register cap that allows six
-// resident blocks per SM.
-#ifndef FE_ATTR_ROUNDS
-#define FE_ATTR_ROUNDS 1
-#endif
-constexpr int kAttrRounds = FE_ATTR_ROUNDS;
-
 __device__ __forceinline__ void prefetch_l2_range(const void* base, long long first, long long last, int elem) {
   // [first, last) elements of a 4-byte array, widened to 16-byte boundaries (the arena pads
   // every buffer to 256 bytes, so the widened range stays inside the allocation)
@@ -906,126 +906,226 @@ __device__ __forceinline__ void prefetch_l2_range(const void* base, long long fi
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a16), "r"((unsigned)(e16 - a16)) : "memory");
 }
 
-__device__ __forceinline__ int int4_at(const int4& v, int c) { return c == 0 ? v.x : c == 1 ? v.y : c == 2 ? v.z : v.w; }
-__device__ __forceinline__ float float4_at(const float4& v, int c) {
-  return c == 0 ? v.x : c == 1 ? v.y : c == 2 ? v.z : v.w;
+// Butterfly of the lane partials of two rows, (x0, y0) and (x1, y1): lanes 0-7 end with the warp's x0
+// sum, 8-15 with x1, 16-23 with y0, 24-31 with y1. A row's sum is the same in either place.
+__device__ __forceinline__ float butterfly_rows(float x0, float y0, float x1, float y1, int lane) {
+  const bool h16 = lane & 16, h8 = lane & 8;
+  float k0 = h16 ? y0 : x0, k1 = h16 ? y1 : x1;
+  k0 += __shfl_xor_sync(0xffffffffu, h16 ? x0 : y0, 16);
+  k1 += __shfl_xor_sync(0xffffffffu, h16 ? x1 : y1, 16);
+  float k = h8 ? k1 : k0;
+  k += __shfl_xor_sync(0xffffffffu, h8 ? k0 : k1, 8);
+  k += __shfl_xor_sync(0xffffffffu, k, 4);
+  k += __shfl_xor_sync(0xffffffffu, k, 2);
+  k += __shfl_xor_sync(0xffffffffu, k, 1);
+  return k;
 }
 
-// Butterfly of lane partials (x, y): the warp's x sum ends in lanes 0-15, its y sum in lanes
-// 16-31 (fixed order).
-__device__ __forceinline__ float butterfly_xy(float x, float y, int lane) {
-  const bool upper = lane >= 16;
-  float keep = upper ? y : x;
-  const float send = upper ? x : y;
-  keep += __shfl_xor_sync(0xffffffffu, send, 16);
-  keep += __shfl_xor_sync(0xffffffffu, keep, 8);
-  keep += __shfl_xor_sync(0xffffffffu, keep, 4);
-  keep += __shfl_xor_sync(0xffffffffu, keep, 2);
-  keep += __shfl_xor_sync(0xffffffffu, keep, 1);
-  return keep;
-}
-
-__device__ __forceinline__ void prefetch_row(const int2* __restrict__ slot_rows, const int* col, const float* val,
-                                             int s) {
-  const int2 se = __ldg(slot_rows + s);
+__device__ __forceinline__ void prefetch_row(const int* col, const float* val, int2 se) {
   prefetch_l2_range(col, se.x, se.y, 4);
   prefetch_l2_range(val, se.x, se.y, 4);
 }
 
-#ifndef FE_ATTR_MIN_BLOCKS
-#define FE_ATTR_MIN_BLOCKS 6
-#endif
-__global__ void __launch_bounds__(kAttrThreads, FE_ATTR_MIN_BLOCKS)
-attractive_kernel(const int2* __restrict__ slot_rows, const int* __restrict__ col, const float* __restrict__ val,
-                  const float2* __restrict__ y, int n, float exag, float2* __restrict__ attr,
-                  unsigned* __restrict__ ctr, int chunk) {
-  const int lane = threadIdx.x & 31;
-  const unsigned nchunks = (unsigned)((n + chunk - 1) / chunk);
-  const unsigned nwarps = gridDim.x * kAttrWarps;
-  // chunk gw first, then chunks nwarps, nwarps + 1, ... from the counter
-  unsigned c = blockIdx.x * kAttrWarps + (threadIdx.x >> 5), next = 0;
-  if (lane == 0) next = nwarps + atomicAdd(ctr, 1u);
-  next = __shfl_sync(0xffffffffu, next, 0);
-  // slot at position t of chunk c (positions past the chunk run into chunk `next`), or -1
-  auto slot_at = [&](int t) -> int {
-    const unsigned ch = t < chunk ? c : next;
-    if (ch >= nchunks) return -1;
-    const int sl = (int)ch * chunk + (t < chunk ? t : t - chunk);
-    return sl < n ? sl : -1;
-  };
-  if (lane == 0)
-    for (int a = 0; a < kAttrAhead; ++a) {
-      const int t = slot_at(a);
-      if (t >= 0) prefetch_row(slot_rows, col, val, t);
-    }
-  while (c < nchunks) {
-    for (int t = 0; t < chunk; ++t) {
-      const int s = slot_at(t);
-      if (s < 0) break;
-      if (lane == 0) {
-        const int pf = slot_at(t + kAttrAhead);
-        if (pf >= 0) prefetch_row(slot_rows, col, val, pf);
-      }
-      const int2 se = __ldg(slot_rows + s);
-      const float2 yi = __ldg(y + s);
-      const int b = se.x, e = se.y;
-      float ax = 0.0f, ay = 0.0f, kx = 0.0f, ky = 0.0f;
-      for (int c0 = b & ~3; c0 < e; c0 += 128 * kAttrRounds) {
-        int4 ci[kAttrRounds];
-        float4 vv[kAttrRounds];
+// P is read once per pass: its columns and values must not displace the layout in L1.
+__device__ __forceinline__ void ld_stream(const int* pc, const float* pv, int (&c)[4], float (&v)[4]) {
+  asm volatile("ld.global.nc.L1::no_allocate.v4.s32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3])
+               : "l"(pc));
+  asm volatile("ld.global.nc.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3])
+               : "l"(pv));
+}
+
+// Lane partials of row [b, e) of the point yi in slot s. Entries of a round outside the row count as
+// the point s itself with value 0, whose term is exactly zero.
+__device__ __forceinline__ float2 attr_row(const int* __restrict__ col, const float* __restrict__ val,
+                                           const float2* __restrict__ y, int b, int e, int s, float2 yi, int lane) {
+  float ax = 0.0f, ay = 0.0f, kx = 0.0f, ky = 0.0f;
+  for (int c0 = b & ~3; c0 < e; c0 += 128) {
+    const int p = c0 + 4 * lane;
+    int c[4] = {s, s, s, s};
+    float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    if (p < e) ld_stream(col + p, val + p, c, v);
+    if (c0 < b || e - c0 < 128) {  // a round that can hold entries of other rows
 #pragma unroll
-        for (int u = 0; u < kAttrRounds; ++u) {
-          const int p = c0 + 128 * u + 4 * lane;
-          if (p < e) {
-            ci[u] = __ldcs(reinterpret_cast<const int4*>(col + p));
-            vv[u] = __ldcs(reinterpret_cast<const float4*>(val + p));
-          } else {
-            ci[u] = make_int4(s, s, s, s);
-            vv[u] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-          }
+      for (int u = 0; u < 4; ++u)
+        if (p + u < b || p + u >= e) {
+          c[u] = s;
+          v[u] = 0.0f;
         }
-        float rx = 0.0f, ry = 0.0f;
-#pragma unroll
-        for (int u = 0; u < kAttrRounds; ++u) {
-#pragma unroll
-          for (int cc = 0; cc < 4; ++cc) {
-            const int p = c0 + 128 * u + 4 * lane + cc;
-            const bool ok = p >= b && p < e;
-            const float w = ok ? float4_at(vv[u], cc) : 0.0f;
-            const float2 yj = ok ? __ldg(y + int4_at(ci[u], cc)) : yi;
-            const float dx = yi.x - yj.x, dy = yi.y - yj.y;
-            // fast reciprocal (within 2 ulp; 1 + d^2 >= 1 is never denormal or huge): the IEEE
-            // division's instruction sequence cost 5 % of this issue-limited pass
-            const float q = __fdividef(1.0f, 1.0f + (dx * dx + dy * dy));
-            const float cq = w * q;
-            rx += cq * dx;
-            ry += cq * dy;
-          }
-        }
-        const float tx = rx - kx, ty = ry - ky;
-        const float nx = ax + tx, ny = ay + ty;
-        kx = (nx - ax) - tx;
-        ky = (ny - ay) - ty;
-        ax = nx;
-        ay = ny;
-      }
-      const float keep = butterfly_xy(ax, ay, lane);
-      const float sy = __shfl_sync(0xffffffffu, keep, 16);
-      if (lane == 0) attr[s] = make_float2(exag * keep, exag * sy);
     }
-    c = next;
-    if (c < nchunks) {
-      if (lane == 0) next = nwarps + atomicAdd(ctr, 1u);
-      next = __shfl_sync(0xffffffffu, next, 0);
+    float rx = 0.0f, ry = 0.0f;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const float2 yj = __ldg(y + c[u]);
+      const float dx = yi.x - yj.x, dy = yi.y - yj.y;
+      // fast reciprocal (within 2 ulp; 1 + d^2 >= 1 is never denormal or huge); the rounding of
+      // d^2 is fixed so that a change of the surrounding code cannot change the force's bits
+      const float q = __fdividef(1.0f, __fadd_rn(1.0f, __fmaf_rn(dy, dy, __fmul_rn(dx, dx))));
+      const float cq = v[u] * q;
+      rx += cq * dx;
+      ry += cq * dy;
+    }
+    const float tx = rx - kx, ty = ry - ky;
+    const float nx = ax + tx, ny = ay + ty;
+    kx = (nx - ax) - tx;
+    ky = (ny - ay) - ty;
+    ax = nx;
+    ay = ny;
+  }
+  return make_float2(ax, ay);
+}
+
+// Chunk queues of the attractive pass: queue q's count of chunks taken, at ctr[(1 + q) *
+// kAttrCtrStride] (a 32-byte sector each); ctr[0] counts finished blocks. All zero between launches.
+constexpr int kAttrCtrStride = 8;
+// A warp whose queue is empty looks at kAttrProbes others and helps one that has more than kAttrLeave
+// chunks left (an SM with long rows, or none of this launch's blocks). No more than that: the last
+// chunks of a queue are taken within microseconds by its own 40 to 48 warps, while thousands of idle
+// warps reading every counter and chasing the last chunks cost 18 us a launch.
+constexpr unsigned kAttrLeave = 16;
+constexpr int kAttrProbes = 2;
+
+// The chunks of queue q of nq: [begin, begin + size) of 0 .. nchunks - 1.
+struct AttrQueue {
+  unsigned begin, size;
+};
+__device__ __forceinline__ AttrQueue attr_queue(unsigned q, unsigned nq, unsigned nchunks) {
+  const unsigned per = nchunks / nq, extra = nchunks - per * nq;
+  return AttrQueue{q * per + min(q, extra), per + (q < extra ? 1u : 0u)};
+}
+
+// The next chunk of queue q, or nchunks when it is empty.
+__device__ __forceinline__ unsigned attr_take(unsigned* __restrict__ ctr, unsigned q, unsigned nq, unsigned nchunks,
+                                              int lane) {
+  const AttrQueue Q = attr_queue(q, nq, nchunks);
+  unsigned t = 0;
+  if (lane == 0) t = atomicAdd(ctr + (1 + q) * kAttrCtrStride, 1u);
+  t = __shfl_sync(0xffffffffu, t, 0);
+  return t < Q.size ? Q.begin + t : nchunks;
+}
+
+// The next chunk of the warp's queue q; once that is empty, of another queue that needs help, which
+// becomes the warp's; nchunks when it found none.
+__device__ __forceinline__ unsigned attr_pop(unsigned* __restrict__ ctr, unsigned& q, unsigned nq, unsigned nchunks,
+                                             unsigned& rnd, int lane) {
+  unsigned c = attr_take(ctr, q, nq, nchunks, lane);
+  for (int probe = 0; c >= nchunks && probe < kAttrProbes; ++probe) {
+    rnd = rnd * 1664525u + 1013904223u;
+    const unsigned v = __umulhi(rnd, nq);
+    const unsigned taken = __ldcg(ctr + (1 + v) * kAttrCtrStride), size = attr_queue(v, nq, nchunks).size;
+    if (size > taken && size - taken > kAttrLeave) {
+      q = v;
+      c = attr_take(ctr, q, nq, nchunks, lane);
     }
   }
-  if (lane == 0) {
-    __threadfence();
-    const unsigned done = atomicAdd(ctr + 1, 1u);
-    if (done == gridDim.x * kAttrWarps - 1u) {
-      atomicExch(ctr, 0u);
-      atomicExch(ctr + 1, 0u);
+  return c;
+}
+
+// A chunk of any queue that has one left, or nchunks (the counters are read by all lanes at once).
+__device__ __forceinline__ unsigned attr_left(unsigned* __restrict__ ctr, unsigned nq, unsigned nchunks, int lane) {
+  for (unsigned v0 = 0; v0 < nq; v0 += 32) {
+    const unsigned v = v0 + lane;
+    const unsigned taken = v < nq ? __ldcg(ctr + (1 + v) * kAttrCtrStride) : 0u;
+    unsigned some = __ballot_sync(0xffffffffu, v < nq && taken < attr_queue(v, nq, nchunks).size);
+    for (; some; some &= some - 1u) {
+      const unsigned c = attr_take(ctr, v0 + __ffs(some) - 1, nq, nchunks, lane);
+      if (c < nchunks) return c;
     }
+  }
+  return nchunks;
+}
+
+// Per iteration at 1M points (143 M entries, 90 neighbours): 0.508 -> 0.326 ms; 200,000: 98 -> 80 us.
+// The queues took the L1 hit rate from 27 to 77 % and the time to 0.35 ms; the rest came from the
+// masks, the shared reductions and the prefetch. Six blocks per SM with a few spilled registers are
+// faster than five without (0.360 ms at 1M). Rounds narrower than 128 entries at a row's end would
+// save instructions but sum a row in another order; they measured 0.317 ms and are not used.
+__global__ void __launch_bounds__(kAttrThreads, 6)
+attractive_kernel(const int2* __restrict__ slot_rows, const int* __restrict__ col, const float* __restrict__ val,
+                  const float2* __restrict__ y, int n, float exag, float2* __restrict__ attr,
+                  unsigned* __restrict__ ctr, int chunk, unsigned nq) {
+  const int lane = threadIdx.x & 31;
+  const unsigned nchunks = (unsigned)((n + chunk - 1) / chunk);
+  // with a warp for every chunk, warp w takes chunk w and no counter is touched
+  const bool queued = nchunks > gridDim.x * kAttrWarps;
+  unsigned q = 0, c = blockIdx.x * kAttrWarps + (threadIdx.x >> 5), next = nchunks;
+  unsigned rnd = c * 2654435761u;
+  bool sweep = false;
+  auto pop = [&]() -> unsigned {
+    if (!queued) return nchunks;
+    if (!sweep) return attr_pop(ctr, q, nq, nchunks, rnd, lane);
+    return attr_left(ctr, nq, nchunks, lane);
+  };
+  if (queued) {
+    asm("mov.u32 %0, %%smid;" : "=r"(q));
+    q %= nq;
+    // a block's first two chunks per warp come with one atomic
+    __shared__ unsigned s_first;
+    if (threadIdx.x == 0) s_first = atomicAdd(ctr + (1 + q) * kAttrCtrStride, 2u * kAttrWarps);
+    __syncthreads();
+    const AttrQueue Q = attr_queue(q, nq, nchunks);
+    const unsigned t0 = s_first + (threadIdx.x >> 5), t1 = t0 + kAttrWarps;
+    c = t0 < Q.size ? Q.begin + t0 : pop();
+    if (c < nchunks) next = t1 < Q.size ? Q.begin + t1 : pop();
+  }
+  // lane l holds the bounds of row l of the chunk (chunk <= 32) and its point, so a row's bounds cost
+  // no load; the next chunk's are loaded while this one is processed
+  auto rows_of = [&](unsigned ch, int2& se, float2& yl) {
+    const long long s = (long long)ch * chunk + lane;
+    se = make_int2(0, 0);
+    yl = make_float2(0.0f, 0.0f);
+    if (ch < nchunks && lane < chunk && s < n) {
+      se = __ldg(slot_rows + s);
+      yl = __ldg(y + s);
+    }
+  };
+  int2 se;
+  float2 yl;
+  for (;;) {
+    rows_of(c, se, yl);
+    if (lane < 2) prefetch_row(col, val, se);
+    while (c < nchunks) {
+      int2 sn;
+      float2 yn;
+      rows_of(next, sn, yn);
+      const int s0 = (int)c * chunk, rows = min(chunk, n - s0);
+      for (int t = 0; t < rows; t += 2) {
+        // L2 prefetch of the two rows after these, in this chunk or the next: further ahead the
+        // rows in flight of all warps no longer fit L2 (8 rows: 0.42 ms at 1M)
+        const bool inside = t + 2 < chunk;
+        if (inside ? (lane >> 1) == (t >> 1) + 1 : lane < 2) prefetch_row(col, val, inside ? se : sn);
+        float2 a[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          // a missing second row has bounds (0, 0) in its lane, or repeats nothing past lane 31
+          const int src = min(t + u, 31);
+          const int b = __shfl_sync(0xffffffffu, se.x, src), e = __shfl_sync(0xffffffffu, se.y, src);
+          const float2 yi = make_float2(__shfl_sync(0xffffffffu, yl.x, src), __shfl_sync(0xffffffffu, yl.y, src));
+          a[u] = attr_row(col, val, y, b, t + u < rows ? e : b, s0 + t + u, yi, lane);
+        }
+        const float sum = exag * butterfly_rows(a[0].x, a[0].y, a[1].x, a[1].y, lane);
+        // lanes 0, 8, 16, 24 hold x0, x1, y0, y1
+        const int u = (lane >> 3) & 1;
+        if ((lane & 7) == 0 && t + u < rows) reinterpret_cast<float*>(attr + s0 + t + u)[lane >> 4] = sum;
+      }
+      c = next;
+      se = sn;
+      yl = yn;
+      if (c < nchunks) next = pop();
+    }
+    if (!queued || sweep) break;
+    // the last block to finish takes whatever is left (chunks of an SM that ran no block of this
+    // launch and that no probe met), then clears the counters for the next launch
+    if (!last_block_done(ctr, gridDim.x)) return;
+    sweep = true;
+    q = 0;
+    c = pop();
+    next = c < nchunks ? pop() : nchunks;
+  }
+  if (sweep) {
+    __syncthreads();
+    for (unsigned v = threadIdx.x; v < nq; v += blockDim.x) ctr[(1 + v) * kAttrCtrStride] = 0u;
   }
 }
 
@@ -1351,7 +1451,13 @@ void tsne_batch_alloc(TsneDevice& d, const std::vector<int>& sizes, const std::v
   const int n = (int)total;
   d.n = n;
   d.nblocks = nblocks;
+  d.attr_queues = sm_count();
   d.attr_blocks = persistent_blocks(attractive_kernel, kAttrThreads, n);
+  // Up to 8 rows for each resident warp: one chunk a warp, without counters (20,000 points: 14 us
+  // against 18 from the queues; 50,000: 24 against 29). More: queues of 4-row chunks (200,000
+  // points: 79 us; 8 rows 84, 2 rows 80), of 8 rows where a warp takes many (1M: 326 against 331).
+  const int warps = d.attr_blocks * kAttrWarps;
+  d.attr_chunk = n <= 8 * warps ? std::max(1, ceil_div(n, warps)) : n <= 64 * warps ? 4 : 8;
   d.arena.release();
   d.arena.reserve(&d.d_inst, ninst);
   d.arena.reserve(&d.blocks, nblocks);
@@ -1367,7 +1473,7 @@ void tsne_batch_alloc(TsneDevice& d, const std::vector<int>& sizes, const std::v
   d.arena.reserve(&d.perm, n);
   d.arena.reserve(&d.inv, n);
   d.arena.reserve(&d.slot_rows, n);
-  d.arena.reserve(&d.attr_ctr, 2);
+  d.arena.reserve(&d.attr_ctr, (1 + (std::size_t)d.attr_queues) * kAttrCtrStride);
   d.arena.reserve(&d.keys, n);
   d.arena.reserve(&d.keys_tmp, n);
   d.arena.reserve(&d.order, n);
@@ -1388,7 +1494,7 @@ void tsne_batch_alloc(TsneDevice& d, const std::vector<int>& sizes, const std::v
   FE_CUDA(cudaMemcpy(d.d_inst, d.inst.data(), sizeof(TsneInstance) * ninst, cudaMemcpyHostToDevice));
   FE_CUDA(cudaMemcpy(d.blocks, blk.data(), sizeof(int2) * nblocks, cudaMemcpyHostToDevice));
   FE_CUDA(cudaMemset(d.counter, 0, sizeof(unsigned) * ninst));
-  FE_CUDA(cudaMemset(d.attr_ctr, 0, sizeof(unsigned) * 2));
+  FE_CUDA(cudaMemset(d.attr_ctr, 0, sizeof(unsigned) * (1 + (std::size_t)d.attr_queues) * kAttrCtrStride));
   FE_CUDA(cudaMemset(d.cur, 0, sizeof(GridState) * ninst));
   if (!d.side) FE_CUDA(cudaStreamCreateWithFlags(&d.side, cudaStreamNonBlocking));
   if (!d.fork) FE_CUDA(cudaEventCreateWithFlags(&d.fork, cudaEventDisableTiming));
@@ -1459,7 +1565,7 @@ void tsne_bind_rows(TsneDevice& d, const DeviceCsr& P, cudaStream_t s) {
 
 void tsne_attractive_stage(TsneDevice& d, const DeviceCsr& P, float exag, cudaStream_t s) {
   attractive_kernel<<<d.attr_blocks, kAttrThreads, 0, s>>>(d.slot_rows, P.col, P.val, d.y, d.n, exag, d.attr,
-                                                           d.attr_ctr, d.attr_chunk);
+                                                           d.attr_ctr, d.attr_chunk, (unsigned)d.attr_queues);
   FE_LAUNCH("attractive_kernel");
 }
 
@@ -1472,7 +1578,7 @@ bool tsne_tune_attractive(TsneDevice& d, const DeviceCsr& P, float exag, cudaStr
   int per_sm = 0;
   FE_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, attractive_kernel, kAttrThreads, 0));
   per_sm = std::max(1, per_sm);
-  const int chunks[] = {4, 8, 16};
+  const int chunks[] = {2, 4, 8};
   const int old_chunk = d.attr_chunk, old_blocks = d.attr_blocks;
   cudaEvent_t e0, e1;
   FE_CUDA(cudaEventCreate(&e0));

@@ -97,7 +97,8 @@ struct TsneDevice {
   int* inv = nullptr;
   int2* slot_rows = nullptr;     // CSR segment (begin, end) of the point in each storage slot
   unsigned* attr_ctr = nullptr;  // work counters of the attractive pass (zero between launches)
-  int attr_chunk = 8;            // slots per work item of the attractive pass
+  int attr_queues = 1;           // chunk queues of the attractive pass: one per SM
+  int attr_chunk = 8;            // slots per work item of the attractive pass (at most 32)
   struct Tuning {
     int chunk, blocks;
     float ms;
