@@ -7,21 +7,13 @@
 // back, combine with the sparse attractive term and apply the gains/momentum update.
 //
 // GB300 layout of one iteration (6 launches, two streams, captured in a CUDA graph):
-//   side stream:  attractive_kernel        warp-per-row CSR attractive force, rows in storage
-//                                          (spatial) order (stream of P + L1/L2 gathers of y)
+//   side stream:  attractive_kernel        warp per CSR row, rows in storage (spatial) order, one
+//                                          queue of rows per SM
 //   main stream:  scatter_kernel           points -> 64-bit fixed-point charges (deterministic)
-//                 rows_forward_kernel      row FFTs of the charges (x + i y plane, paired mass
-//                                          rows as half spectra) and of the kernel rows; the top
-//                                          stages run in registers on the values as loaded
-//                 columns_convolve_kernel  column FFTs per conjugate column pair, Z by Parseval,
-//                                          multiply, inverse column FFTs in shared memory; the
-//                                          passes next to global memory and to the product run
-//                                          in registers
-//                 rows_inverse_kernel      inverse row FFTs -> float4 potentials, Z finalised
+//                 row FFTs, column FFTs with the products, inverse row FFTs (tsne_fft.cu)
 //   join:         update_kernel            potential gather + gains/momentum/step clip +
 //                                          recentring; epilogue reduces the new bounding box and
 //                                          mean into the next iteration's grid
-// The attractive pass (load-latency-bound) runs beside the grid stage (shared-memory bound).
 // Interpolation: the reference bilinear splat on G shared nodes (default), or 3 equispaced
 // Lagrange nodes per box over floor(G / 3) boxes, as in FIt-SNE-style interpolation.
 #include <cfloat>
@@ -35,9 +27,6 @@
 namespace fe {
 
 constexpr int kStepThreads = 256;
-constexpr int kFftThreads = 256;
-constexpr int kColThreads = 256;  // the column pass holds 4 x M complex values of shared memory
-                                  // (70 KB at M = 2048: 3 blocks per SM)
 
 // ---------------------------------------------------------------- stencils
 template <int TAPS>
@@ -351,519 +340,6 @@ scatter_kernel(const float2* __restrict__ y, const TsneInstance* __restrict__ in
       red_add_i64(dst, (long long)((unsigned long long)(long long)a0 << sh));
       red_add_i64(dst + 1, (long long)((unsigned long long)(long long)a1 << sh));
       red_add_i64(dst + 2, (long long)((unsigned long long)(long long)a2 << sh));
-    }
-  }
-}
-
-// ---------------------------------------------------------------- shared-memory FFT
-__device__ __forceinline__ float2 cmul(float2 a, float2 b) {
-  return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
-}
-// Shared-memory index with one pad slot after every 16 complex values: the radix-2^4 passes with
-// small butterfly strides (1, 16) touch elements 16 or 256 apart from consecutive threads, which
-// would otherwise land on the same banks (with this padding every pass of M = 512 .. 2048 is
-// free of bank conflicts for 64-bit accesses).
-__device__ __forceinline__ int sidx(int i) { return i + (i >> 4); }
-__host__ __device__ constexpr int padded(int count) { return count + count / 16; }
-
-// Radix-2 FFTs over `count` sequences of length M = 2^logm stored at buf + seq * M, with R
-// consecutive radix-2 stages fused per shared-memory pass (R <= MAXR <= 4; with 4, M = 2048 takes
-// three passes): each work item keeps the 2^R elements i0 + t * 2^s of one butterfly group in
-// registers. tw[t] = exp(-2 pi i t / M). The forward row pass uses MAXR = 3.
-__device__ __forceinline__ float2 twiddle(const float2* __restrict__ tw, int x, int shift, bool inverse) {
-  float2 w = tw[x << shift];
-  if (inverse) w.y = -w.y;
-  return w;
-}
-
-// Radix-2 butterflies of one work item held in registers: v[e] is element i0 + e * h of its
-// sequence, h = 2^s, j = i0 mod h. Decimation in time: stages s .. s + R - 1 (input of the FFT
-// in bit-reversed order).
-template <int R>
-__device__ __forceinline__ void dit_regs(float2 (&v)[1 << R], int j, int s, int logm, const float2* __restrict__ tw,
-                                         bool inverse) {
-  constexpr int E = 1 << R;
-  const int h = 1 << s;
-#pragma unroll
-  for (int st = 0; st < R; ++st) {
-    const int span = 1 << st;               // partner distance in units of h
-    const int shift = logm - 1 - (s + st);  // twiddle stride for block length 2^(s+st+1)
-#pragma unroll
-    for (int e = 0; e < E; ++e) {
-      if (e & span) continue;
-      const float2 w = twiddle(tw, j + (e & (span - 1)) * h, shift, inverse);
-      const float2 x = cmul(v[e + span], w);
-      const float2 u = v[e];
-      v[e] = make_float2(u.x + x.x, u.y + x.y);
-      v[e + span] = make_float2(u.x - x.x, u.y - x.y);
-    }
-  }
-}
-
-// Decimation in frequency: stages s + R - 1 down to s (output in bit-reversed order).
-template <int R>
-__device__ __forceinline__ void dif_regs(float2 (&v)[1 << R], int j, int s, int logm, const float2* __restrict__ tw,
-                                         bool inverse) {
-  constexpr int E = 1 << R;
-  const int h = 1 << s;
-#pragma unroll
-  for (int st = R - 1; st >= 0; --st) {
-    const int span = 1 << st;
-    const int shift = logm - 1 - (s + st);
-#pragma unroll
-    for (int e = 0; e < E; ++e) {
-      if (e & span) continue;
-      const float2 w = twiddle(tw, j + (e & (span - 1)) * h, shift, inverse);
-      const float2 u = v[e], x = v[e + span];
-      v[e] = make_float2(u.x + x.x, u.y + x.y);
-      v[e + span] = cmul(make_float2(u.x - x.x, u.y - x.y), w);
-    }
-  }
-}
-
-// One shared-memory pass of R stages starting at stage s over `count` sequences.
-template <int R>
-__device__ __forceinline__ void dit_pass(float2* buf, int count, int logm, int s, const float2* __restrict__ tw,
-                                         bool inverse) {
-  constexpr int E = 1 << R;
-  const int h = 1 << s;
-  const int items = count << (logm - R);
-  for (int t = threadIdx.x; t < items; t += blockDim.x) {
-    const int seq = t >> (logm - R);
-    const int rem = t & ((1 << (logm - R)) - 1);
-    const int j = rem & (h - 1);
-    const int i0 = (seq << logm) + ((rem >> s) << (s + R)) + j;
-    float2 v[E];
-#pragma unroll
-    for (int e = 0; e < E; ++e) v[e] = buf[sidx(i0 + e * h)];
-    dit_regs<R>(v, j, s, logm, tw, inverse);
-#pragma unroll
-    for (int e = 0; e < E; ++e) buf[sidx(i0 + e * h)] = v[e];
-  }
-}
-
-template <int R>
-__device__ __forceinline__ void dif_pass(float2* buf, int count, int logm, int s, const float2* __restrict__ tw,
-                                         bool inverse) {
-  constexpr int E = 1 << R;
-  const int h = 1 << s;
-  const int items = count << (logm - R);
-  for (int t = threadIdx.x; t < items; t += blockDim.x) {
-    const int seq = t >> (logm - R);
-    const int rem = t & ((1 << (logm - R)) - 1);
-    const int j = rem & (h - 1);
-    const int i0 = (seq << logm) + ((rem >> s) << (s + R)) + j;
-    float2 v[E];
-#pragma unroll
-    for (int e = 0; e < E; ++e) v[e] = buf[sidx(i0 + e * h)];
-    dif_regs<R>(v, j, s, logm, tw, inverse);
-#pragma unroll
-    for (int e = 0; e < E; ++e) buf[sidx(i0 + e * h)] = v[e];
-  }
-}
-
-// Stages lo .. hi - 1 (decimation in time) or top down to lo (decimation in frequency), at most
-// MAXR per shared-memory pass; each pass ends with a barrier.
-template <int MAXR = 4>
-__device__ void fft_dit(float2* buf, int count, int logm, const float2* __restrict__ tw, bool inverse, int lo = 0,
-                        int hi = -1) {
-  if (hi < 0) hi = logm;
-  for (int s = lo; s < hi;) {
-    const int r = min(MAXR, hi - s);
-    if (r == 4) dit_pass<4>(buf, count, logm, s, tw, inverse);
-    else if (r == 3) dit_pass<3>(buf, count, logm, s, tw, inverse);
-    else if (r == 2) dit_pass<2>(buf, count, logm, s, tw, inverse);
-    else dit_pass<1>(buf, count, logm, s, tw, inverse);
-    __syncthreads();
-    s += r;
-  }
-}
-
-template <int MAXR = 4>
-__device__ void fft_dif(float2* buf, int count, int logm, const float2* __restrict__ tw, bool inverse, int top = -1,
-                        int lo = 0) {
-  if (top < 0) top = logm - 1;
-  while (top >= lo) {
-    const int r = min(MAXR, top - lo + 1);
-    const int s = top - r + 1;
-    if (r == 4) dif_pass<4>(buf, count, logm, s, tw, inverse);
-    else if (r == 3) dif_pass<3>(buf, count, logm, s, tw, inverse);
-    else if (r == 2) dif_pass<2>(buf, count, logm, s, tw, inverse);
-    else dif_pass<1>(buf, count, logm, s, tw, inverse);
-    __syncthreads();
-    top = s - 1;
-  }
-}
-
-// Forward transforms are decimation in frequency (natural order in, bit-reversed order out) and
-// inverse transforms decimation in time (bit-reversed in, natural out); spectra are stored in
-// natural frequency order between the passes (written from, and loaded into, bit-reversed
-// shared-memory positions), and the column pass multiplies its spectra element by element in
-// the bit-reversed order both of its operands share.
-//
-// Real-input savings (the three charge planes and the kernel are real):
-//   * the x and y charges travel as one complex plane A = x-charge + i y-charge (all M columns);
-//   * the mass plane B is real, so its row spectra are Hermitian: B^[r][M - f] = conj(B^[r][f]),
-//     and only f = 0 .. M/2 is kept. Rows are transformed in pairs (r, r + npairs): one complex
-//     FFT of m_r + i m_r2 gives both half spectra;
-//   * the kernel rows q + i q^2 are real and even in x: their spectra Kq + i Kq2 have real parts,
-//     and K^[dy][M - f] = K^[dy][f], so f = 0 .. M/2 is kept;
-//   * the column pass takes frequency columns in conjugate pairs (c, M - c): A_c, A_(M-c), B_c and
-//     one kernel column (K_(M-c) = K_c) are transformed, B_(M-c) being conj(B_c) row by row;
-//     the Parseval sum of the pair is twice that of column c (once for c = 0 and c = M/2);
-//   * the inverse row pass rebuilds each B row's full spectrum from its half and transforms two
-//     rows in one complex FFT (real parts: row r, imaginary parts: row r2).
-// Per pair of rows and pair of columns that is 3 + 4 + 3 + 3 transforms of length M where the
-// plain complex scheme needs 4 + 6 + 4 + 4 (and the kernel rows once per row in both).
-__device__ __forceinline__ int bitrev(int f, int logm) { return (int)(__brev((unsigned)f) >> (32 - logm)); }
-__device__ __forceinline__ float2 conjf2(float2 a) { return make_float2(a.x, -a.y); }
-
-// The row pass's top forward pass (stages logm - 1 .. logm - kRowTop) runs on values loaded or
-// computed straight into registers rather than staged in shared memory first; the butterflies
-// are those of dif_pass.
-constexpr int kRowTop = 3;
-
-// Charge rows: the fixed-point charges of nodes j + e h of rows r1 (c1) and r2 (c2) are read,
-// cleared for the next scatter and converted, then transformed as A_r1, A_r2 and m_r1 + i m_r2.
-template <int R>
-__device__ __forceinline__ void rows_charges_dif_top(float2* sbuf, longlong2* __restrict__ c1,
-                                                     longlong2* __restrict__ c2, bool has2, int nodes, float inv_q,
-                                                     int logm, const float2* __restrict__ tw) {
-  constexpr int E = 1 << R;
-  const int m = 1 << logm, s = logm - R, h = 1 << s;
-  for (int j = threadIdx.x; j < h; j += blockDim.x) {
-    float2 a[E];
-    float mx[E], my[E];
-#pragma unroll
-    for (int e = 0; e < E; ++e) {
-      const int c = j + e * h;
-      a[e] = make_float2(0.0f, 0.0f);
-      mx[e] = 0.0f;
-      if (c < nodes) {
-        const longlong2 p0 = c1[2 * c], p1 = c1[2 * c + 1];
-        c1[2 * c] = make_longlong2(0, 0);
-        c1[2 * c + 1] = make_longlong2(0, 0);
-        a[e] = make_float2((float)p0.y * inv_q, (float)p1.x * inv_q);
-        mx[e] = (float)p0.x * inv_q;
-      }
-    }
-    dif_regs<R>(a, j, s, logm, tw, false);
-#pragma unroll
-    for (int e = 0; e < E; ++e) sbuf[sidx(j + e * h)] = a[e];
-#pragma unroll
-    for (int e = 0; e < E; ++e) {
-      const int c = j + e * h;
-      a[e] = make_float2(0.0f, 0.0f);
-      my[e] = 0.0f;
-      if (has2 && c < nodes) {
-        const longlong2 p0 = c2[2 * c], p1 = c2[2 * c + 1];
-        c2[2 * c] = make_longlong2(0, 0);
-        c2[2 * c + 1] = make_longlong2(0, 0);
-        a[e] = make_float2((float)p0.y * inv_q, (float)p1.x * inv_q);
-        my[e] = (float)p0.x * inv_q;
-      }
-    }
-    dif_regs<R>(a, j, s, logm, tw, false);
-#pragma unroll
-    for (int e = 0; e < E; ++e) sbuf[sidx(m + j + e * h)] = a[e];
-#pragma unroll
-    for (int e = 0; e < E; ++e) a[e] = make_float2(mx[e], my[e]);
-    dif_regs<R>(a, j, s, logm, tw, false);
-#pragma unroll
-    for (int e = 0; e < E; ++e) sbuf[sidx(2 * m + j + e * h)] = a[e];
-  }
-}
-
-// Kernel rows dy1 and dy2 (offsets yo1, yo2): (q, q^2) of columns j + e h, q = 1 / (1 + d^2),
-// zero beyond +-(nodes - 1) columns.
-template <int R>
-__device__ __forceinline__ void rows_kernel_dif_top(float2* sbuf, int nodes, float h_node, float yo1, float yo2,
-                                                    int logm, const float2* __restrict__ tw) {
-  constexpr int E = 1 << R;
-  const int m = 1 << logm, hm = m >> 1, s = logm - R, h = 1 << s;
-  for (int j = threadIdx.x; j < h; j += blockDim.x) {
-    float2 v1[E], v2[E];
-#pragma unroll
-    for (int e = 0; e < E; ++e) {
-      const int c = j + e * h;
-      const int dx = c < hm ? c : c - m;
-      v1[e] = make_float2(0.0f, 0.0f);
-      v2[e] = v1[e];
-      if (dx <= nodes - 1 && dx >= -(nodes - 1)) {
-        const float xo = (float)dx * h_node;
-        const float q1 = 1.0f / (1.0f + (xo * xo + yo1 * yo1));
-        const float q2 = 1.0f / (1.0f + (xo * xo + yo2 * yo2));
-        v1[e] = make_float2(q1, q1 * q1);
-        v2[e] = make_float2(q2, q2 * q2);
-      }
-    }
-    dif_regs<R>(v1, j, s, logm, tw, false);
-    dif_regs<R>(v2, j, s, logm, tw, false);
-#pragma unroll
-    for (int e = 0; e < E; ++e) {
-      sbuf[sidx(j + e * h)] = v1[e];
-      sbuf[sidx(m + j + e * h)] = v2[e];
-    }
-  }
-}
-
-// Row pass. Blocks [0, npairs): charge rows r1 = p and r2 = p + npairs (r2 < nodes or absent):
-// forward FFTs of A_r1, A_r2 and m_r1 + i m_r2; A spectra to arow (natural order, all M),
-// separated B half spectra to brow (f = 0 .. M/2); the charge rows are cleared for the next
-// scatter. Blocks [npairs, 2 npairs): kernel rows dy1 = p and dy2 = p + npairs -> forward FFTs of
-// (q + i q^2), f = 0 .. M/2 kept. blockIdx.y selects the instance members[blockIdx.y] of the grid
-// class.
-#ifndef FE_ROW_MIN_BLOCKS
-#define FE_ROW_MIN_BLOCKS 4
-#endif
-__global__ void __launch_bounds__(kFftThreads, FE_ROW_MIN_BLOCKS)
-rows_forward_kernel(const TsneInstance* __restrict__ inst, const int* __restrict__ members, int grid, int nodes,
-                    int logm, const float2* __restrict__ tw, const GridState* __restrict__ cur,
-                    float2* __restrict__ arow, float2* __restrict__ brow, float2* __restrict__ krow) {
-  extern __shared__ float2 sbuf[];
-  const int m = 1 << logm, hm = m >> 1;
-  const int npairs = (nodes + 1) >> 1;
-  const int b = members[blockIdx.y];
-  long long* __restrict__ charges = inst[b].charges;
-  cur += b;
-  arow += (long long)blockIdx.y * nodes * m;
-  brow += (long long)blockIdx.y * nodes * (hm + 1);
-  krow += (long long)blockIdx.y * nodes * (hm + 1);
-  if ((int)blockIdx.x < npairs) {
-    const int r1 = blockIdx.x, r2 = blockIdx.x + npairs;
-    const bool has2 = r2 < nodes;
-    const float inv_q = cur->inv_qscale;
-    longlong2* c1 = reinterpret_cast<longlong2*>(charges + (long long)r1 * grid * kChargeStride);
-    longlong2* c2 = reinterpret_cast<longlong2*>(charges + (long long)(has2 ? r2 : r1) * grid * kChargeStride);
-    rows_charges_dif_top<kRowTop>(sbuf, c1, c2, has2, nodes, inv_q, logm, tw);
-    __syncthreads();
-    fft_dif<3>(sbuf, 3, logm, tw, false, logm - kRowTop - 1, 0);
-    float2* o1 = arow + (long long)r1 * m;
-    float2* o2 = arow + (long long)r2 * m;
-    for (int f = threadIdx.x; f < m; f += blockDim.x) {
-      const int p = bitrev(f, logm);
-      o1[f] = sbuf[sidx(p)];
-      if (has2) o2[f] = sbuf[sidx(m + p)];
-    }
-    float2* b1 = brow + (long long)r1 * (hm + 1);
-    float2* b2 = brow + (long long)r2 * (hm + 1);
-    for (int f = threadIdx.x; f <= hm; f += blockDim.x) {
-      const float2 z = sbuf[sidx(2 * m + bitrev(f, logm))];
-      const float2 zc = conjf2(sbuf[sidx(2 * m + bitrev((m - f) & (m - 1), logm))]);
-      b1[f] = make_float2(0.5f * (z.x + zc.x), 0.5f * (z.y + zc.y));
-      if (has2) b2[f] = make_float2(0.5f * (z.y - zc.y), -0.5f * (z.x - zc.x));
-    }
-  } else {
-    const int k1 = blockIdx.x - npairs, k2 = k1 + npairs;
-    const bool has2 = k2 < nodes;
-    const float h = cur->h;
-    const float yo1 = (float)k1 * h, yo2 = (float)k2 * h;
-    rows_kernel_dif_top<kRowTop>(sbuf, nodes, h, yo1, yo2, logm, tw);
-    __syncthreads();
-    fft_dif<3>(sbuf, 2, logm, tw, false, logm - kRowTop - 1, 0);
-    float2* o1 = krow + (long long)k1 * (hm + 1);
-    float2* o2 = krow + (long long)k2 * (hm + 1);
-    for (int f = threadIdx.x; f <= hm; f += blockDim.x) {
-      const int p = bitrev(f, logm);
-      o1[f] = sbuf[sidx(p)];
-      if (has2) o2[f] = sbuf[sidx(m + p)];
-    }
-  }
-}
-
-// Column pass for the conjugate pair (c, c') = (j, M - j), j = 0 .. M/2 (c' = c for j = 0 and
-// M/2): column FFTs of A_c, A_c', B_c and the kernel column K_c (giving the real spectra
-// Kq + i Kq2), the Parseval sum of |B^|^2 Kq over both columns of the pair (Z + n up to the
-// 1 / M^2 scale), the products with Kq2 and their inverse column FFTs; rows < nodes of the
-// results go back to arow / brow.
-//
-// Three shared-memory round trips of the plain scheme are kept in registers, with the same
-// radix-2 butterflies: the top forward pass takes its inputs straight from global memory, the
-// last forward pass (stages 2 .. 0, groups of 8 consecutive positions), the products and the
-// first inverse pass (stages 0 .. 2, the same groups) run in one pass, and the top inverse pass
-// writes its outputs straight to global memory.
-constexpr int kColBottom = 3;
-
-template <int R>
-__device__ __forceinline__ void col_load_dif_top(float2* sbuf, const float2* __restrict__ arow,
-                                                 const float2* __restrict__ brow, const float2* __restrict__ krow,
-                                                 int c, int c2, int nodes, int logm, const float2* __restrict__ tw) {
-  constexpr int E = 1 << R;
-  const int m = 1 << logm, hm = m >> 1;
-  const int s = logm - R, h = 1 << s;
-  const int items = 4 << s;
-  for (int t = threadIdx.x; t < items; t += blockDim.x) {
-    const int seq = t >> s, j = t & (h - 1);
-    float2 v[E];
-#pragma unroll
-    for (int e = 0; e < E; ++e) {
-      const int r = j + e * h;
-      float2 x = make_float2(0.0f, 0.0f);
-      if (seq == 3) {
-        const int dy = r < hm ? r : m - r;
-        if (dy <= nodes - 1) x = krow[(long long)dy * (hm + 1) + c];
-      } else if (r < nodes) {
-        x = seq == 2 ? brow[(long long)r * (hm + 1) + c] : arow[(long long)r * m + (seq == 0 ? c : c2)];
-      }
-      v[e] = x;
-    }
-    dif_regs<R>(v, j, s, logm, tw, false);
-#pragma unroll
-    for (int e = 0; e < E; ++e) sbuf[sidx((seq << logm) + j + e * h)] = v[e];
-  }
-}
-
-template <int R>
-__device__ __forceinline__ void col_dit_top_store(const float2* sbuf, float2* __restrict__ arow,
-                                                  float2* __restrict__ brow, int c, int c2, int nodes, int logm,
-                                                  const float2* __restrict__ tw) {
-  constexpr int E = 1 << R;
-  const int m = 1 << logm, hm = m >> 1;
-  const int s = logm - R, h = 1 << s;
-  const int items = 3 << s;
-  for (int t = threadIdx.x; t < items; t += blockDim.x) {
-    const int seq = t >> s, j = t & (h - 1);
-    if (seq == 1 && c2 == c) continue;
-    float2 v[E];
-#pragma unroll
-    for (int e = 0; e < E; ++e) v[e] = sbuf[sidx((seq << logm) + j + e * h)];
-    dit_regs<R>(v, j, s, logm, tw, true);
-#pragma unroll
-    for (int e = 0; e < E; ++e) {
-      const int r = j + e * h;
-      if (r < nodes) {
-        if (seq == 2) brow[(long long)r * (hm + 1) + c] = v[e];
-        else arow[(long long)r * m + (seq == 0 ? c : c2)] = v[e];
-      }
-    }
-  }
-}
-
-// 3 blocks per SM, as the 4 x M complex shared-memory buffer allows at M = 2048
-#ifndef FE_COL_MIN_BLOCKS
-#define FE_COL_MIN_BLOCKS 3
-#endif
-__global__ void __launch_bounds__(kColThreads, FE_COL_MIN_BLOCKS)
-columns_convolve_kernel(float2* __restrict__ arow, float2* __restrict__ brow, const float2* __restrict__ krow,
-                        int nodes, int logm, const float2* __restrict__ tw, double* __restrict__ zpart) {
-  extern __shared__ float2 sbuf[];  // [A_c][A_c'][B_c][K_c]
-  __shared__ double s_z[kColThreads / 32];
-  const int m = 1 << logm, hm = m >> 1;
-  const int j = blockIdx.x;
-  const int c = j, c2 = (m - j) & (m - 1);
-  arow += (long long)blockIdx.y * nodes * m;
-  brow += (long long)blockIdx.y * nodes * (hm + 1);
-  krow += (long long)blockIdx.y * nodes * (hm + 1);
-  zpart += (long long)blockIdx.y * gridDim.x;
-  // logm >= 4 (M >= 16): the top pass has 1 .. 4 stages above the fused bottom three
-  const int rt = min(4, logm - kColBottom);
-  if (rt == 4) col_load_dif_top<4>(sbuf, arow, brow, krow, c, c2, nodes, logm, tw);
-  else if (rt == 3) col_load_dif_top<3>(sbuf, arow, brow, krow, c, c2, nodes, logm, tw);
-  else if (rt == 2) col_load_dif_top<2>(sbuf, arow, brow, krow, c, c2, nodes, logm, tw);
-  else col_load_dif_top<1>(sbuf, arow, brow, krow, c, c2, nodes, logm, tw);
-  __syncthreads();
-  fft_dif(sbuf, 4, logm, tw, false, logm - rt - 1, kColBottom);
-  double zl = 0.0;
-  constexpr int E = 1 << kColBottom;
-  for (int g = threadIdx.x; g < (m >> kColBottom); g += blockDim.x) {
-    const int i0 = g << kColBottom;
-    float2 kv[E];
-#pragma unroll
-    for (int e = 0; e < E; ++e) kv[e] = sbuf[sidx(3 * m + i0 + e)];
-    dif_regs<kColBottom>(kv, 0, 0, logm, tw, false);
-#pragma unroll
-    for (int seq = 0; seq < 3; ++seq) {
-      float2 v[E];
-#pragma unroll
-      for (int e = 0; e < E; ++e) v[e] = sbuf[sidx(seq * m + i0 + e)];
-      dif_regs<kColBottom>(v, 0, 0, logm, tw, false);
-#pragma unroll
-      for (int e = 0; e < E; ++e) {
-        if (seq == 2) zl += ((double)v[e].x * v[e].x + (double)v[e].y * v[e].y) * (double)kv[e].x;
-        v[e].x *= kv[e].y;
-        v[e].y *= kv[e].y;
-      }
-      dit_regs<kColBottom>(v, 0, 0, logm, tw, true);
-#pragma unroll
-      for (int e = 0; e < E; ++e) sbuf[sidx(seq * m + i0 + e)] = v[e];
-    }
-  }
-  __syncthreads();
-  fft_dit(sbuf, 3, logm, tw, true, kColBottom, logm - rt);
-  if (rt == 4) col_dit_top_store<4>(sbuf, arow, brow, c, c2, nodes, logm, tw);
-  else if (rt == 3) col_dit_top_store<3>(sbuf, arow, brow, c, c2, nodes, logm, tw);
-  else if (rt == 2) col_dit_top_store<2>(sbuf, arow, brow, c, c2, nodes, logm, tw);
-  else col_dit_top_store<1>(sbuf, arow, brow, c, c2, nodes, logm, tw);
-  zl = warp_sum(zl);
-  if ((threadIdx.x & 31) == 0) s_z[threadIdx.x >> 5] = zl;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double z = 0.0;
-    for (int w = 0; w < (int)(blockDim.x / 32); ++w) z += s_z[w];
-    zpart[blockIdx.x] = c2 != c ? 2.0 * z : z;
-  }
-}
-
-// Inverse row pass for the row pair (r1, r2) -> potentials (phi_q2, phi_x, phi_y) per node; block
-// 0 also finalises Z = sum_k |F_mass|^2 Kq / M^2 - n (the reference's sum_i q_grid(y_i) - n).
-__global__ void __launch_bounds__(kFftThreads, 4)
-rows_inverse_kernel(const float2* __restrict__ arow, const float2* __restrict__ brow,
-                    const TsneInstance* __restrict__ inst, const int* __restrict__ members, int grid, int nodes,
-                    int logm, const float2* __restrict__ tw, const double* __restrict__ zpart, int zblocks,
-                    GridState* __restrict__ cur) {
-  extern __shared__ float2 sbuf[];
-  const int m = 1 << logm, hm = m >> 1;
-  const int npairs = (nodes + 1) >> 1;
-  const int r1 = blockIdx.x, r2 = blockIdx.x + npairs;
-  const bool has2 = r2 < nodes;
-  const int b = members[blockIdx.y];
-  const TsneInstance& I = inst[b];
-  float4* __restrict__ potential = I.potential;
-  const int n = I.n;
-  cur += b;
-  arow += (long long)blockIdx.y * nodes * m;
-  brow += (long long)blockIdx.y * nodes * (hm + 1);
-  zpart += (long long)blockIdx.y * zblocks;
-  const float2* a1 = arow + (long long)r1 * m;
-  const float2* a2 = arow + (long long)r2 * m;
-  const float2* b1 = brow + (long long)r1 * (hm + 1);
-  const float2* b2 = brow + (long long)r2 * (hm + 1);
-  for (int f = threadIdx.x; f < m; f += blockDim.x) {
-    const int p = bitrev(f, logm);
-    sbuf[sidx(p)] = a1[f];
-    sbuf[sidx(m + p)] = has2 ? a2[f] : make_float2(0.0f, 0.0f);
-    // full spectra of the two real B rows from their halves, packed as X1 + i X2
-    const float2 x1 = f <= hm ? b1[f] : conjf2(b1[m - f]);
-    const float2 x2 = has2 ? (f <= hm ? b2[f] : conjf2(b2[m - f])) : make_float2(0.0f, 0.0f);
-    sbuf[sidx(2 * m + p)] = make_float2(x1.x - x2.y, x1.y + x2.x);
-  }
-  __syncthreads();
-  fft_dit(sbuf, 3, logm, tw, true);
-  const float scale = 1.0f / ((float)m * (float)m);
-  float4* o1 = potential + (long long)r1 * grid;
-  float4* o2 = potential + (long long)r2 * grid;
-  for (int c = threadIdx.x; c < nodes; c += blockDim.x) {
-    const float2 q1 = sbuf[sidx(c)], pb = sbuf[sidx(2 * m + c)];
-    o1[c] = make_float4(pb.x * scale, q1.x * scale, q1.y * scale, 0.0f);
-    if (has2) {
-      const float2 q2 = sbuf[sidx(m + c)];
-      o2[c] = make_float4(pb.y * scale, q2.x * scale, q2.y * scale, 0.0f);
-    }
-  }
-  if (r1 == 0) {
-    __shared__ double s_z[kFftThreads];
-    double z = 0.0;
-    for (int t = threadIdx.x; t < zblocks; t += blockDim.x) z += zpart[t];
-    s_z[threadIdx.x] = z;
-    __syncthreads();
-    for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-      if ((int)threadIdx.x < w) s_z[threadIdx.x] += s_z[threadIdx.x + w];
-      __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-      const double zz = s_z[0] / ((double)m * (double)m) - (double)n;
-      cur->z = zz;
-      cur->inv_z = (float)(1.0 / fmax(zz, (double)FLT_MIN));
     }
   }
 }
@@ -1376,24 +852,22 @@ void build_grid_classes(TsneDevice& d, const std::vector<int>& grids) {
     k.fft = 2 * k.grid;
     k.log_fft = log2_ceil(k.fft);
     k.count = (int)members[c].size();
-    k.col_blocks = k.fft / 2 + 1;
-    const std::size_t m = k.fft;
+    fft_class_layout(k);
+    const std::size_t m = k.fft, ld = k.ld;
     d.grid_arena.reserve(&k.charges, (std::size_t)k.count * k.grid * k.grid * kChargeStride);
     d.grid_arena.reserve(&k.potential, (std::size_t)k.count * k.grid * k.grid);
-    d.grid_arena.reserve(&k.arow, (std::size_t)k.count * k.nodes * m);
-    d.grid_arena.reserve(&k.brow, (std::size_t)k.count * k.nodes * (m / 2 + 1));
-    d.grid_arena.reserve(&k.krow, (std::size_t)k.count * k.nodes * (m / 2 + 1));
-    d.grid_arena.reserve(&k.twiddle, m / 2);
+    d.grid_arena.reserve(&k.arow, (std::size_t)k.count * ld * m);
+    d.grid_arena.reserve(&k.brow, (std::size_t)k.count * ld * (m / 2 + 1));
+    d.grid_arena.reserve(&k.krow, (std::size_t)k.count * ld * (m / 2 + 1));
+    d.grid_arena.reserve(&k.twiddle, k.twiddles);
     d.grid_arena.reserve(&k.zpart, (std::size_t)k.count * k.col_blocks);
   }
   d.grid_arena.commit("t-SNE grid workspaces");
   std::vector<int> flat;
-  int max_m = 0, max_grid = 0;
+  int max_grid = 0;
   for (std::size_t c = 0; c < distinct.size(); ++c) {
     GridClass& k = d.classes[c];
     k.members = d_members + flat.size();
-    const int m = k.fft;
-    max_m = std::max(max_m, m);
     max_grid = std::max(max_grid, k.grid);
     for (int j = 0; j < k.count; ++j) {
       const int b = members[c][j];
@@ -1404,11 +878,7 @@ void build_grid_classes(TsneDevice& d, const std::vector<int>& grids) {
       I.charges = k.charges + (std::size_t)j * k.grid * k.grid * kChargeStride;
       I.potential = k.potential + (std::size_t)j * k.grid * k.grid;
     }
-    std::vector<float2> tw(m / 2);
-    for (int t = 0; t < m / 2; ++t) {
-      const double ang = -2.0 * M_PI * (double)t / (double)m;
-      tw[t] = make_float2((float)std::cos(ang), (float)std::sin(ang));
-    }
+    const std::vector<float2> tw = fft_class_twiddles(k);
     FE_CUDA(cudaMemcpy(k.twiddle, tw.data(), sizeof(float2) * tw.size(), cudaMemcpyHostToDevice));
     FE_CUDA(cudaMemset(k.charges, 0, sizeof(long long) * kChargeStride * (std::size_t)k.count * k.grid * k.grid));
     FE_CUDA(cudaMemset(k.potential, 0, sizeof(float4) * (std::size_t)k.count * k.grid * k.grid));
@@ -1419,11 +889,6 @@ void build_grid_classes(TsneDevice& d, const std::vector<int>& grids) {
   d.key_bits = 2 * log2_ceil(max_grid);
   d.sort_bits = d.key_bits + log2_ceil(ninst);
   if (d.sort_bits > 32) throw Error("t-SNE batch: too many instances for the spatial sort key");
-  const int big = padded(4 * max_m) * (int)sizeof(float2);
-  FE_CUDA(cudaFuncSetAttribute(columns_convolve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-  const int rowb = padded(3 * max_m) * (int)sizeof(float2);
-  FE_CUDA(cudaFuncSetAttribute(rows_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, rowb));
-  FE_CUDA(cudaFuncSetAttribute(rows_inverse_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, rowb));
 }
 }  // namespace
 
@@ -1542,19 +1007,7 @@ void tsne_grid_stage(TsneDevice& d, cudaStream_t s) {
   else
     scatter_kernel<3><<<d.nblocks, kPointBlock, 0, s>>>(d.y, d.d_inst, d.blocks, d.cur, d.next);
   FE_LAUNCH("scatter_kernel");
-  for (const GridClass& c : d.classes) {
-    const int m = c.fft;
-    const int npairs = (c.nodes + 1) / 2;
-    rows_forward_kernel<<<dim3(2 * npairs, c.count), kFftThreads, padded(3 * m) * sizeof(float2), s>>>(
-        d.d_inst, c.members, c.grid, c.nodes, c.log_fft, c.twiddle, d.cur, c.arow, c.brow, c.krow);
-    FE_LAUNCH("rows_forward_kernel");
-    columns_convolve_kernel<<<dim3(c.col_blocks, c.count), kColThreads, padded(4 * m) * sizeof(float2), s>>>(
-        c.arow, c.brow, c.krow, c.nodes, c.log_fft, c.twiddle, c.zpart);
-    FE_LAUNCH("columns_convolve_kernel");
-    rows_inverse_kernel<<<dim3(npairs, c.count), kFftThreads, padded(3 * m) * sizeof(float2), s>>>(
-        c.arow, c.brow, d.d_inst, c.members, c.grid, c.nodes, c.log_fft, c.twiddle, c.zpart, c.col_blocks, d.cur);
-    FE_LAUNCH("rows_inverse_kernel");
-  }
+  fft_convolve(d, s);
 }
 
 void tsne_bind_rows(TsneDevice& d, const DeviceCsr& P, cudaStream_t s) {

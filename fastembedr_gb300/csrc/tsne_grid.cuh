@@ -57,12 +57,16 @@ struct GridClass {
   int grid = 0, nodes = 0, fft = 0, log_fft = 0;
   int count = 0;
   int* members = nullptr;     // device: the class's instance indices
-  int col_blocks = 0;          // M / 2 + 1 conjugate column pairs
-  float2* arow = nullptr;      // count x (nodes x M): row spectra of A = x-charge + i y-charge
-  float2* brow = nullptr;      // count x (nodes x (M/2 + 1)): half row spectra of the mass plane
-  float2* krow = nullptr;      // count x (nodes x (M/2 + 1)): row spectra of the kernel (q + i q^2)
+  int ld = 0;                  // rows of a column of the spectra: nodes rounded up to even
+  int col_blocks = 0;          // blocks of the column pass
+  int twiddles = 0;
+  // Row spectra, stored column by column (all rows of a frequency consecutive: the column pass
+  // reads and writes consecutive addresses, the row passes 16 bytes for a pair of rows).
+  float2* arow = nullptr;      // count x (M x ld): row spectra of A = x-charge + i y-charge
+  float2* brow = nullptr;      // count x ((M/2 + 1) x ld): half row spectra of the mass plane
+  float2* krow = nullptr;      // count x ((M/2 + 1) x ld): row spectra of the kernel (q + i q^2)
   double* zpart = nullptr;     // count x col_blocks
-  float2* twiddle = nullptr;  // M / 2 forward twiddles
+  float2* twiddle = nullptr;   // twiddle tables of the class's transform length
   long long* charges = nullptr;  // count x G x G x kChargeStride
   float4* potential = nullptr;
 };
@@ -166,5 +170,11 @@ void tsne_finalize(TsneDevice& d, float* d_out, cudaStream_t s);
 void tsne_forces(TsneDevice& d, const DeviceCsr& P, float exaggeration, float* d_attr, float* d_rep,
                  cudaStream_t s);
 int tsne_launches_per_iteration(const TsneDevice& d);
+
+// FFT convolution of the charges with q and q^2 (tsne_fft.cu): three launches per grid class.
+// fft_class_layout fills ld, col_blocks and twiddles from the class's G and nodes.
+void fft_class_layout(GridClass& k);
+std::vector<float2> fft_class_twiddles(const GridClass& k);
+void fft_convolve(TsneDevice& d, cudaStream_t s);
 
 }  // namespace fe
