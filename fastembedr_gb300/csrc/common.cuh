@@ -121,11 +121,13 @@ __device__ __forceinline__ Float2Sum two_sum(float a, float b) {
 }
 __device__ __forceinline__ Float2Sum add(Float2Sum a, Float2Sum b) {
   const Float2Sum s = two_sum(a.hi, b.hi);
-  const float lo = __fadd_rn(s.lo, __fadd_rn(a.lo, b.lo));
+  // an infinite sum keeps no low part (its residual would be NaN)
+  const float lo = isfinite(s.hi) ? __fadd_rn(s.lo, __fadd_rn(a.lo, b.lo)) : 0.0f;
   const float hi = __fadd_rn(s.hi, lo);  // |lo| is far below |s.hi|: renormalise
   return Float2Sum{hi, __fsub_rn(lo, __fsub_rn(hi, s.hi))};
 }
 __device__ __forceinline__ Float2Sum add(Float2Sum a, float b) { return add(a, Float2Sum{b, 0.0f}); }
+// hi is rounded to nearest, so lo is at most half a unit of hi's last place
 __device__ __forceinline__ double value(Float2Sum a) { return (double)a.hi + (double)a.lo; }
 __device__ __forceinline__ Float2Sum warp_sum(Float2Sum v) {
 #pragma unroll

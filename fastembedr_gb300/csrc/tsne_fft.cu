@@ -274,20 +274,31 @@ rows_inverse_kernel(const float2* __restrict__ arow, const float2* __restrict__ 
   float4* __restrict__ potential = inst[b].potential;
   arow += (long long)blockIdx.y * M * ld;
   brow += (long long)blockIdx.y * (HM + 1) * ld;
-  for (int t = threadIdx.x; t < NP * M; t += THREADS) {
-    const int q = t % NP, p = t / NP, f = bitrev(p, LOGM);
-    if (pair0 + q >= npairs) continue;
-    const bool two = pair0 + q + npairs < nodes;  // the column pass writes `nodes` rows
-    const long long at = (long long)f * ld + 2 * (pair0 + q);
-    float2* S = sbuf + 3 * q * M;
-    const float4 a = *reinterpret_cast<const float4*>(arow + at);
-    S[P::slot(p)] = make_float2(a.x, a.y);
-    S[M + P::slot(p)] = two ? make_float2(a.z, a.w) : make_float2(0.0f, 0.0f);
-    if (f <= HM) {
-      float4 x = *reinterpret_cast<const float4*>(brow + at);
-      if (!two) x.z = x.w = 0.0f;
-      S[2 * M + P::slot(p)] = make_float2(x.x - x.w, x.y + x.z);
-      if (f > 0 && f < HM) S[2 * M + P::slot(bitrev(M - f, LOGM))] = make_float2(x.x + x.w, x.z - x.y);
+  // in batches whose loads are all in flight before the first is stored
+  constexpr int U = 4;
+  for (int t0 = threadIdx.x; t0 < NP * M; t0 += U * THREADS) {
+    float4 a[U], x[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int t = t0 + u * THREADS, q = t % NP, f = bitrev(t / NP, LOGM);
+      if (t >= NP * M || pair0 + q >= npairs) continue;
+      const long long at = (long long)f * ld + 2 * (pair0 + q);
+      a[u] = __ldg(reinterpret_cast<const float4*>(arow + at));
+      if (f <= HM) x[u] = __ldg(reinterpret_cast<const float4*>(brow + at));
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int t = t0 + u * THREADS, q = t % NP, p = t / NP, f = bitrev(p, LOGM);
+      if (t >= NP * M || pair0 + q >= npairs) continue;
+      const bool two = pair0 + q + npairs < nodes;  // the column pass writes `nodes` rows
+      float2* S = sbuf + 3 * q * M;
+      S[P::slot(p)] = make_float2(a[u].x, a[u].y);
+      S[M + P::slot(p)] = two ? make_float2(a[u].z, a[u].w) : make_float2(0.0f, 0.0f);
+      if (f <= HM) {
+        if (!two) x[u].z = x[u].w = 0.0f;
+        S[2 * M + P::slot(p)] = make_float2(x[u].x - x[u].w, x[u].y + x[u].z);
+        if (f > 0 && f < HM) S[2 * M + P::slot(bitrev(M - f, LOGM))] = make_float2(x[u].x + x[u].w, x[u].z - x[u].y);
+      }
     }
   }
   __syncthreads();

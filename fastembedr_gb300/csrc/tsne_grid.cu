@@ -67,8 +67,7 @@ __device__ __forceinline__ Stencil<TAPS> make_stencil(float x, float x0, float i
 // (the bounding-square rule of src/tsne_neighbors.cpp:1168-1184).
 __device__ void finish_layout_stats(const StepPartial* __restrict__ part, int nblocks, int n, int grid, int mode,
                                     GridState* __restrict__ next) {
-  __shared__ float s_min_x[kStepThreads], s_max_x[kStepThreads], s_min_y[kStepThreads], s_max_y[kStepThreads];
-  __shared__ double s_sx[kStepThreads], s_sy[kStepThreads];
+  __shared__ StepPartial s_stat[kStepThreads / 32];
   float mnx = FLT_MAX, mxx = -FLT_MAX, mny = FLT_MAX, mxy = -FLT_MAX;
   double sx = 0.0, sy = 0.0;
   // partials written by the other blocks of this launch: read through L2, eight loads in flight
@@ -83,26 +82,28 @@ __device__ void finish_layout_stats(const StepPartial* __restrict__ part, int nb
     sx += ss.x;
     sy += ss.y;
   }
-  s_min_x[threadIdx.x] = mnx;
-  s_max_x[threadIdx.x] = mxx;
-  s_min_y[threadIdx.x] = mny;
-  s_max_y[threadIdx.x] = mxy;
-  s_sx[threadIdx.x] = sx;
-  s_sy[threadIdx.x] = sy;
-  __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if ((int)threadIdx.x < w) {
-      s_min_x[threadIdx.x] = fminf(s_min_x[threadIdx.x], s_min_x[threadIdx.x + w]);
-      s_max_x[threadIdx.x] = fmaxf(s_max_x[threadIdx.x], s_max_x[threadIdx.x + w]);
-      s_min_y[threadIdx.x] = fminf(s_min_y[threadIdx.x], s_min_y[threadIdx.x + w]);
-      s_max_y[threadIdx.x] = fmaxf(s_max_y[threadIdx.x], s_max_y[threadIdx.x + w]);
-      s_sx[threadIdx.x] += s_sx[threadIdx.x + w];
-      s_sy[threadIdx.x] += s_sy[threadIdx.x + w];
-    }
-    __syncthreads();
+  mnx = warp_min(mnx);
+  mxx = warp_max(mxx);
+  mny = warp_min(mny);
+  mxy = warp_max(mxy);
+  if (nblocks > 1) {
+    sx = warp_sum(sx);
+    sy = warp_sum(sy);
   }
+  if ((threadIdx.x & 31) == 0) s_stat[threadIdx.x >> 5] = StepPartial{mnx, mxx, mny, mxy, sx, sy};
+  __syncthreads();
   if (threadIdx.x == 0) {
-    const float min_x = s_min_x[0], max_x = s_max_x[0], min_y = s_min_y[0], max_y = s_max_y[0];
+    StepPartial p = s_stat[0];
+    // warps without a partial hold the neutral values
+    for (int w = 1; w < (int)(blockDim.x / 32) && w * 32 < nblocks; ++w) {
+      p.min_x = fminf(p.min_x, s_stat[w].min_x);
+      p.max_x = fmaxf(p.max_x, s_stat[w].max_x);
+      p.min_y = fminf(p.min_y, s_stat[w].min_y);
+      p.max_y = fmaxf(p.max_y, s_stat[w].max_y);
+      p.sum_x += s_stat[w].sum_x;
+      p.sum_y += s_stat[w].sum_y;
+    }
+    const float min_x = p.min_x, max_x = p.max_x, min_y = p.min_y, max_y = p.max_y;
     GridState g;
     g.cx = 0.5f * (min_x + max_x);
     g.cy = 0.5f * (min_y + max_y);
@@ -123,8 +124,8 @@ __device__ void finish_layout_stats(const StepPartial* __restrict__ part, int nb
     }
     g.inv_h = 1.0f / g.h;
     g.inv_box = 1.0f / g.box;
-    g.mean_x = s_sx[0] / (double)n;
-    g.mean_y = s_sy[0] / (double)n;
+    g.mean_x = p.sum_x / (double)n;
+    g.mean_y = p.sum_y / (double)n;
     g.z = 0.0;
     g.inv_z = 0.0f;
     // |mass| and |mass * d| summed over any subset of points stay below 1.5625 n max(half, 1)
@@ -147,29 +148,40 @@ __device__ void finish_layout_stats(const StepPartial* __restrict__ part, int nb
   }
 }
 
-__device__ __forceinline__ void block_partial(float mnx, float mxx, float mny, float mxy, double sx, double sy,
+// Statistics of the block's points (one per thread). The coordinate sums are kept in two floats, within
+// 2^-47 of the sum of magnitudes (256 floats of similar size add up exactly), and go on in FP64
+// from the partials; with FP64 warp sums the update took 52 us at 1M points.
+__device__ __forceinline__ void block_partial(float mnx, float mxx, float mny, float mxy, float sx, float sy,
                                               StepPartial* out) {
-  __shared__ StepPartial s_part[kStepThreads / 32];
+  __shared__ float4 s_box[kStepThreads / 32];
+  __shared__ Float2Sum s_sum[kStepThreads / 32][2];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   mnx = warp_min(mnx);
   mxx = warp_max(mxx);
   mny = warp_min(mny);
   mxy = warp_max(mxy);
-  sx = warp_sum(sx);
-  sy = warp_sum(sy);
-  if (lane == 0) s_part[warp] = StepPartial{mnx, mxx, mny, mxy, sx, sy};
+  const Float2Sum wx = warp_sum(Float2Sum{sx, 0.0f}), wy = warp_sum(Float2Sum{sy, 0.0f});
+  if (lane == 0) {
+    s_box[warp] = make_float4(mnx, mxx, mny, mxy);
+    s_sum[warp][0] = wx;
+    s_sum[warp][1] = wy;
+  }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    StepPartial p = s_part[0];
-    for (int w = 1; w < (int)(blockDim.x / 32); ++w) {
-      p.min_x = fminf(p.min_x, s_part[w].min_x);
-      p.max_x = fmaxf(p.max_x, s_part[w].max_x);
-      p.min_y = fminf(p.min_y, s_part[w].min_y);
-      p.max_y = fmaxf(p.max_y, s_part[w].max_y);
-      p.sum_x += s_part[w].sum_x;
-      p.sum_y += s_part[w].sum_y;
+  if (warp == 0) {
+    constexpr int W = kStepThreads / 32;
+    const float4 b = s_box[lane & (W - 1)];
+    float4 r = b;
+    Float2Sum x = s_sum[lane & (W - 1)][0], y = s_sum[lane & (W - 1)][1];
+#pragma unroll
+    for (int o = W / 2; o > 0; o >>= 1) {
+      r.x = fminf(r.x, __shfl_xor_sync(0xffffffffu, r.x, o));
+      r.y = fmaxf(r.y, __shfl_xor_sync(0xffffffffu, r.y, o));
+      r.z = fminf(r.z, __shfl_xor_sync(0xffffffffu, r.z, o));
+      r.w = fmaxf(r.w, __shfl_xor_sync(0xffffffffu, r.w, o));
+      x = add(x, Float2Sum{__shfl_xor_sync(0xffffffffu, x.hi, o), __shfl_xor_sync(0xffffffffu, x.lo, o)});
+      y = add(y, Float2Sum{__shfl_xor_sync(0xffffffffu, y.hi, o), __shfl_xor_sync(0xffffffffu, y.lo, o)});
     }
-    *out = p;
+    if (lane == 0) *out = StepPartial{r.x, r.y, r.z, r.w, value(x), value(y)};
   }
 }
 
@@ -198,8 +210,7 @@ layout_stats_kernel(const float2* __restrict__ ynew, const TsneInstance* __restr
   const int2 bl = blocks[blockIdx.x];
   const TsneInstance I = inst[bl.x];
   const int i = bl.y + threadIdx.x;
-  float mnx = FLT_MAX, mxx = -FLT_MAX, mny = FLT_MAX, mxy = -FLT_MAX;
-  double sx = 0.0, sy = 0.0;
+  float mnx = FLT_MAX, mxx = -FLT_MAX, mny = FLT_MAX, mxy = -FLT_MAX, sx = 0.0f, sy = 0.0f;
   if (i < I.pt_begin + I.n) {
     const float2 p = ynew[i];
     mnx = mxx = p.x;
@@ -636,9 +647,20 @@ __global__ void __launch_bounds__(kStepThreads)
 update_kernel(float2* __restrict__ y, const float2* __restrict__ attr, float2* __restrict__ gains,
               float2* __restrict__ update, const TsneInstance* __restrict__ inst, const int2* __restrict__ blocks,
               const GridState* __restrict__ cur, GridState* __restrict__ next, StepPartial* __restrict__ part,
-              unsigned* __restrict__ counter, int mode, float lr, float mom, float min_gain, float max_step,
+              unsigned* __restrict__ counter, int n, int mode, float lr, float mom, float min_gain, float max_step,
               float2* __restrict__ out_rep) {
   const int2 bl = blocks[blockIdx.x];
+  const int i = bl.y + threadIdx.x;
+  // the point's state is requested beside the instance and grid records (clamped: the last block of
+  // the last instance may reach past the end)
+  const int ic = min(i, n - 1);
+  const float2 p = y[ic];
+  float2 a = make_float2(0.0f, 0.0f), ga = a, up = a;
+  if constexpr (!DIAG) {
+    a = attr[ic];
+    ga = gains[ic];
+    up = update[ic];
+  }
   const TsneInstance I = inst[bl.x];
   const GridState g = cur[bl.x];
   const float4* __restrict__ pot = I.potential;
@@ -646,20 +668,17 @@ update_kernel(float2* __restrict__ y, const float2* __restrict__ attr, float2* _
   const float lr_i = lr * I.lr_mult;
   const bool clip = isfinite(max_step) && max_step > 0.0f;
   const float max2 = max_step * max_step;
-  float mnx = FLT_MAX, mxx = -FLT_MAX, mny = FLT_MAX, mxy = -FLT_MAX;
-  double sx = 0.0, sy = 0.0;
-  const int i = bl.y + threadIdx.x;
+  float mnx = FLT_MAX, mxx = -FLT_MAX, mny = FLT_MAX, mxy = -FLT_MAX, sx = 0.0f, sy = 0.0f;
   if (i < I.pt_begin + I.n) {
-    const float2 p = y[i];
     const Stencil<TAPS> stx = make_stencil<TAPS>(p.x, g.x0, g.inv_h, g.inv_box, g.nodes);
     const Stencil<TAPS> sty = make_stencil<TAPS>(p.y, g.y0, g.inv_h, g.inv_box, g.nodes);
     float r0 = 0.0f, r1 = 0.0f, r2 = 0.0f;
 #pragma unroll
-    for (int a = 0; a < TAPS; ++a) {
-      const float4* row = pot + (long long)(sty.base + a) * grid + stx.base;
+    for (int v = 0; v < TAPS; ++v) {
+      const float4* row = pot + (long long)(sty.base + v) * grid + stx.base;
 #pragma unroll
       for (int b = 0; b < TAPS; ++b) {
-        const float w = sty.w[a] * stx.w[b];
+        const float w = sty.w[v] * stx.w[b];
         const float4 f = __ldg(row + b);
         r0 += w * f.x;
         r1 += w * f.y;
@@ -671,9 +690,7 @@ update_kernel(float2* __restrict__ y, const float2* __restrict__ attr, float2* _
     if constexpr (DIAG) {
       out_rep[i] = make_float2(repx, repy);
     } else {
-      const float2 a = attr[i];
       const float gx = repx + a.x, gy = repy + a.y;
-      const float2 ga = gains[i], up = update[i];
       float gnx = sign3(up.x) != sign3(gx) ? ga.x + 0.2f : ga.x * 0.8f + min_gain;
       float gny = sign3(up.y) != sign3(gy) ? ga.y + 0.2f : ga.y * 0.8f + min_gain;
       if (gnx < min_gain) gnx = min_gain;
@@ -1072,11 +1089,11 @@ bool tsne_tune_attractive(TsneDevice& d, const DeviceCsr& P, float exag, cudaStr
 void tsne_update_stage(TsneDevice& d, float lr, float mom, float min_gain, float max_step, cudaStream_t s) {
   if (d.mode == kInterpBilinear)
     update_kernel<2, false><<<d.nblocks, kStepThreads, 0, s>>>(d.y, d.attr, d.gains, d.update, d.d_inst, d.blocks,
-                                                                d.cur, d.next, d.partial, d.counter, d.mode, lr, mom,
+                                                                d.cur, d.next, d.partial, d.counter, d.n, d.mode, lr, mom,
                                                                 min_gain, max_step, nullptr);
   else
     update_kernel<3, false><<<d.nblocks, kStepThreads, 0, s>>>(d.y, d.attr, d.gains, d.update, d.d_inst, d.blocks,
-                                                                d.cur, d.next, d.partial, d.counter, d.mode, lr, mom,
+                                                                d.cur, d.next, d.partial, d.counter, d.n, d.mode, lr, mom,
                                                                 min_gain, max_step, nullptr);
   FE_LAUNCH("update_kernel");
 }
@@ -1099,11 +1116,11 @@ void tsne_forces(TsneDevice& d, const DeviceCsr& P, float exag, float* d_attr, f
   float2* r = reinterpret_cast<float2*>(d_rep);
   if (d.mode == kInterpBilinear)
     update_kernel<2, true><<<d.nblocks, kStepThreads, 0, s>>>(d.y, d.attr, d.gains, d.update, d.d_inst, d.blocks,
-                                                               d.cur, d.next, d.partial, d.counter, d.mode, 0.0f,
+                                                               d.cur, d.next, d.partial, d.counter, d.n, d.mode, 0.0f,
                                                                0.0f, 0.0f, 0.0f, r);
   else
     update_kernel<3, true><<<d.nblocks, kStepThreads, 0, s>>>(d.y, d.attr, d.gains, d.update, d.d_inst, d.blocks,
-                                                               d.cur, d.next, d.partial, d.counter, d.mode, 0.0f,
+                                                               d.cur, d.next, d.partial, d.counter, d.n, d.mode, 0.0f,
                                                                0.0f, 0.0f, 0.0f, r);
   FE_LAUNCH("update_kernel(diagnostic)");
 }
