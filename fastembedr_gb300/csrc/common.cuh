@@ -127,6 +127,25 @@ __device__ __forceinline__ Float2Sum add(Float2Sum a, Float2Sum b) {
   return Float2Sum{hi, __fsub_rn(lo, __fsub_rn(hi, s.hi))};
 }
 __device__ __forceinline__ Float2Sum add(Float2Sum a, float b) { return add(a, Float2Sum{b, 0.0f}); }
+__device__ __forceinline__ Float2Sum mul(Float2Sum a, float b) {
+  const float p = __fmul_rn(a.hi, b);
+  return Float2Sum{p, __fmaf_rn(a.lo, b, __fmaf_rn(a.hi, b, -p))};
+}
+__device__ __forceinline__ Float2Sum mul(Float2Sum a, Float2Sum b) {
+  const float p = __fmul_rn(a.hi, b.hi);
+  return Float2Sum{p, __fmaf_rn(a.hi, b.lo, __fmaf_rn(a.lo, b.hi, __fmaf_rn(a.hi, b.hi, -p)))};
+}
+__device__ __forceinline__ Float2Sum split(double v) {
+  const float h = (float)v;
+  return Float2Sum{h, (float)(v - (double)h)};
+}
+// a / b for normal b of moderate size: one Newton step on the quotient of the high parts.
+__device__ __forceinline__ Float2Sum divide(Float2Sum a, Float2Sum b) {
+  const float r = __frcp_rn(b.hi), q = __fmul_rn(a.hi, r);
+  const float res = __fadd_rn(__fmaf_rn(-q, b.hi, a.hi), __fmaf_rn(-q, b.lo, a.lo));
+  const float c = __fmul_rn(res, r), h = __fadd_rn(q, c);
+  return Float2Sum{h, __fadd_rn(c, __fsub_rn(q, h))};
+}
 // hi is rounded to nearest, so lo is at most half a unit of hi's last place
 __device__ __forceinline__ double value(Float2Sum a) { return (double)a.hi + (double)a.lo; }
 __device__ __forceinline__ Float2Sum warp_sum(Float2Sum v) {

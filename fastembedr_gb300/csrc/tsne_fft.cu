@@ -82,7 +82,7 @@ __device__ __forceinline__ void kernel_rows(float2* sbuf, int row0, int nodes, i
 // cleared for the next scatter. A spectra to arow, separated B half spectra to brow, the rows of a
 // pair side by side (places 2 p and 2 p + 1 of a column). blockIdx.y: member of the grid class.
 template <int LOGM>
-__global__ void __launch_bounds__(3 * Blocks<LOGM>::PAIRS* FftPlan<LOGM>::T)
+__global__ void __launch_bounds__(3 * Blocks<LOGM>::PAIRS* FftPlan<LOGM>::T, LOGM == 11 ? 2 : 1)
 rows_forward_kernel(const TsneInstance* __restrict__ inst, const int* __restrict__ members, int grid, int nodes, int ld,
                     const float2* __restrict__ tw, const GridState* __restrict__ cur, int charge_blocks,
                     float2* __restrict__ arow, float2* __restrict__ brow, float2* __restrict__ krow) {
@@ -245,7 +245,7 @@ columns_convolve_kernel(float2* __restrict__ arow, float2* __restrict__ brow, co
 // an instance instead finalises Z = sum_k |F_mass|^2 Kq / M^2 - n (the reference's
 // sum_i q_grid(y_i) - n).
 template <int LOGM>
-__global__ void __launch_bounds__(3 * Blocks<LOGM>::PAIRS* FftPlan<LOGM>::T)
+__global__ void __launch_bounds__(3 * Blocks<LOGM>::PAIRS* FftPlan<LOGM>::T, LOGM == 11 ? 2 : 1)
 rows_inverse_kernel(const float2* __restrict__ arow, const float2* __restrict__ brow,
                     const TsneInstance* __restrict__ inst, const int* __restrict__ members, int grid, int nodes, int ld,
                     const float2* __restrict__ tw, const double* __restrict__ zpart, int zblocks,
