@@ -22,6 +22,7 @@
 
 #include "sort.cuh"
 #include "tsne.cuh"
+#include "twofloat.cuh"
 
 namespace fe {
 
@@ -67,19 +68,32 @@ void validate_knn(const int* d_idx, const float* d_dist, int n, int k, int offse
 // ---------------------------------------------------------------- bisection
 // One thread per row. The CTA stages its rows' distances (column-major in global memory, so
 // each column read is coalesced) in shared memory with a stride of k + 1 floats (consecutive rows
-// on distinct banks), next to each row's shifted squared distances s_j = d_j^2 - min d^2 (FP64,
+// on distinct banks), next to each row's shifted squared distances s_j = d_j^2 - min d^2 (exact,
 // rounded to float once). Every thread bisects its own row: per entry FP32 exp of -beta s_j and
 // compensated (Kahan) FP32 sums, whose error (~1e-7 relative) stays far inside the 1e-6 band
-// around the stop tolerance in which an iteration is re-evaluated from the distances with FP64
-// exp and FP64 sums; entropy, the update of beta and the stop test are FP64. The FP64 pipe of
-// this part is narrow, so the per-entry work stays on the FP32 pipe. The probabilities overwrite
-// the row's distances and the CTA stores them row-major with coalesced writes.
+// around the stop tolerance in which an iteration is re-evaluated from the distances with about
+// 40-bit exponentials and sums. The entropy and its distance from the target are two-float values
+// (about 1e-12), beta is FP64. So the search takes the FP64 search's steps: a decision could differ
+// only within 1e-10 of the stop tolerance, where it is evaluated in FP64. The FP64 pipe is narrow: 90
+// FP64 exponentials of a row in the band, which nearly every warp met, and the 80 FP64 instructions
+// of each step's entropy were four fifths of the time (100,000 rows of 45: 1.19 -> 0.26 ms; the
+// rest is FP32 exp and Kahan sums). The probabilities overwrite the row's distances and the CTA stores
+// them row-major with coalesced writes.
 constexpr int kBisectRows = 128;
+
+__device__ __forceinline__ Float2Sum shifted_square(float d, Float2Sum min2) {
+  const float p = __fmul_rn(d, d);
+  return add(Float2Sum{p, __fmaf_rn(d, d, -p)}, Float2Sum{-min2.hi, -min2.lo});
+}
 
 __global__ void __launch_bounds__(kBisectRows)
 row_probabilities_kernel(const float* __restrict__ dist, int n, int k, double log_perplexity,
                          float* __restrict__ p_out, double* __restrict__ entropy_out) {
   extern __shared__ float tile[];  // blockDim.x rows x (k + 1) distances, then as many s_j
+  __shared__ float2 exp_table[kExpEntries];
+  __shared__ float4 log_table[kLogEntries];
+  fill_exp_table(exp_table);
+  fill_log_table(log_table);
   const int rows = blockDim.x, stride = k + 1;
   float* stile = tile + (long long)rows * stride;
   const int r0 = blockIdx.x * rows;
@@ -93,14 +107,12 @@ row_probabilities_kernel(const float* __restrict__ dist, int n, int k, double lo
   if (rr < nrows) {
     float* d = tile + rr * stride;
     // zero-spread test in float arithmetic, as compute_row_probabilities_float does it
-    float min_f = FLT_MAX, max_f = 0.0f;
-    double min_d2 = DBL_MAX;
+    float min_f = FLT_MAX, max_f = 0.0f, min_d = FLT_MAX;
     for (int j = 0; j < k; ++j) {
       const float df = d[j] * d[j];
       min_f = fminf(min_f, df);
       max_f = fmaxf(max_f, df);
-      const double dj = d[j];
-      min_d2 = fmin(min_d2, dj * dj);  // exact: a float squared fits in a double
+      min_d = fminf(min_d, d[j]);  // distances are not negative
     }
     double entropy_eval;
     if (max_f - min_f <= FLT_EPSILON * fmaxf(1.0f, max_f)) {
@@ -109,16 +121,21 @@ row_probabilities_kernel(const float* __restrict__ dist, int n, int k, double lo
       entropy_eval = log((double)k);
     } else {
       float* sf = stile + rr * stride;
-      for (int j = 0; j < k; ++j) {
-        const double dj = d[j];
-        sf[j] = (float)(dj * dj - min_d2);
-      }
+      const float m2 = __fmul_rn(min_d, min_d);
+      const Float2Sum min2{m2, __fmaf_rn(min_d, min_d, -m2)};
+      // squares near the smallest floats have no room for a low part: FP64 for such a row
+      const bool tiny = max_f < 1.0e-28f;
+      const double dmin2 = (double)min_d * (double)min_d;
+      for (int j = 0; j < k; ++j)
+        sf[j] = tiny ? (float)((double)d[j] * (double)d[j] - dmin2) : shifted_square(d[j], min2).hi;
+      const Float2Sum target = split(-log_perplexity);
       double beta = 1.0, beta_min = -DBL_MAX, beta_max = DBL_MAX;
-      double beta_eval = beta, sum_eval = 1.0;
+      double beta_eval = beta;
+      Float2Sum sum_eval{1.0f, 0.0f}, ent{0.0f, 0.0f};
       bool exact_eval = false;
-      entropy_eval = 0.0;
       for (int it = 0; it < 200; ++it) {
         const float nb = (float)(-beta);
+        const Float2Sum b2 = split(beta);
         float ps = 0.0f, pc = 0.0f, ws = 0.0f, wc = 0.0f;
         for (int j = 0; j < k; ++j) {
           const float sj = sf[j];
@@ -132,32 +149,38 @@ row_probabilities_kernel(const float* __restrict__ dist, int n, int k, double lo
           wc = (tw - ws) - yw;
           ws = tw;
         }
-        double sp = (double)ps - (double)pc;
-        double sw = (double)ws - (double)wc;
-        double entropy = beta * sw / sp + log(sp);
-        double diff = entropy - log_perplexity;
+        Float2Sum sp = two_sum(ps, -pc), sw = two_sum(ws, -wc);
+        ent = add(divide(mul(sw, b2), sp), log_two(sp, log_table));
+        Float2Sum diff = add(ent, target);
         exact_eval = false;
-        // The stop test is the only decision FP32 exp can flip: re-evaluate near its boundary
-        // with FP64 exp so the bisection follows the FP64 path.
-        if (fabs(fabs(diff) - 1e-5) < 1e-6) {
-          sp = 0.0;
-          sw = 0.0;
+        // The stop test is the only decision FP32 exp can flip: re-evaluate near its boundary.
+        if (fabsf(fabsf(diff.hi) - 1e-5f) < 1e-6f) {
+          sp = sw = Float2Sum{0.0f, 0.0f};
           for (int j = 0; j < k; ++j) {
-            const double dj = d[j];
-            const double s = dj * dj - min_d2;
-            const double p = exp(-beta * s);
-            sp += p;
-            sw += s * p;
+            const Float2Sum s = shifted_square(d[j], min2);
+            const Float2Sum p = exp_two(mul(s, Float2Sum{-b2.hi, -b2.lo}), exp_table);
+            sp = add(sp, p);
+            sw = add(sw, mul(s, p));
           }
-          entropy = beta * sw / sp + log(sp);
-          diff = entropy - log_perplexity;
+          ent = add(divide(mul(sw, b2), sp), log_two(sp, log_table));
+          diff = add(ent, target);
           exact_eval = true;
         }
         beta_eval = beta;
         sum_eval = sp;
-        entropy_eval = entropy;
-        if (fabs(diff) < 1e-5) break;
-        if (diff > 0.0) {
+        double dd = value(diff);
+        if (exact_eval && (tiny || fabs(fabs(dd) - 1e-5) < 1e-10)) {
+          double xp = 0.0, xw = 0.0;
+          for (int j = 0; j < k; ++j) {
+            const double s = (double)d[j] * (double)d[j] - dmin2, p = exp(-beta * s);
+            xp += p;
+            xw += s * p;
+          }
+          dd = beta * xw / xp + log(xp) - log_perplexity;
+          sum_eval = split(xp);
+        }
+        if (fabs(dd) < 1e-5) break;
+        if (dd > 0.0) {
           beta_min = beta;
           beta = (beta_max == DBL_MAX) ? beta * 2.0 : 0.5 * (beta + beta_max);
         } else {
@@ -166,12 +189,17 @@ row_probabilities_kernel(const float* __restrict__ dist, int n, int k, double lo
         }
         if (!isfinite(beta)) break;
       }
-      const double inv = 1.0 / sum_eval;
+      entropy_eval = value(ent);
+      const Float2Sum inv = divide(Float2Sum{1.0f, 0.0f}, sum_eval);
       const float nb = (float)(-beta_eval);
+      const Float2Sum b2 = split(-beta_eval);
       for (int j = 0; j < k; ++j) {
-        const double dj = d[j];
-        const double p = exact_eval ? exp(-beta_eval * (dj * dj - min_d2)) : (double)expf(nb * sf[j]);
-        d[j] = (float)(p * inv);
+        Float2Sum p{0.0f, 0.0f};
+        if (!exact_eval) p.hi = expf(nb * sf[j]);
+        else if (tiny) p = split(exp(-beta_eval * ((double)d[j] * (double)d[j] - dmin2)));
+        else p = exp_two(mul(shifted_square(d[j], min2), b2), exp_table);
+        const Float2Sum v = mul(inv, p);
+        d[j] = __fadd_rn(v.hi, v.lo);
       }
     }
     if (entropy_out) entropy_out[r0 + rr] = entropy_eval;

@@ -1,12 +1,14 @@
 // Exact O(n^2) t-SNE quantities on the GPU: repulsive forces with the all-pairs Z, and the
 // KL divergence of evaluate_kl_f (fastEmbedR src/tsne_neighbors.cpp:1034-1059, :1338-1365).
-// Pair terms are FP32; each thread accumulates a tile of 1024 partners in FP32 and folds the
-// tile into FP64, so the n^2 sums carry FP64 error at N = 1M (5e11 pairs).
+// Pair terms are FP32; the forces accumulate tiles of 1024 partners in FP32 and fold them into FP64, the
+// normaliser folds 128 partners into two-float sums, so the n^2 sums at N = 1M (5e11 pairs) carry no more
+// than the FP32 error of a tile.
 #include <algorithm>
 #include <cfloat>
 #include <cmath>
 
 #include "tsne_exact.cuh"
+#include "twofloat.cuh"
 
 namespace fe {
 
@@ -179,39 +181,6 @@ __global__ void reduce_double_kernel(const double* __restrict__ v, int n, double
     __syncthreads();
   }
   if (threadIdx.x == 0) *out = part[0];
-}
-
-// Natural logarithm in two floats (absolute error about 1e-12), the table method of Tang (1990): x = 2^e m
-// with m in [2/3, 4/3), r a tabulated reciprocal of m's neighbourhood, log x = e log 2 - log r +
-// log1p(m r - 1), |m r - 1| < 0.007. The table is (r, -log r high, low, 0) for m = (kLogFirst + i) / 128.
-constexpr int kLogFirst = 85, kLogEntries = 87;
-__device__ __forceinline__ void fill_log_table(float4* t) {
-  for (int i = threadIdx.x; i < kLogEntries; i += blockDim.x) {
-    const float r = 128.0f / (float)(kLogFirst + i);
-    const Float2Sum l = split(-log((double)r));
-    t[i] = make_float4(r, l.hi, l.lo, 0.0f);
-  }
-}
-__device__ __forceinline__ Float2Sum log_two(Float2Sum x, const float4* __restrict__ table) {
-  const int bits = __float_as_int(x.hi);
-  const int e = (bits - 0x3f2aaaab) >> 23;  // x.hi = 2^e m, m in [2/3, 4/3)
-  const float scale = __int_as_float((127 - e) << 23);
-  const float m = x.hi * scale, ml = x.lo * scale;
-  // (clamped: a NaN must not index outside the table)
-  const float4 t = table[min(max(__float2int_rn(m * 128.0f) - kLogFirst, 0), kLogEntries - 1)];
-  const float p = __fmul_rn(m, t.x);
-  const float z = __fsub_rn(p, 1.0f);  // exact
-  const float zl = __fadd_rn(__fmaf_rn(m, t.x, -p), __fmul_rn(ml, t.x));
-  // log1p(z + zl) = z + zl - z^2 / 2 - z zl + z^3 / 3 - ...
-  const float w = __fmul_rn(z, z), wl = __fmaf_rn(z, z, -w);
-  const float poly = __fmul_rn(__fmul_rn(w, z), __fmaf_rn(z, __fmaf_rn(z, __fmaf_rn(z, -1.0f / 6.0f, 0.2f), -0.25f),
-                                                          1.0f / 3.0f));
-  // log 2 = 0.693145751953125 (16 bits: e times it is exact) + 1.42860676533018e-6
-  Float2Sum s = two_sum((float)e * 0.693145751953125f, t.y);
-  const Float2Sum u = two_sum(s.hi, z), v = two_sum(u.hi, -0.5f * w);
-  const float lo = s.lo + u.lo + v.lo + t.z + zl - 0.5f * wl - z * zl + poly + (float)e * 1.42860676533018e-6f;
-  s = two_sum(v.hi, lo);
-  return s;
 }
 
 // KL = sum_CSR p log((p + 1e-9) / (q / Z + 1e-9)); Z rounded to float as the reference keeps it.
