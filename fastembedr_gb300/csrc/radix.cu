@@ -7,19 +7,20 @@
 namespace fe {
 
 constexpr int kRadixThreads = 256;
-constexpr int kRadixItems = 16;
-constexpr int kRadixTile = kRadixThreads * kRadixItems;
 constexpr int kRadixWarps = kRadixThreads / 32;
+// Keys per thread, each a serial round of a tile: 4 while that many tiles are few (a tile of 16 rounds
+// took 27 us however small the input; 4: 8 us), 16 beyond, where 256 counters a tile would cost more.
+int radix_items(int n) { return n <= (1 << 18) ? 4 : 16; }
 
-int radix_sort_blocks(int n) { return std::max(1, ceil_div(n, kRadixTile)); }
+int radix_sort_blocks(int n) { return std::max(1, ceil_div(n, kRadixThreads * radix_items(n))); }
 
 __global__ void __launch_bounds__(kRadixThreads)
-radix_hist_kernel(const unsigned* __restrict__ keys, int n, int shift, int* __restrict__ hist) {
+radix_hist_kernel(const unsigned* __restrict__ keys, int n, int items, int shift, int* __restrict__ hist) {
   __shared__ int cnt[256];
   cnt[threadIdx.x] = 0;
   __syncthreads();
-  const int base = blockIdx.x * kRadixTile;
-  for (int t = threadIdx.x; t < kRadixTile; t += kRadixThreads) {
+  const int tile = kRadixThreads * items, base = blockIdx.x * tile;
+  for (int t = threadIdx.x; t < tile; t += kRadixThreads) {
     const int i = base + t;
     if (i < n) atomicAdd(&cnt[(keys[i] >> shift) & 255u], 1);
   }
@@ -28,14 +29,14 @@ radix_hist_kernel(const unsigned* __restrict__ keys, int n, int shift, int* __re
 }
 
 __global__ void __launch_bounds__(kRadixThreads)
-radix_scatter_kernel(const unsigned* __restrict__ keys, const int* __restrict__ vals, int n, int shift,
+radix_scatter_kernel(const unsigned* __restrict__ keys, const int* __restrict__ vals, int n, int items, int shift,
                      const long long* __restrict__ offs, unsigned* __restrict__ keys_out, int* __restrict__ vals_out) {
   __shared__ int running[256];
   __shared__ int wcnt[kRadixWarps][256];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   running[threadIdx.x] = 0;
-  const int base = blockIdx.x * kRadixTile;
-  for (int round = 0; round < kRadixItems; ++round) {
+  const int base = blockIdx.x * kRadixThreads * items;
+  for (int round = 0; round < items; ++round) {
     for (int t = threadIdx.x; t < kRadixWarps * 256; t += kRadixThreads) (&wcnt[0][0])[t] = 0;
     __syncthreads();
     const int i = base + round * kRadixThreads + threadIdx.x;
@@ -63,15 +64,15 @@ radix_scatter_kernel(const unsigned* __restrict__ keys, const int* __restrict__ 
 
 void radix_sort_pairs(unsigned* keys, int* vals, unsigned* keys_tmp, int* vals_tmp, int n, int bits,
                       const RadixWorkspace& ws, cudaStream_t s) {
-  const int nb = radix_sort_blocks(n);
+  const int nb = radix_sort_blocks(n), items = radix_items(n);
   unsigned *ka = keys, *kb = keys_tmp;
   int *va = vals, *vb = vals_tmp;
   int passes = 0;
   for (int shift = 0; shift < bits; shift += 8, ++passes) {
-    radix_hist_kernel<<<nb, kRadixThreads, 0, s>>>(ka, n, shift, ws.hist);
+    radix_hist_kernel<<<nb, kRadixThreads, 0, s>>>(ka, n, items, shift, ws.hist);
     FE_LAUNCH("radix_hist_kernel");
     exclusive_scan(ws.hist, ws.offs, 256 * nb, ws.scan_tmp, s);
-    radix_scatter_kernel<<<nb, kRadixThreads, 0, s>>>(ka, va, n, shift, ws.offs, kb, vb);
+    radix_scatter_kernel<<<nb, kRadixThreads, 0, s>>>(ka, va, n, items, shift, ws.offs, kb, vb);
     FE_LAUNCH("radix_scatter_kernel");
     std::swap(ka, kb);
     std::swap(va, vb);

@@ -41,4 +41,37 @@ __device__ __forceinline__ void bitonic_sort(unsigned long long* a, int len, int
   }
 }
 
+// Ascending sort of 32 E keys held by a warp, lane l holding positions l E .. l E + E - 1: the same
+// always-ascending network with strides below E inside a lane and the others by shuffles.
+template <int E>
+__device__ __forceinline__ void warp_sort(unsigned long long (&a)[E], int lane) {
+#pragma unroll
+  for (int size = 2; size <= 32 * E; size <<= 1) {
+#pragma unroll
+    for (int step = size >> 1; step > 0; step >>= 1) {
+      // first step of a size: partner = position ^ (size - 1); then position ^ step
+      const int x = step == (size >> 1) ? size - 1 : step;
+      const int lx = x / E, ix = x % E;
+      if (lx == 0) {
+#pragma unroll
+        for (int i = 0; i < E; ++i) {
+          const int j = i ^ ix;
+          if (j > i) {
+            const unsigned long long u = a[i], v = a[j];
+            a[i] = u < v ? u : v;
+            a[j] = u < v ? v : u;
+          }
+        }
+      } else {
+        const bool low = (lane & (1 << (31 - __clz(lx)))) == 0;
+        unsigned long long b[E];
+#pragma unroll
+        for (int i = 0; i < E; ++i) b[i] = __shfl_xor_sync(0xffffffffu, a[i ^ ix], lx);
+#pragma unroll
+        for (int i = 0; i < E; ++i) a[i] = ((a[i] < b[i]) == low) ? a[i] : b[i];
+      }
+    }
+  }
+}
+
 }  // namespace fe

@@ -350,90 +350,119 @@ constexpr int kSortCap = 8192;  // entries of a row sorted in shared memory
 
 // Sort each row bucket by (column, p bits), then collapse runs of equal columns: the compacted
 // (column, float(sum)) entries are written back to the start of the bucket, `ucount` gets the
-// unique count and `row_mass` the double sum of the row's pair sums. Rows of up to 256 entries
-// (nearly all) take one warp each (sort_unique_small_rows_kernel); longer rows are listed for a
-// CTA each (this kernel), and rows above kSortCap for the global-memory path.
+// unique count and `row_mass` the two-float sum of the row's pair sums. Rows of up to 256 entries
+// (nearly all) take one warp each, their keys in its registers (sort_unique_small_rows_kernel);
+// longer rows are listed for a CTA each (sort_unique_rows_kernel), and rows above kSortCap for the
+// global-memory path. A run of one or two entries is rounded once, as its FP64 sum would be.
 constexpr int kWarpSortCap = 256;
 constexpr int kWarpSortWarps = 8;
 
-// One warp per row of at most kWarpSortCap entries: the same ascending bitonic network in the
-// warp's slice of shared memory, then the run sums and the row mass with exactly the arithmetic
-// of the CTA path for such a row (thread t of 256 owning position t: each run summed in order by
-// its first position, warp sums over positions 32w .. 32w + 31, added for w = 0 .. 7), so the
-// result does not depend on which kernel took the row.
+// Sorted row of len entries in a[] (position lane E + i) -> compacted runs at out, count, mass.
+template <int E>
+__device__ __forceinline__ void unique_row(unsigned long long* __restrict__ row, int len, int lane,
+                                           int* __restrict__ ucount, float2* __restrict__ row_mass) {
+  unsigned long long a[E];
+#pragma unroll
+  for (int i = 0; i < E; ++i) {
+    // any placement sorts: load coalesced
+    const int t = i * 32 + lane;
+    a[i] = t < len ? row[t] : ~0ull;
+  }
+  warp_sort<E>(a, lane);
+  const unsigned prev_col = (unsigned)(__shfl_up_sync(0xffffffffu, a[E - 1], 1) >> 32);
+  const unsigned long long next_key = __shfl_down_sync(0xffffffffu, a[0], 1);
+  const unsigned long long after = lane == 31 ? ~0ull : next_key;
+  Float2Sum mass{0.0f, 0.0f};
+  bool start[E];
+  int mine = 0;
+#pragma unroll
+  for (int i = 0; i < E; ++i) {
+    const int pos = lane * E + i;
+    const unsigned before = i > 0 ? (unsigned)(a[i > 0 ? i - 1 : 0] >> 32) : prev_col;
+    start[i] = pos < len && (pos == 0 || (unsigned)(a[i] >> 32) != before);
+    mine += start[i];
+    if (pos < len) mass = add(mass, __uint_as_float((unsigned)a[i]));
+  }
+  int at = mine;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, at, o);
+    if (lane >= o) at += y;
+  }
+  const int total = __shfl_sync(0xffffffffu, at, 31);
+  at -= mine;
+  // a run of three or more (a neighbour listed twice) may span lanes: its start walks the sorted keys
+  bool longer = false;
+#pragma unroll
+  for (int i = 0; i < E; ++i) {
+    const unsigned col = (unsigned)(a[i] >> 32);
+    const unsigned long long n1 = i + 1 < E ? a[i + 1 < E ? i + 1 : 0] : after;
+    const unsigned long long n2 = i + 2 < E ? a[i + 2 < E ? i + 2 : 0]
+                                            : __shfl_down_sync(0xffffffffu, a[(i + 2) % E], E == 1 ? 2 : 1);
+    const bool in2 = E == 1 ? lane < 30 : (i + 2 < E || lane < 31);
+    if (start[i] && lane * E + i + 2 < len && in2 && (unsigned)(n2 >> 32) == col) longer = true;
+    if (start[i]) {
+      float sum = __uint_as_float((unsigned)a[i]);
+      if (lane * E + i + 1 < len && (unsigned)(n1 >> 32) == col) sum = __fadd_rn(sum, __uint_as_float((unsigned)n1));
+      // every lane has loaded its keys: the bucket may be overwritten
+      row[at++] = ((unsigned long long)col << 32) | (unsigned long long)__float_as_uint(sum);
+    }
+  }
+  if (__any_sync(0xffffffffu, longer)) {
+    // rare: sum every run over the whole row, key by key
+    __syncwarp();  // after the lanes' writes above
+    Float2Sum run{0.0f, 0.0f};
+    int w = -1;
+    unsigned cur = 0;
+    for (int l = 0; l < 32; ++l)
+#pragma unroll
+      for (int i = 0; i < E; ++i) {
+        const unsigned long long key = __shfl_sync(0xffffffffu, a[i], l);
+        if (l * E + i >= len) continue;
+        const unsigned col = (unsigned)(key >> 32);
+        if (w < 0 || col != cur) {
+          ++w;
+          cur = col;
+          run = Float2Sum{0.0f, 0.0f};
+        }
+        run = add(run, __uint_as_float((unsigned)key));
+        if (lane == 0) row[w] = ((unsigned long long)col << 32) | (unsigned long long)__float_as_uint(run.hi);
+      }
+  }
+  mass = warp_sum(mass);
+  if (lane == 0) {
+    *row_mass = make_float2(mass.hi, mass.lo);
+    *ucount = total;
+  }
+}
+
 __global__ void __launch_bounds__(kWarpSortWarps * 32)
 sort_unique_small_rows_kernel(unsigned long long* __restrict__ bucket, const long long* __restrict__ offs, int n,
-                              int* __restrict__ ucount, double* __restrict__ row_mass, int* __restrict__ mid_rows,
+                              int* __restrict__ ucount, float2* __restrict__ row_mass, int* __restrict__ mid_rows,
                               int* __restrict__ mid_count) {
-  __shared__ unsigned long long sm[kWarpSortWarps][kWarpSortCap];
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  unsigned long long* a = sm[wib];
+  const int lane = threadIdx.x & 31;
   const int warps = gridDim.x * kWarpSortWarps;
-  for (int row = blockIdx.x * kWarpSortWarps + wib; row < n; row += warps) {
+  for (int row = blockIdx.x * kWarpSortWarps + (threadIdx.x >> 5); row < n; row += warps) {
     const long long b = offs[row];
     const int len = (int)(offs[row + 1] - b);
     if (len > kWarpSortCap) {
       if (lane == 0) mid_rows[atomicAdd(mid_count, 1)] = row;
-      continue;
+    } else if (len > 128) {
+      unique_row<8>(bucket + b, len, lane, ucount + row, row_mass + row);
+    } else if (len > 64) {
+      unique_row<4>(bucket + b, len, lane, ucount + row, row_mass + row);
+    } else if (len > 32) {
+      unique_row<2>(bucket + b, len, lane, ucount + row, row_mass + row);
+    } else {
+      unique_row<1>(bucket + b, len, lane, ucount + row, row_mass + row);
     }
-    int pw = 1;
-    while (pw < len) pw <<= 1;
-    for (int t = lane; t < pw; t += 32) a[t] = t < len ? bucket[b + t] : ~0ull;
-    __syncwarp();
-    for (int size = 2; size <= pw && len > 1; size <<= 1) {
-      const int half = size >> 1;
-      for (int t = lane; t < pw / 2; t += 32) {
-        const int blk = t / half, off = t % half;
-        const int i = blk * size + off, j = blk * size + size - 1 - off;
-        const unsigned long long x = a[i], y = a[j];
-        if (y < x) {
-          a[i] = y;
-          a[j] = x;
-        }
-      }
-      __syncwarp();
-      for (int stride = half >> 1; stride > 0; stride >>= 1) {
-        for (int t = lane; t < pw / 2; t += 32) {
-          const int blk = t / stride, off = t % stride;
-          const int i = blk * 2 * stride + off, j = i + stride;
-          const unsigned long long x = a[i], y = a[j];
-          if (y < x) {
-            a[i] = y;
-            a[j] = x;
-          }
-        }
-        __syncwarp();
-      }
-    }
-    int cnt = 0;
-    double tot = 0.0;
-    for (int w = 0; w < kWarpSortCap / 32; ++w) {
-      const int t = w * 32 + lane;
-      bool start = false;
-      if (t < len) start = (t == 0) || ((a[t] >> 32) != (a[t - 1] >> 32));
-      const unsigned ballot = __ballot_sync(0xffffffffu, start);
-      double sum = 0.0;
-      if (start) {
-        const unsigned col = (unsigned)(a[t] >> 32);
-        for (int u = t; u < len && (unsigned)(a[u] >> 32) == col; ++u) sum += (double)__uint_as_float((unsigned)a[u]);
-        const int pos = cnt + __popc(ballot & ((1u << lane) - 1u));
-        bucket[b + pos] = ((unsigned long long)col << 32) | (unsigned long long)__float_as_uint((float)sum);
-      }
-      cnt += __popc(ballot);
-      tot += warp_sum(sum);
-    }
-    if (lane == 0) {
-      row_mass[row] = tot;
-      ucount[row] = cnt;
-    }
-    __syncwarp();
   }
 }
 
 __global__ void __launch_bounds__(kSortThreads)
 sort_unique_rows_kernel(unsigned long long* __restrict__ bucket, const long long* __restrict__ offs,
                         const int* __restrict__ rows, const int* __restrict__ row_count, int* __restrict__ ucount,
-                        double* __restrict__ row_mass, int* __restrict__ big_rows, int* __restrict__ big_count) {
+                        float2* __restrict__ row_mass, int* __restrict__ big_rows, int* __restrict__ big_count) {
   extern __shared__ unsigned long long sm[];
   __shared__ int warp_cnt[kSortThreads / 32];
   __shared__ double warp_mass[kSortThreads / 32];
@@ -484,7 +513,8 @@ sort_unique_rows_kernel(unsigned long long* __restrict__ bucket, const long long
     if (threadIdx.x == 0) {
       double tot = 0.0;
       for (int w = 0; w < (int)(blockDim.x / 32); ++w) tot += warp_mass[w];
-      row_mass[row] = tot;
+      const Float2Sum m2 = split(tot);
+      row_mass[row] = make_float2(m2.hi, m2.lo);
       ucount[row] = my_cnt;
     }
     __syncthreads();
@@ -496,7 +526,7 @@ sort_unique_rows_kernel(unsigned long long* __restrict__ bucket, const long long
 __global__ void __launch_bounds__(1024)
 sort_unique_big_rows_kernel(unsigned long long* __restrict__ bucket, const long long* __restrict__ offs,
                             const int* __restrict__ big_rows, const int* __restrict__ big_count,
-                            int* __restrict__ ucount, double* __restrict__ row_mass) {
+                            int* __restrict__ ucount, float2* __restrict__ row_mass) {
   const int count = *big_count;
   for (int r = blockIdx.x; r < count; r += gridDim.x) {
     const int row = big_rows[r];
@@ -520,7 +550,8 @@ sort_unique_big_rows_kernel(unsigned long long* __restrict__ bucket, const long 
         mass += sum;
       }
       ucount[row] = w;
-      row_mass[row] = mass;
+      const Float2Sum m2 = split(mass);
+      row_mass[row] = make_float2(m2.hi, m2.lo);
     }
     __syncthreads();
   }
@@ -528,22 +559,26 @@ sort_unique_big_rows_kernel(unsigned long long* __restrict__ bucket, const long 
 
 // Deterministic totals: block b sums the rows [first[b], first[b + 1]) of instance b with a
 // fixed assignment and a fixed tree (a single instance is first = {0, n}).
-__global__ void total_mass_kernel(const double* __restrict__ row_mass, const int* __restrict__ first,
-                                  double* __restrict__ out_total, float* __restrict__ out_norm) {
-  __shared__ double part[1024];
+__global__ void __launch_bounds__(1024)
+total_mass_kernel(const float2* __restrict__ row_mass, const int* __restrict__ first, double* __restrict__ out_total,
+                  float* __restrict__ out_norm) {
+  __shared__ Float2Sum part[32];
   const int r0 = first[blockIdx.x], r1 = first[blockIdx.x + 1];
-  double s = 0.0;
-  for (int i = r0 + threadIdx.x; i < r1; i += blockDim.x) s += row_mass[i];
-  part[threadIdx.x] = s;
-  __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if ((int)threadIdx.x < w) part[threadIdx.x] += part[threadIdx.x + w];
-    __syncthreads();
+  Float2Sum s{0.0f, 0.0f};
+#pragma unroll 4
+  for (int i = r0 + threadIdx.x; i < r1; i += 1024) {
+    const float2 m = row_mass[i];
+    s = add(s, Float2Sum{m.x, m.y});
   }
-  if (threadIdx.x == 0) {
-    const double total = 0.5 * part[0];  // every pair sum appears in both of its rows
-    out_total[blockIdx.x] = total;
-    out_norm[blockIdx.x] = (float)(0.5 / total);
+  s = warp_sum(s);
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    const double total = 0.5 * value(warp_sum(part[threadIdx.x]));  // every pair sum appears in both of its rows
+    if (threadIdx.x == 0) {
+      out_total[blockIdx.x] = total;
+      out_norm[blockIdx.x] = (float)(0.5 / total);
+    }
   }
 }
 
@@ -602,7 +637,7 @@ void symmetrise_batch(const int* d_idx, const float* d_p, int n, int k, int offs
   unsigned long long* cursor = nullptr;
   unsigned long long* bucket = nullptr;
   int* ucount = nullptr;
-  double* row_mass = nullptr;
+  float2* row_mass = nullptr;
   int* big_rows = nullptr;
   int* big_count = nullptr;
   int* mid_rows = nullptr;

@@ -32,26 +32,27 @@
 #include "philox.cuh"
 #include "sort.cuh"
 #include "tsne.cuh"
+#include "twofloat.cuh"
 #include "umap_spectral.cuh"
 
 namespace fe {
 
 // ---------------------------------------------------------------- smooth kNN
 __global__ void umap_distance_sum_kernel(const float* __restrict__ dist, long long total, double* __restrict__ acc) {
-  double s = 0.0;
+  Float2Sum f{0.0f, 0.0f};
   unsigned long long c = 0;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
     const float d = dist[t];
     if (isfinite(d) && d >= 0.0f) {
-      s += (double)d;
+      f = add(f, d);
       ++c;
     }
   }
-  s = warp_sum(s);
+  f = warp_sum(f);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
   if ((threadIdx.x & 31) == 0) {
-    atomicAdd(acc, s);
+    atomicAdd(acc, value(f));
     atomicAdd(reinterpret_cast<unsigned long long*>(acc + 1), c);
   }
 }
@@ -94,6 +95,19 @@ __device__ double smooth_sigma_exact(const float* __restrict__ d, int k, double 
   return best;
 }
 
+// The same sum with 40-bit exponentials (relative error about 1e-12 a term).
+__device__ Float2Sum smooth_psum_two(const float* __restrict__ d, int k, float rho, Float2Sum inv,
+                                     const float2* __restrict__ table) {
+  Float2Sum psum{0.0f, 0.0f};
+  for (int j = 0; j < k; ++j) {
+    const float raw = d[j];
+    if (!isfinite(raw)) continue;
+    const Float2Sum x = two_sum(rho, -raw);
+    psum = raw <= rho ? add(psum, 1.0f) : add(psum, exp_two(mul(x, inv), table));
+  }
+  return psum;
+}
+
 // smooth_knn_dist (:876-996), one thread per row; distances column-major n x k, staged through
 // shared memory (blockDim.x rows x (k + 1) raw distances, then as many positive offsets d - rho).
 // The search runs its membership sums on the FP32 pipe: exp of float offsets times a float
@@ -101,14 +115,19 @@ __device__ double smooth_sigma_exact(const float* __restrict__ d, int k, double 
 // at most 1.2e-7 per unit of the total, so |psum32 - psum64| < 4e-7 k. The decisions of the
 // search are the sign of psum - target and the stop test |psum - target| < 1e-5; an FP32 sum
 // farther than that margin from the stop boundary takes both as FP64 would (a sum inside the
-// stop band stops either way), and one inside the margin is re-evaluated in FP64. The FP64
+// stop band stops either way), and one inside the margin is re-evaluated with 40-bit exponentials, and
+// in FP64 if that comes within 1e-10 of the boundary. The FP64
 // search keeps the sigma of the smallest |psum - target|, which at a stop is the stopping sigma
 // (every earlier difference was >= 1e-5), so the result is the FP64 search's. A row that does not
 // stop within 64 steps is searched again in FP64 from the start.
+// What bounds it is the FP32 sums now: FP64 quotients, differences and re-evaluations (the margin
+// spans two octaves around the boundary, so nearly every row met one) took 747 us for 100,000 rows of 15.
 __global__ void __launch_bounds__(kSmoothRows)
-umap_smooth_knn_kernel(const float* __restrict__ dist, int n, int k, const double* __restrict__ acc,
+umap_smooth_knn_kernel(const float* __restrict__ dist, int n, int k, double target, const double* __restrict__ acc,
                        float* __restrict__ sigmas, float* __restrict__ rhos) {
   extern __shared__ float s_tile[];
+  __shared__ float2 exp_table[kExpEntries];
+  fill_exp_table(exp_table);
   const int rows = blockDim.x, stride = k + 1;
   float* s_off = s_tile + (long long)rows * stride;
   const int r0 = blockIdx.x * rows;
@@ -122,55 +141,56 @@ umap_smooth_knn_kernel(const float* __restrict__ dist, int n, int k, const doubl
   if (rr >= nrows) return;
   const float* d = s_tile + rr * stride;
   float* off = s_off + rr * stride;
-  const unsigned long long cnt = reinterpret_cast<const unsigned long long*>(acc)[1];
-  const double global_mean = cnt > 0 ? acc[0] / (double)cnt : 1.0;
-  const double target = log2((double)k);
-  double rho = INFINITY, row_sum = 0.0;
+  float rho = INFINITY;
+  Float2Sum row_sum{0.0f, 0.0f};
   int row_count = 0;
   for (int j = 0; j < k; ++j) {
     const float v = d[j];
     if (!isfinite(v)) continue;
     if (v >= 0.0f) {
-      row_sum += (double)v;
+      row_sum = add(row_sum, v);
       ++row_count;
     }
-    if (v > 0.0f && (double)v < rho) rho = (double)v;
+    if (v > 0.0f && v < rho) rho = v;
   }
-  if (!isfinite(rho)) rho = 0.0;
+  if (!isfinite(rho)) rho = 0.0f;
   // finite entries at or below rho contribute exactly 1; the others their float offset, which
   // is positive (the difference of two distinct floats does not round to zero in FP32)
   int ones = 0, m = 0;
   for (int j = 0; j < k; ++j) {
     const float v = d[j];
     if (!isfinite(v)) continue;
-    const double x = (double)v - rho;
-    if (x <= 0.0) ++ones;
-    else off[m++] = (float)x;
+    if (v <= rho) ++ones;
+    else off[m++] = __fsub_rn(v, rho);
   }
-  const double margin = 4.0e-7 * (double)k;
+  const float margin = 4.0e-7f * (float)k;
+  const Float2Sum goal = split(-target);
   double sigma = 1.0, best = 1.0, lo = 0.0, hi = DBL_MAX;
   bool stopped = false;
   for (int it = 0; it < 64; ++it) {
-    const float inv = (float)(1.0 / fmax(sigma, 1.0e-12));
+    const Float2Sum inv = divide(Float2Sum{1.0f, 0.0f}, split(fmax(sigma, 1.0e-12)));
     float ps = (float)ones, pc = 0.0f;
     for (int j = 0; j < m; ++j) {
-      const float y = expf(-off[j] * inv) - pc;
+      const float y = expf(-off[j] * inv.hi) - pc;
       const float t = ps + y;
       pc = (t - ps) - y;
       ps = t;
     }
-    double psum = (double)ps - (double)pc;
-    double diff = fabs(psum - target);
-    if (fabs(diff - 1.0e-5) < margin) {
-      psum = smooth_psum_exact(d, k, rho, sigma);
-      diff = fabs(psum - target);
+    Float2Sum diff = add(two_sum(ps, -pc), goal);
+    float gap = fabsf(diff.hi) - 1.0e-5f;
+    if (fabsf(gap) < margin) {
+      diff = add(smooth_psum_two(d, k, rho, inv, exp_table), goal);
+      double exact = value(diff);
+      if (fabs(fabs(exact) - 1.0e-5) < 1.0e-10) exact = smooth_psum_exact(d, k, (double)rho, sigma) - target;
+      gap = fabs(exact) < 1.0e-5 ? -1.0f : 1.0f;
+      diff.hi = exact > 0.0 ? 1.0f : -1.0f;
     }
-    if (diff < 1.0e-5) {
+    if (gap < 0.0f) {
       best = sigma;
       stopped = true;
       break;
     }
-    if (psum > target) {
+    if (diff.hi > 0.0f) {
       hi = sigma;
       sigma = 0.5 * (lo + hi);
     } else {
@@ -178,11 +198,16 @@ umap_smooth_knn_kernel(const float* __restrict__ dist, int n, int k, const doubl
       sigma = hi == DBL_MAX ? sigma * 2.0 : 0.5 * (lo + hi);
     }
   }
-  if (!stopped) best = smooth_sigma_exact(d, k, rho, target);
-  const double row_mean = row_count > 0 ? row_sum / (double)row_count : global_mean;
-  const double floor_s = 1.0e-3 * (rho > 0.0 ? row_mean : global_mean);
-  best = fmax(best, floor_s);
-  rhos[r0 + rr] = (float)rho;
+  if (!stopped) best = smooth_sigma_exact(d, k, (double)rho, target);
+  double mean = 0.0;
+  if (rho > 0.0f && row_count > 0) {
+    mean = value(divide(row_sum, Float2Sum{(float)row_count, 0.0f}));
+  } else {
+    const unsigned long long cnt = reinterpret_cast<const unsigned long long*>(acc)[1];
+    mean = cnt > 0 ? acc[0] / (double)cnt : 1.0;
+  }
+  best = fmax(best, 1.0e-3 * mean);
+  rhos[r0 + rr] = rho;
   sigmas[r0 + rr] = (float)fmax(best, 1.0e-12);
 }
 
@@ -193,7 +218,7 @@ void smooth_knn(const float* d_dist, int n, int k, const double* acc, float* sig
   if (smem > 200 * 1024) throw Error("k is too large for the UMAP smooth-kNN search (at most 25,000 neighbours)");
   if (smem > 48 * 1024)
     FE_CUDA(cudaFuncSetAttribute(umap_smooth_knn_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  umap_smooth_knn_kernel<<<ceil_div(n, rows), rows, smem, s>>>(d_dist, n, k, acc, sig, rho);
+  umap_smooth_knn_kernel<<<ceil_div(n, rows), rows, smem, s>>>(d_dist, n, k, std::log2((double)k), acc, sig, rho);
   FE_LAUNCH("umap_smooth_knn_kernel");
 }
 
@@ -237,6 +262,8 @@ __global__ void umap_fill_kernel(const int* __restrict__ idx, const float* __res
   }
 }
 
+__device__ __forceinline__ float union_of(float f, float r) { return __fmaf_rn(-f, r, __fadd_rn(f, r)); }
+
 // Forward / reverse weights of one column run [t, end): the maximum per direction (duplicates
 // of a directed edge keep their maximum), then the fuzzy union.
 __device__ __forceinline__ float union_weight(const unsigned long long* a, int t, int len, unsigned col, int* end) {
@@ -249,20 +276,152 @@ __device__ __forceinline__ float union_weight(const unsigned long long* a, int t
     else f = fmaxf(f, w);
   }
   *end = u;
-  return f + r - f * r;
+  return union_of(f, r);
 }
 
 constexpr int kUmapSortThreads = 256;
 constexpr int kUmapSortCap = 4096;
+constexpr int kUmapWarpCap = 256;  // longest row sorted by one warp
+
+// The largest weight over all rows: weights are positive, so their bits order as integers.
+__device__ __forceinline__ void raise_max(float* __restrict__ max_w, float m) {
+  if (m > 0.0f) atomicMax(reinterpret_cast<int*>(max_w), __float_as_int(m));
+}
+
+// One warp per row of at most kUmapWarpCap directed entries, keys in registers (position lane E + i):
+// sorted by column, each column's run of directions united, weights above 1e-6 written back
+// compacted. Returns the row's largest weight.
+template <int E>
+__device__ __forceinline__ float union_row(unsigned long long* __restrict__ row, int len, int lane,
+                                           int* __restrict__ ucount) {
+  unsigned long long a[E];
+#pragma unroll
+  for (int i = 0; i < E; ++i) {
+    const int t = i * 32 + lane;
+    a[i] = t < len ? row[t] : ~0ull;
+  }
+  warp_sort<E>(a, lane);
+  const unsigned prev_col = (unsigned)(__shfl_up_sync(0xffffffffu, a[E - 1], 1) >> 32);
+  const unsigned long long next_key = __shfl_down_sync(0xffffffffu, a[0], 1);
+  const unsigned long long after = lane == 31 ? ~0ull : next_key;
+  float w[E];
+  bool keep[E], longer = false;
+  int mine = 0;
+#pragma unroll
+  for (int i = 0; i < E; ++i) {
+    const int pos = lane * E + i;
+    const unsigned col = (unsigned)(a[i] >> 32);
+    const unsigned before = i > 0 ? (unsigned)(a[i > 0 ? i - 1 : 0] >> 32) : prev_col;
+    const unsigned long long n1 = i + 1 < E ? a[i + 1 < E ? i + 1 : 0] : after;
+    const unsigned long long n2 = i + 2 < E ? a[i + 2 < E ? i + 2 : 0]
+                                            : __shfl_down_sync(0xffffffffu, a[(i + 2) % E], E == 1 ? 2 : 1);
+    const bool in2 = E == 1 ? lane < 30 : (i + 2 < E || lane < 31);
+    const bool start = pos < len && (pos == 0 || col != before);
+    const bool two = pos + 1 < len && (unsigned)(n1 >> 32) == col;
+    if (start && two && pos + 2 < len && in2 && (unsigned)(n2 >> 32) == col) longer = true;
+    const unsigned k0 = (unsigned)a[i], k1 = (unsigned)n1;
+    float f = 0.0f, r = 0.0f;
+    if (k0 & 0x80000000u) r = __uint_as_float(k0 & 0x7fffffffu);
+    else f = __uint_as_float(k0);
+    if (two) {
+      if (k1 & 0x80000000u) r = fmaxf(r, __uint_as_float(k1 & 0x7fffffffu));
+      else f = fmaxf(f, __uint_as_float(k1));
+    }
+    w[i] = union_of(f, r);
+    keep[i] = start && isfinite(w[i]) && w[i] > 1.0e-6f;
+    mine += keep[i];
+  }
+  int at = mine;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, at, o);
+    if (lane >= o) at += y;
+  }
+  int total = __shfl_sync(0xffffffffu, at, 31);
+  at -= mine;
+  float mx = 0.0f;
+  if (!__any_sync(0xffffffffu, longer)) {
+    // every lane has loaded its keys: the bucket may be overwritten
+#pragma unroll
+    for (int i = 0; i < E; ++i)
+      if (keep[i]) {
+        row[at++] = (a[i] & 0xffffffff00000000ull) | (unsigned long long)__float_as_uint(w[i]);
+        mx = fmaxf(mx, w[i]);
+      }
+  } else {
+    // rare (a neighbour listed more than once): unite every run over the whole row, key by key
+    float f = 0.0f, r = 0.0f;
+    unsigned cur = 0;
+    int out = 0;
+    auto flush = [&]() {
+      const float u = union_of(f, r);
+      if (isfinite(u) && u > 1.0e-6f) {
+        if (lane == 0) row[out] = ((unsigned long long)cur << 32) | (unsigned long long)__float_as_uint(u);
+        ++out;
+        mx = fmaxf(mx, u);
+      }
+    };
+    for (int l = 0; l < 32; ++l)
+#pragma unroll
+      for (int i = 0; i < E; ++i) {
+        const unsigned long long key = __shfl_sync(0xffffffffu, a[i], l);
+        if (l * E + i >= len) continue;
+        if (l * E + i > 0 && (unsigned)(key >> 32) != cur) {
+          flush();
+          f = r = 0.0f;
+        }
+        cur = (unsigned)(key >> 32);
+        const float v = __uint_as_float((unsigned)key & 0x7fffffffu);
+        if ((unsigned)key & 0x80000000u) r = fmaxf(r, v);
+        else f = fmaxf(f, v);
+      }
+    flush();
+    total = out;
+  }
+  if (lane == 0) *ucount = total;
+  return mx;
+}
 
 __global__ void __launch_bounds__(kUmapSortThreads)
-umap_union_rows_kernel(unsigned long long* __restrict__ bucket, const long long* __restrict__ offs, int n,
-                       int* __restrict__ ucount, float* __restrict__ row_max, int* __restrict__ big_rows,
-                       int* __restrict__ big_count) {
+umap_union_small_rows_kernel(unsigned long long* __restrict__ bucket, const long long* __restrict__ offs, int n,
+                             int* __restrict__ ucount, float* __restrict__ max_w, int* __restrict__ mid_rows,
+                             int* __restrict__ mid_count) {
+  const int lane = threadIdx.x & 31, warps = gridDim.x * (kUmapSortThreads / 32);
+  float mx = 0.0f;
+  for (int row = blockIdx.x * (kUmapSortThreads / 32) + (threadIdx.x >> 5); row < n; row += warps) {
+    const long long b = offs[row];
+    const int len = (int)(offs[row + 1] - b);
+    float m = 0.0f;
+    if (len == 0) {
+      if (lane == 0) ucount[row] = 0;
+    } else if (len > kUmapWarpCap) {
+      if (lane == 0) mid_rows[atomicAdd(mid_count, 1)] = row;
+    } else if (len > 128) {
+      m = union_row<8>(bucket + b, len, lane, ucount + row);
+    } else if (len > 64) {
+      m = union_row<4>(bucket + b, len, lane, ucount + row);
+    } else if (len > 32) {
+      m = union_row<2>(bucket + b, len, lane, ucount + row);
+    } else {
+      m = union_row<1>(bucket + b, len, lane, ucount + row);
+    }
+    mx = fmaxf(mx, m);
+  }
+  mx = warp_max(mx);
+  if (lane == 0) raise_max(max_w, mx);
+}
+
+// Rows longer than kUmapWarpCap (listed by the kernel above), a CTA each.
+__global__ void __launch_bounds__(kUmapSortThreads)
+umap_union_rows_kernel(unsigned long long* __restrict__ bucket, const long long* __restrict__ offs,
+                       const int* __restrict__ rows, const int* __restrict__ row_count, int* __restrict__ ucount,
+                       float* __restrict__ max_w, int* __restrict__ big_rows, int* __restrict__ big_count) {
   extern __shared__ unsigned long long sm[];
   __shared__ int warp_cnt[kUmapSortThreads / 32];
   __shared__ float s_wmax[kUmapSortThreads / 32];
-  for (int row = blockIdx.x; row < n; row += gridDim.x) {
+  const int count = *row_count;
+  for (int item = blockIdx.x; item < count; item += gridDim.x) {
+    const int row = rows[item];
     const long long b = offs[row];
     const int len = (int)(offs[row + 1] - b);
     if (len > kUmapSortCap) {
@@ -310,7 +469,7 @@ umap_union_rows_kernel(unsigned long long* __restrict__ bucket, const long long*
     if (threadIdx.x == 0) {
       float mm = 0.0f;
       for (int wi = 0; wi < (int)(blockDim.x / 32); ++wi) mm = fmaxf(mm, s_wmax[wi]);
-      row_max[row] = mm;
+      raise_max(max_w, mm);
       ucount[row] = kept_before;
     }
     __syncthreads();
@@ -320,7 +479,7 @@ umap_union_rows_kernel(unsigned long long* __restrict__ bucket, const long long*
 __global__ void __launch_bounds__(1024)
 umap_union_big_rows_kernel(unsigned long long* __restrict__ bucket, const long long* __restrict__ offs,
                            const int* __restrict__ big_rows, const int* __restrict__ big_count,
-                           int* __restrict__ ucount, float* __restrict__ row_max) {
+                           int* __restrict__ ucount, float* __restrict__ max_w) {
   const int count = *big_count;
   for (int r = blockIdx.x; r < count; r += gridDim.x) {
     const int row = big_rows[r];
@@ -343,23 +502,10 @@ umap_union_big_rows_kernel(unsigned long long* __restrict__ bucket, const long l
         }
       }
       ucount[row] = w_out;
-      row_max[row] = mm;
+      raise_max(max_w, mm);
     }
     __syncthreads();
   }
-}
-
-__global__ void umap_max_kernel(const float* __restrict__ row_max, int n, float* __restrict__ out) {
-  __shared__ float part[1024];
-  float m = 0.0f;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) m = fmaxf(m, row_max[i]);
-  part[threadIdx.x] = m;
-  __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if ((int)threadIdx.x < w) part[threadIdx.x] = fmaxf(part[threadIdx.x], part[threadIdx.x + w]);
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) *out = part[0];
 }
 
 __global__ void umap_fill_csr_kernel(const unsigned long long* __restrict__ bucket, const long long* __restrict__ offs,
@@ -401,9 +547,10 @@ struct UmapGraph {
 // batch reuses one workspace for every instance, in stream order.
 struct UmapGraphWork {
   int cap_n = 0, k = 0;
-  float *sig = nullptr, *rho = nullptr, *row_max = nullptr, *d_max = nullptr;
+  float *sig = nullptr, *rho = nullptr, *d_max = nullptr;
   double* acc = nullptr;
   int *counts = nullptr, *ucount = nullptr, *big_rows = nullptr, *big_count = nullptr;
+  int *mid_rows = nullptr, *mid_count = nullptr;
   long long *offs = nullptr, *scan_tmp = nullptr, *out64 = nullptr;
   unsigned long long *cursor = nullptr, *bucket = nullptr;
   Arena arena;
@@ -414,13 +561,14 @@ struct UmapGraphWork {
     const long long directed = (long long)max_n * k;
     arena.reserve(&sig, max_n);
     arena.reserve(&rho, max_n);
-    arena.reserve(&row_max, max_n);
     arena.reserve(&d_max, 1);
     arena.reserve(&acc, 2);
     arena.reserve(&counts, max_n);
     arena.reserve(&ucount, max_n);
     arena.reserve(&big_rows, max_n);
     arena.reserve(&big_count, 1);
+    arena.reserve(&mid_rows, max_n);
+    arena.reserve(&mid_count, 1);
     arena.reserve(&offs, max_n + 1);
     arena.reserve(&scan_tmp, std::max(1, ceil_div(max_n, 1024)));
     arena.reserve(&out64, max_n + 1);
@@ -438,6 +586,8 @@ struct UmapGraphWork {
     FE_CUDA(cudaMemsetAsync(acc, 0, 2 * sizeof(double), s));
     FE_CUDA(cudaMemsetAsync(counts, 0, sizeof(int) * n, s));
     FE_CUDA(cudaMemsetAsync(big_count, 0, sizeof(int), s));
+    FE_CUDA(cudaMemsetAsync(mid_count, 0, sizeof(int), s));
+    FE_CUDA(cudaMemsetAsync(d_max, 0, sizeof(float), s));
     umap_distance_sum_kernel<<<grid, 256, 0, s>>>(d_dist, directed, acc);
     FE_LAUNCH("umap_distance_sum_kernel");
     smooth_knn(d_dist, n, k, acc, sig, rho, s);
@@ -449,14 +599,15 @@ struct UmapGraphWork {
     FE_LAUNCH("umap_fill_kernel");
     const std::size_t smem = kUmapSortCap * sizeof(unsigned long long);
     FE_CUDA(cudaFuncSetAttribute(umap_union_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    umap_union_rows_kernel<<<std::min(n, sm_count() * 8), kUmapSortThreads, smem, s>>>(bucket, offs, n, ucount,
-                                                                                       row_max, big_rows, big_count);
+    umap_union_small_rows_kernel<<<std::max(1, std::min(ceil_div(n, kUmapSortThreads / 32), sm_count() * 8)),
+                                   kUmapSortThreads, 0, s>>>(bucket, offs, n, ucount, d_max, mid_rows, mid_count);
+    FE_LAUNCH("umap_union_small_rows_kernel");
+    umap_union_rows_kernel<<<sm_count(), kUmapSortThreads, smem, s>>>(bucket, offs, mid_rows, mid_count, ucount, d_max,
+                                                                      big_rows, big_count);
     FE_LAUNCH("umap_union_rows_kernel");
-    umap_union_big_rows_kernel<<<sm_count(), 1024, 0, s>>>(bucket, offs, big_rows, big_count, ucount, row_max);
+    umap_union_big_rows_kernel<<<sm_count(), 1024, 0, s>>>(bucket, offs, big_rows, big_count, ucount, d_max);
     FE_LAUNCH("umap_union_big_rows_kernel");
     exclusive_scan(ucount, out64, n, scan_tmp, s);
-    umap_max_kernel<<<1, 1024, 0, s>>>(row_max, n, d_max);
-    FE_LAUNCH("umap_max_kernel");
   }
 };
 
