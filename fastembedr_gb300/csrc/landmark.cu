@@ -302,7 +302,7 @@ extern "C" int fastembedr_cuda_landmark_tsne_from_device_knn(
     FE_CUDA(cudaMemcpyAsync(d_seg, &seg, sizeof(seg), cudaMemcpyHostToDevice, s));
     const fe::XorshiftJump jump = fe::xorshift_jump_table(tp.n_negatives);
     FE_CUDA(cudaMemcpyAsync(d_jump, &jump, sizeof(jump), cudaMemcpyHostToDevice, s));
-    fe::transform_prepare(d_ref, d_ref_d, d_seg, 1, n_query, tp, s);
+    fe::transform_prepare(d_ref, d_ref_d, d_seg, 1, n_query, k, tp, s);
     const int chunk = fe::transform_chunk(n_query, tp, k);
     for (int it = 0; it < tp.iter_total; it += chunk)
       fe::transform_iterate(d_ref, d_seg, 1, n_query, tp, d_jump, it, std::min(tp.iter_total, it + chunk), s);

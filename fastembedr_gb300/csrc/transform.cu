@@ -18,6 +18,7 @@
 // Precision: pair terms, sums, gains and momentum in FP32; the layout is a two-float
 // (compensated) value so 250 small steps keep their low bits; P in FP64, stored as FP32.
 #include "transform.cuh"
+#include "twofloat.cuh"
 
 #include <cfloat>
 #include <climits>
@@ -97,9 +98,16 @@ __device__ __forceinline__ int find_segment(const TransformSegment* segs, int ns
   return lo;
 }
 
+// Place of neighbour j of query i in the segment's KNN arrays.
+__device__ __forceinline__ long long seg_place(const TransformSegment& sg, int j, int i) {
+  return sg.row_major ? (long long)i * sg.k + j : (long long)j * sg.nq + i;
+}
 __device__ __forceinline__ double seg_dist(const TransformSegment& sg, int j, int i) {
-  const long long pos = (long long)j * sg.nq + i;
+  const long long pos = seg_place(sg, j, i);
   return sg.dist_f ? (double)sg.dist_f[pos] : sg.dist_d[pos];
+}
+__device__ __forceinline__ int seg_index(const TransformSegment& sg, int j, int i) {
+  return sg.idx[seg_place(sg, j, i)] - sg.offset;
 }
 
 __global__ void transform_reference_kernel(const double* __restrict__ ref_cm, int n_ref, float2* __restrict__ ref,
@@ -111,9 +119,24 @@ __global__ void transform_reference_kernel(const double* __restrict__ ref_cm, in
   }
 }
 
-// Warp per query: FP64 bisection of compute_row_probabilities_flat, P stored as FP32 [query][k].
-__global__ void transform_row_p_kernel(const TransformSegment* __restrict__ segs, int nseg, long long total_q,
-                                       double perplexity) {
+constexpr int kPrepareWarps = 8;
+constexpr int kRowCache = 512;  // shifted squares of a row kept in shared memory up to this k
+
+// Warp per query: bisection of compute_row_probabilities_flat, P stored as FP32 [query][k].
+// The search evaluates its sums with two-float exponentials (about 1e-12 relative); a step within 1e-9
+// of the stop tolerance, or with beta or distances near the ends of the float range, is evaluated in
+// FP64 as the reference does, so the search stops at the same beta. The sum at that beta and the
+// probabilities are FP64. (FP64 throughout took 1.57 ms for 10,000 queries of 90 neighbours: about 230
+// FP64 instructions a step at 19 cycles each.)
+__global__ void __launch_bounds__(kPrepareWarps * 32)
+transform_row_p_kernel(const TransformSegment* __restrict__ segs, int nseg, long long total_q, double target,
+                       int cache_k) {
+  extern __shared__ float2 s_cache[];  // kPrepareWarps x cache_k
+  __shared__ float2 exp_table[kExpEntries];
+  __shared__ float4 log_table[kLogEntries];
+  fill_exp_table(exp_table);
+  fill_log_table(log_table);
+  __syncthreads();
   const int lane = threadIdx.x & 31;
   const long long q = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (q >= total_q) return;
@@ -121,10 +144,12 @@ __global__ void transform_row_p_kernel(const TransformSegment* __restrict__ segs
   const int i = (int)(q - sg.query_begin), k = sg.k;
   float* prow = sg.p + (long long)i * k;
   double mn = DBL_MAX, mx = 0.0;
+  bool odd = false;
   for (int j = lane; j < k; j += 32) {
     const double d = seg_dist(sg, j, i);
     mn = fmin(mn, d * d);
     mx = fmax(mx, d * d);
+    odd |= !(d * d < 1.0e30);
   }
   mn = warp_min(mn);
   mx = warp_max(mx);
@@ -132,9 +157,16 @@ __global__ void transform_row_p_kernel(const TransformSegment* __restrict__ segs
     for (int j = lane; j < k; j += 32) prow[j] = (float)(1.0 / (double)k);
     return;
   }
-  const double target = log(perplexity);
-  double beta = 1.0, bmin = -DBL_MAX, bmax = DBL_MAX, beta_eval = 1.0, sum_p = DBL_MIN;
-  for (int it = 0; it < 200; ++it) {
+  const bool wide = __any_sync(0xffffffffu, odd) || !(mx > 1.0e-25);
+  float2* cache = k <= cache_k ? s_cache + (threadIdx.x >> 5) * cache_k : nullptr;
+  if (cache)
+    for (int j = lane; j < k; j += 32) {  // read back by the same lane
+      const double d = seg_dist(sg, j, i);
+      const Float2Sum t = split(d * d - mn);
+      cache[j] = make_float2(t.hi, t.lo);
+    }
+  // the reference's evaluation at beta: sum (plus DBL_MIN) and distance of the entropy from the target
+  auto evaluate = [&](double beta, double* diff) -> double {
     double sp = 0.0, ent = 0.0;
     for (int j = lane; j < k; j += 32) {
       const double d = seg_dist(sg, j, i);
@@ -144,10 +176,39 @@ __global__ void transform_row_p_kernel(const TransformSegment* __restrict__ segs
       ent += beta * (s * pv);
     }
     sp = warp_sum(sp);
-    ent = warp_sum(ent);
+    const double sum = DBL_MIN + sp;
+    if (diff) *diff = warp_sum(ent) / sum + log(sum) - target;
+    return sum;
+  };
+  double beta = 1.0, bmin = -DBL_MAX, bmax = DBL_MAX, beta_eval = 1.0;
+  const Float2Sum goal = split(-target);
+  for (int it = 0; it < 200; ++it) {
+    double diff = 0.0;
+    bool exact = wide || beta > 1.0e30;
+    if (!exact) {
+      const Float2Sum b = split(-beta);
+      Float2Sum sp{0.0f, 0.0f}, sw{0.0f, 0.0f};
+      for (int j = lane; j < k; j += 32) {
+        Float2Sum s;
+        if (cache) {
+          const float2 c = cache[j];
+          s = Float2Sum{c.x, c.y};
+        } else {
+          const double d = seg_dist(sg, j, i);
+          s = split(d * d - mn);
+        }
+        const Float2Sum pv = exp_two(mul(s, b), exp_table);
+        sp = add(sp, pv);
+        sw = add(sw, mul(s, pv));
+      }
+      sp = warp_sum(sp);
+      sw = warp_sum(sw);
+      const Float2Sum nb{-b.hi, -b.lo};
+      diff = value(add(add(divide(mul(sw, nb), sp), log_two(sp, log_table)), goal));
+      exact = !(fabs(fabs(diff) - 1e-5) > 1e-9);
+    }
+    if (exact) evaluate(beta, &diff);
     beta_eval = beta;
-    sum_p = DBL_MIN + sp;
-    const double diff = ent / sum_p + log(sum_p) - target;
     if (fabs(diff) < 1e-5) break;
     if (diff > 0.0) {
       bmin = beta;
@@ -158,6 +219,7 @@ __global__ void transform_row_p_kernel(const TransformSegment* __restrict__ segs
     }
     if (!isfinite(beta)) break;
   }
+  const double sum_p = evaluate(beta_eval, nullptr);
   if (!isfinite(sum_p) || sum_p <= DBL_MIN) {
     // every term underflowed: uniform over the neighbours tied at the minimum distance
     const double tol = DBL_EPSILON * fmax(1.0, mn);
@@ -183,16 +245,34 @@ __global__ void transform_row_p_kernel(const TransformSegment* __restrict__ segs
 // Warp per query: neighbour coordinates, initial layout and optimizer state.
 // init_mode 0 = supplied y_init, 1 = median, 2 = inverse-distance weighted; a segment that
 // carries y_init uses it whatever the mode.
-__global__ void transform_init_kernel(const float2* __restrict__ ref, const double2* __restrict__ ref_d,
-                                      const TransformSegment* __restrict__ segs, int nseg, long long total_q,
-                                      int init_mode) {
+__device__ __forceinline__ long long order_key(double v) {
+  const long long b = __double_as_longlong(v + 0.0);  // -0 counts as 0
+  return b < 0 ? b ^ 0x7fffffffffffffffll : b;
+}
+__device__ __forceinline__ double key_value(long long k) {
+  return __longlong_as_double(k < 0 ? k ^ 0x7fffffffffffffffll : k);
+}
+__device__ __forceinline__ long long warp_max_key(long long v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const long long w = __shfl_xor_sync(0xffffffffu, v, o);
+    v = w > v ? w : v;
+  }
+  return v;
+}
+
+__global__ void __launch_bounds__(kPrepareWarps * 32)
+transform_init_kernel(const float2* __restrict__ ref, const double2* __restrict__ ref_d,
+                      const TransformSegment* __restrict__ segs, int nseg, long long total_q, int init_mode,
+                      int cache_k) {
+  extern __shared__ longlong2 s_keys[];  // kPrepareWarps x cache_k
   const int lane = threadIdx.x & 31;
   const long long q = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (q >= total_q) return;
   const TransformSegment& sg = segs[find_segment(segs, nseg, q)];
   const int i = (int)(q - sg.query_begin), k = sg.k, nq = sg.nq;
   float2* nrow = sg.nb + (long long)i * k;
-  for (int j = lane; j < k; j += 32) nrow[j] = ref[sg.idx[(long long)j * nq + i] - sg.offset];
+  for (int j = lane; j < k; j += 32) nrow[j] = ref[seg_index(sg, j, i)];
   double y[2];
   if (sg.y_init) {
     y[0] = sg.y_init[i];
@@ -200,7 +280,7 @@ __global__ void transform_init_kernel(const float2* __restrict__ ref, const doub
   } else if (init_mode == 2) {
     double nx = 0.0, ny = 0.0, den = 0.0;
     for (int j = lane; j < k; j += 32) {
-      const double2 r = ref_d[sg.idx[(long long)j * nq + i] - sg.offset];
+      const double2 r = ref_d[seg_index(sg, j, i)];
       const double w = 1.0 / (fmax(0.0, seg_dist(sg, j, i)) + 1e-6);
       nx += w * r.x;
       ny += w * r.y;
@@ -210,16 +290,56 @@ __global__ void transform_init_kernel(const float2* __restrict__ ref, const doub
     y[0] = warp_sum(nx) / den;
     y[1] = warp_sum(ny) / den;
   } else {
-    // median per dimension: the values of rank k/2 (and k/2 - 1 for even k), by counting ranks
+    // median per dimension: the values of rank k/2 (and k/2 - 1 for even k), by counting ranks. The
+    // neighbours' coordinates are compared as integers of the same order, from shared memory (FP64
+    // comparisons of values fetched again for every pair took 0.75 ms for 10,000 queries of 90
+    // neighbours); rows too long for it, or with a NaN, are counted in FP64.
     const int mid = k / 2;
-    for (int d = 0; d < 2; ++d) {
+    bool nan = false;
+    if (k <= cache_k) {
+      longlong2* keys = s_keys + (threadIdx.x >> 5) * cache_k;
+      for (int j = lane; j < k; j += 32) {
+        const double2 r = ref_d[seg_index(sg, j, i)];
+        nan |= isnan(r.x) || isnan(r.y);
+        keys[j] = make_longlong2(order_key(r.x), order_key(r.y));
+      }
+      nan = __any_sync(0xffffffffu, nan);
+      __syncwarp();
+      if (!nan) {
+        // the key of each rank, from the lane that holds it; smaller than every key elsewhere
+        long long hi_x = LLONG_MIN, lo_x = LLONG_MIN, hi_y = LLONG_MIN, lo_y = LLONG_MIN;
+        for (int j = lane; j < k; j += 32) {
+          const longlong2 v = keys[j];
+          int less_x = 0, upto_x = 0, less_y = 0, upto_y = 0;
+#pragma unroll 4
+          for (int u = 0; u < k; ++u) {
+            const longlong2 w = keys[u];
+            less_x += w.x < v.x;
+            upto_x += w.x <= v.x;
+            less_y += w.y < v.y;
+            upto_y += w.y <= v.y;
+          }
+          if (less_x <= mid && mid < upto_x) hi_x = v.x;
+          if (less_x <= mid - 1 && mid - 1 < upto_x) lo_x = v.x;
+          if (less_y <= mid && mid < upto_y) hi_y = v.y;
+          if (less_y <= mid - 1 && mid - 1 < upto_y) lo_y = v.y;
+        }
+        hi_x = warp_max_key(hi_x);
+        lo_x = warp_max_key(lo_x);
+        hi_y = warp_max_key(hi_y);
+        lo_y = warp_max_key(lo_y);
+        y[0] = (k & 1) ? key_value(hi_x) : 0.5 * (key_value(hi_x) + key_value(lo_x));
+        y[1] = (k & 1) ? key_value(hi_y) : 0.5 * (key_value(hi_y) + key_value(lo_y));
+      }
+    }
+    for (int d = 0; d < 2 && (nan || k > cache_k); ++d) {
       double hi_v = -DBL_MAX, lo_v = -DBL_MAX;
       for (int j = lane; j < k; j += 32) {
-        const double2 rv = ref_d[sg.idx[(long long)j * nq + i] - sg.offset];
+        const double2 rv = ref_d[seg_index(sg, j, i)];
         const double v = d ? rv.y : rv.x;
         int less = 0, equal = 0;
         for (int u = 0; u < k; ++u) {
-          const double2 ru = ref_d[sg.idx[(long long)u * nq + i] - sg.offset];
+          const double2 ru = ref_d[seg_index(sg, u, i)];
           const double w = d ? ru.y : ru.x;
           less += w < v;
           equal += w == v;
@@ -258,21 +378,41 @@ __device__ __forceinline__ void two_sum_add(float& hi, float& lo, float u) {
 
 __device__ __forceinline__ float sign_f(float v) { return v == 0.0f ? 0.0f : (v < 0.0f ? -1.0f : 1.0f); }
 
+// Correctly rounded 1 / x for x in [1, 2^126): one Newton step by fused multiply-add on an approximation
+// within one unit in the last place rounds correctly (Markstein 1990); larger x, where the result is
+// below 1.2e-38, give 0. Free of the branch to a slow path, so that several pairs are in flight.
+__device__ __forceinline__ float reciprocal(float x) {
+  float r;
+  const float c = fminf(x, 3.4e38f);
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(c));
+  return __fmaf_rn(r, __fmaf_rn(-c, r, 1.0f), r);
+}
+
 // One repulsion pair: q, q^2 (y - r) with the compensated query position.
 __device__ __forceinline__ void repulse(float2 rr, float yhx, float yhy, float ylx, float yly, float& fz, float& fx,
                                         float& fy) {
   const float dx = (yhx - rr.x) + ylx, dy = (yhy - rr.y) + yly;
-  const float qv = __frcp_rn(1.0f + dx * dx + dy * dy);
+  const float qv = reciprocal(__fmaf_rn(dy, dy, __fmaf_rn(dx, dx, 1.0f)));
   const float q2 = qv * qv;
   fz += qv;
   fx += q2 * dx;
   fy += q2 * dy;
 }
 
+// One attractive term: p q (y - r).
+__device__ __forceinline__ void attract(float2 nb, float pj, float yhx, float yhy, float ylx, float yly, float& ax,
+                                        float& ay) {
+  const float dx = (yhx - nb.x) + ylx, dy = (yhy - nb.y) + yly;
+  const float c = pj * reciprocal(__fmaf_rn(dy, dy, __fmaf_rn(dx, dx, 1.0f)));
+  ax += c * dx;
+  ay += c * dy;
+}
+
 // MODE 0: sampled repulsion; 1: exact, whole reference staged in shared memory once;
 // 2: exact, reference streamed through shared memory in tiles every iteration.
 constexpr int kTransformWarps = 8;
 constexpr int kTransformTile = 4096;
+constexpr int kNeighbourRegs = 4;  // neighbours per lane kept in registers for all iterations
 
 template <int MODE>
 __global__ void __launch_bounds__(kTransformWarps * 32)
@@ -305,6 +445,16 @@ transform_iterate_kernel(const float2* __restrict__ ref, const TransformSegment*
   const int s_begin = (int)(((long long)lane * tp.n_negatives) >> 5);
   const int s_end = (int)(((long long)(lane + 1) * tp.n_negatives) >> 5);
   const std::uint32_t salt = (std::uint32_t)(i + 1) * 0x9e3779b9u;
+  // the attractive terms' inputs do not change between iterations
+  const bool in_regs = k <= 32 * kNeighbourRegs;
+  float2 nbr[kNeighbourRegs];
+  float pr[kNeighbourRegs];
+#pragma unroll
+  for (int u = 0; u < kNeighbourRegs; ++u) {
+    const int j = lane + 32 * u;
+    nbr[u] = in_regs && j < k ? nrow[j] : make_float2(0.0f, 0.0f);
+    pr[u] = in_regs && j < k ? prow[j] : 0.0f;
+  }
   for (int it = it_begin; it < it_end; ++it) {
     const bool early = it < tp.early_iter;
     const float exg = early ? tp.early_exag : tp.exag;
@@ -328,13 +478,14 @@ transform_iterate_kernel(const float2* __restrict__ ref, const TransformSegment*
     } else if (MODE == 0) {
       const std::uint32_t iter_seed = (std::uint32_t)tp.seed + 65537u * (std::uint32_t)(it + 1);
       std::uint32_t s = gf2_apply(sjump, lane, mix_u32(iter_seed ^ salt));
-#pragma unroll 4
+#pragma unroll 8
       for (int m = s_begin; m < s_end; ++m) {
         s = xorshift32_step(s);
         const int r = (int)(((unsigned long long)s * (unsigned long long)tp.n_ref) >> 32);
         repulse(__ldg(&ref[r]), yhx, yhy, ylx, yly, fz, fx, fy);
       }
     } else if (MODE == 1) {
+#pragma unroll 8
       for (int t = lane; t < tp.n_ref; t += 32) repulse(sref[t], yhx, yhy, ylx, yly, fz, fx, fy);
     } else {
       for (int t0 = 0; t0 < tp.n_ref; t0 += kTransformTile) {
@@ -342,17 +493,17 @@ transform_iterate_kernel(const float2* __restrict__ ref, const TransformSegment*
         __syncthreads();
         for (int t = threadIdx.x; t < cnt; t += blockDim.x) sref[t] = ref[t0 + t];
         __syncthreads();
+#pragma unroll 8
         for (int t = lane; t < cnt; t += 32) repulse(sref[t], yhx, yhy, ylx, yly, fz, fx, fy);
       }
     }
     float ax = 0.0f, ay = 0.0f;
-    for (int j = lane; j < k; j += 32) {
-      const float2 nb = nrow[j];
-      const float pj = prow[j];
-      const float dx = (yhx - nb.x) + ylx, dy = (yhy - nb.y) + yly;
-      const float c = pj * __frcp_rn(1.0f + dx * dx + dy * dy);
-      ax += c * dx;
-      ay += c * dy;
+    if (in_regs) {
+#pragma unroll
+      for (int u = 0; u < kNeighbourRegs; ++u)
+        if (lane + 32 * u < k) attract(nbr[u], pr[u], yhx, yhy, ylx, yly, ax, ay);
+    } else {
+      for (int j = lane; j < k; j += 32) attract(nrow[j], prow[j], yhx, yhy, ylx, yly, ax, ay);
     }
     fz = warp_sum(fz);
     fx = warp_sum(fx);
@@ -360,9 +511,10 @@ transform_iterate_kernel(const float2* __restrict__ ref, const TransformSegment*
     ax = warp_sum(ax);
     ay = warp_sum(ay);
     const float zq = fmaxf(fz, FLT_MIN);
-    float gx = exg * ax - fx / zq;
-    float gy = exg * ay - fy / zq;
-    const float g2 = gx * gx + gy * gy;
+    // roundings written out, so that a result's bits do not depend on the code around them
+    float gx = __fsub_rn(__fmul_rn(exg, ax), fx / zq);
+    float gy = __fsub_rn(__fmul_rn(exg, ay), fy / zq);
+    const float g2 = __fmaf_rn(gx, gx, __fmul_rn(gy, gy));
     if (g2 > tp.max_grad * tp.max_grad) {
       const float sc = tp.max_grad / (sqrtf(g2) + 1e-12f);
       gx *= sc;
@@ -372,9 +524,9 @@ transform_iterate_kernel(const float2* __restrict__ ref, const TransformSegment*
     gny = sign_f(upy) != sign_f(gy) ? gny + 0.2f : gny * 0.8f + 0.01f;
     gnx = fmaxf(gnx, 0.01f);
     gny = fmaxf(gny, 0.01f);
-    upx = mom * upx - tp.lr * gnx * gx;
-    upy = mom * upy - tp.lr * gny * gy;
-    const float s2 = upx * upx + upy * upy;
+    upx = __fmaf_rn(mom, upx, -__fmul_rn(__fmul_rn(tp.lr, gnx), gx));
+    upy = __fmaf_rn(mom, upy, -__fmul_rn(__fmul_rn(tp.lr, gny), gy));
+    const float s2 = __fmaf_rn(upx, upx, __fmul_rn(upy, upy));
     if (s2 > tp.max_step * tp.max_step) {
       const float sc = tp.max_step / (sqrtf(s2) + 1e-12f);
       upx *= sc;
@@ -395,11 +547,17 @@ transform_iterate_kernel(const float2* __restrict__ ref, const TransformSegment*
 
 // ------------------------------------------------------------------ host launchers
 void transform_prepare(const float2* ref, const double2* ref_d, const TransformSegment* segs, int nseg,
-                       long long total_q, const TransformParams& tp, cudaStream_t s) {
-  const int blocks = ceil_div(total_q * 32, 256);
-  transform_row_p_kernel<<<blocks, 256, 0, s>>>(segs, nseg, total_q, tp.perplexity);
+                       long long total_q, int max_k, const TransformParams& tp, cudaStream_t s) {
+  const int blocks = ceil_div(total_q, kPrepareWarps), threads = kPrepareWarps * 32;
+  // shared memory for the longest row of the launch, where that is short enough
+  const int row_k = max_k <= kRowCache ? max_k : 0;
+  static_assert(kPrepareWarps * kRowCache * sizeof(float2) + 4096 <= 48 * 1024, "row cache");
+  transform_row_p_kernel<<<blocks, threads, kPrepareWarps * row_k * sizeof(float2), s>>>(
+      segs, nseg, total_q, std::log(tp.perplexity), row_k);
   FE_LAUNCH("transform_row_p_kernel");
-  transform_init_kernel<<<blocks, 256, 0, s>>>(ref, ref_d, segs, nseg, total_q, tp.init_mode);
+  const int key_k = max_k <= kRowCache / 2 ? max_k : 0;
+  transform_init_kernel<<<blocks, threads, kPrepareWarps * key_k * sizeof(longlong2), s>>>(
+      ref, ref_d, segs, nseg, total_q, tp.init_mode, key_k);
   FE_LAUNCH("transform_init_kernel");
 }
 
@@ -411,8 +569,10 @@ void transform_iterate(const float2* ref, const TransformSegment* segs, int nseg
     cudaFuncSetAttribute(transform_iterate_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)(kTransformSmemRefs * sizeof(float2)));
   });
-  const int blocks = ceil_div(total_q, kTransformWarps);
-  const int threads = kTransformWarps * 32;
+  // few queries: fewer warps a block, so that every SM has some (300 queries: 2 a block instead of 8)
+  const int warps = (int)std::max<long long>(1, std::min<long long>(kTransformWarps, ceil_div(total_q, sm_count())));
+  const int blocks = ceil_div(total_q, warps);
+  const int threads = warps * 32;
   if (!tp.exact) {
     transform_iterate_kernel<0><<<blocks, threads, 0, s>>>(ref, segs, nseg, total_q, tp, jump, it_begin, it_end);
   } else if (tp.n_ref <= kTransformSmemRefs) {
@@ -564,7 +724,7 @@ extern "C" int fastembedr_cuda_transform_tsne(const double* reference_layout, in
     const fe::XorshiftJump jump = fe::xorshift_jump_table(tp.n_negatives);
     FE_CUDA(cudaMemcpyAsync(d_jump, &jump, sizeof(jump), cudaMemcpyHostToDevice, s));
     fe::transform_upload_reference(d_ref_cm, n_reference, d_ref, d_ref_d, s);
-    fe::transform_prepare(d_ref, d_ref_d, d_seg, 1, n_query, tp, s);
+    fe::transform_prepare(d_ref, d_ref_d, d_seg, 1, n_query, k, tp, s);
     const int chunk = fe::transform_chunk(n_query, tp, k);
     for (int it = 0; it < tp.iter_total; it += chunk)
       fe::transform_iterate(d_ref, d_seg, 1, n_query, tp, d_jump, it, std::min(tp.iter_total, it + chunk), s);

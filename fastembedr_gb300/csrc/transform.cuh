@@ -41,6 +41,7 @@ struct TransformSegment {
   double* out;             // column-major n_query x 2 result
   long long query_begin;   // first warp of this segment within the launch
   int nq, k, offset;
+  int row_major = 0;       // idx and dist are row-major n_query x k instead
 };
 
 // Lane l of a warp draws samples [l*n/32, (l+1)*n/32) of the reference's per-query xorshift32
@@ -54,11 +55,11 @@ XorshiftJump xorshift_jump_table(int n_negatives);
 // Bytes of device memory one query of width k needs in a segment (excluding inputs).
 std::size_t transform_query_bytes(int k);
 
-// Prepare: per-query P (FP64 bisection of compute_row_probabilities_flat), neighbour
-// coordinates and the initial layout. `segs` is a device array of `nseg` segments covering
-// `total_q` queries.
+// Prepare: per-query P (bisection of compute_row_probabilities_flat), neighbour coordinates and the
+// initial layout. `segs` is a device array of `nseg` segments covering `total_q` queries of at most
+// `max_k` neighbours.
 void transform_prepare(const float2* ref, const double2* ref_d, const TransformSegment* segs, int nseg,
-                       long long total_q, const TransformParams& tp, cudaStream_t s);
+                       long long total_q, int max_k, const TransformParams& tp, cudaStream_t s);
 // Iterations [it_begin, it_end) for every query; writes `out` when it_end == iter_total.
 void transform_iterate(const float2* ref, const TransformSegment* segs, int nseg, long long total_q,
                        const TransformParams& tp, const XorshiftJump* jump, int it_begin, int it_end,

@@ -230,10 +230,10 @@ class TransformServer {
     FE_CUDA(cudaMemcpyAsync(slot.d_segs, slot.h_segs, sizeof(TransformSegment) * nseg, cudaMemcpyHostToDevice, s));
     slot.group_queries = total;
     FE_CUDA(cudaEventRecord(slot.ev_begin, s));
-    transform_prepare(ref, ref_d, slot.d_segs, nseg, total, tp, s);
-    FE_CUDA(cudaEventRecord(slot.ev_iterate, s));
     int max_k = 1;
     for (Request* r : slot.reqs) max_k = std::max(max_k, r->k);
+    transform_prepare(ref, ref_d, slot.d_segs, nseg, total, max_k, tp, s);
+    FE_CUDA(cudaEventRecord(slot.ev_iterate, s));
     const int chunk = transform_chunk(total, tp, max_k);
     int n_launch = 2;
     for (int it = 0; it < tp.iter_total; it += chunk, ++n_launch)
