@@ -28,6 +28,14 @@ SIGNATURES = {
     "fastembedr_cuda_opentsne_fft_grid_size": (I, [I]),
     "fastembedr_cuda_opentsne_fft_from_knn_float": (I, [vp, vp, vp, I, I, I, I, F, I, I, F, F, F, I, F, F, F, F, U,
                                                         I, vp]),
+    "fastembedr_cuda_opentsne_fft_from_knn_rows_float": (I, [vp, vp, vp, I, I, I, I, F, I, I, F, F, F, I, F, F, F, F,
+                                                             U, I, vp]),
+    "fastembedr_cuda_umap_from_knn_rows": (I, [vp, vp, vp, I, I, I, I, I, F, F, F, U, vp]),
+    "fastembedr_cuda_umap_knn_spectral_rows": (I, [vp, vp, I, I, I, I, I, F, F, F, I, D, U, vp]),
+    "fastembedr_cuda_tsne_pca_init_rows": (I, [vp, I, I, I, vp]),
+    "fastembedr_cuda_transform_tsne_rows": (I, [vp, I, vp, vp, I, I, vp, I, C.c_char_p, D, I, I, D, D, D, D, D, D, D,
+                                                I, I, I, vp]),
+    "fastembedr_transform_server_submit_rows": (I, [vp, vp, vp, I, I, C.POINTER(C.c_ulonglong)]),
     "fastembedr_cuda_opentsne_fft_from_knn": (I, [vp, vp, vp, I, I, I, I, F, I, I, F, F, F, I, F, F, F, F, U, I, vp]),
     "fastembedr_cuda_opentsne_fft_from_device_knn_float": (I, [vp, vp, vp, I, I, I, I, F, I, I, F, F, F, I, F, F, F, F,
                                                                U, I, vp]),

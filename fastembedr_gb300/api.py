@@ -43,6 +43,27 @@ def knn_index_offset(indices) -> int:
     return 1 if idx.min() >= 1 and idx.max() <= n else 0
 
 
+def _host_matrix(a, dtype):
+    """(array, rows): the matrix in the order it has, row-major unless it is column-major already (the
+    library reads either; a transpose on the host costs more than the copy to the device)."""
+    a = np.asarray(a, dtype)
+    if a.flags.f_contiguous and not a.flags.c_contiguous:
+        return a, False
+    return np.ascontiguousarray(a), True
+
+
+def _host_knn(indices, distances, dist_dtype=np.float32):
+    """(indices, distances, rows, index offset) for the library: both in one order; int32 labels are
+    left to the library to detect (-1), others are detected before the conversion."""
+    src = np.asarray(indices)
+    idx, rows = _host_matrix(src, np.int32)
+    dist, dist_rows = _host_matrix(distances, dist_dtype)
+    if rows != dist_rows:
+        idx, dist, rows = np.ascontiguousarray(idx), np.ascontiguousarray(dist), True
+    detect = rows and src.dtype == np.int32 and src.size > 0
+    return idx, dist, rows, -1 if detect else knn_index_offset(src)
+
+
 @dataclass
 class TsneFit:
     layout: np.ndarray
@@ -105,12 +126,12 @@ def tsne_knn(indices, distances, n_neighbors=None, perplexity=None, n_components
         raise ValueError("`Y_init` must contain only finite coordinates.")
     out = np.zeros((n, 2), np.float32)
     lib = _lib.require_gpu()
-    idx_cm = _colmajor(idx, np.int32)
-    dist_cm = _colmajor(dist, np.float32)
-    st = lib.fastembedr_cuda_opentsne_fft_from_knn_float(
-        idx_cm.ctypes.data, dist_cm.ctypes.data, init.ctypes.data, int(has_init), n, k, 2, perp, ee_iter, nn_iter,
-        ee, ex, lr_value, lr_auto, float(initial_momentum), float(final_momentum), float(min_gain), msn,
-        int(seed) & 0xFFFFFFFF, knn_index_offset(idx), out.ctypes.data)
+    h_idx, h_dist, rows, offset = _host_knn(idx, dist)
+    fit = (lib.fastembedr_cuda_opentsne_fft_from_knn_rows_float if rows
+           else lib.fastembedr_cuda_opentsne_fft_from_knn_float)
+    st = fit(h_idx.ctypes.data, h_dist.ctypes.data, init.ctypes.data, int(has_init), n, k, 2, perp, ee_iter, nn_iter,
+             ee, ex, lr_value, lr_auto, float(initial_momentum), float(final_momentum), float(min_gain), msn,
+             int(seed) & 0xFFFFFFFF, offset, out.ctypes.data)
     _lib.check(st, "CUDA openTSNE FFT-grid")
     lr_early = n / ee if lr_auto else lr_value
     lr_normal = n / max(ex, 1.0) if lr_auto else lr_value
@@ -134,10 +155,12 @@ def tsne_pca_init(data):
     centred and scaled so the larger standard deviation is 1e-4. (n, 2) float32."""
     x = np.asarray(data)
     is_double = x.dtype != np.float32
-    xc = np.asfortranarray(x, np.float64 if is_double else np.float32)
+    xc, rows = _host_matrix(x, np.float64 if is_double else np.float32)
     n, p = xc.shape
     out = np.zeros((n, 2), np.float32)
-    st = _lib.require_gpu().fastembedr_cuda_tsne_pca_init(xc.ctypes.data, int(is_double), n, p, out.ctypes.data)
+    lib = _lib.require_gpu()
+    start = lib.fastembedr_cuda_tsne_pca_init_rows if rows else lib.fastembedr_cuda_tsne_pca_init
+    st = start(xc.ctypes.data, int(is_double), n, p, out.ctypes.data)
     _lib.check(st, "CUDA PCA initialization")
     return out
 
@@ -540,11 +563,12 @@ def umap_knn(indices, distances, init="spectral", n_components=2, seed=42, n_epo
     if isinstance(init, str) and init == "spectral":
         rounds = umap_spectral_n_iter(n, k) if spectral_n_iter is None else int(spectral_n_iter)
         out = np.zeros((n, 2), np.float32)
-        idx_cm, dist_cm = _colmajor(idx, np.int32), _colmajor(distances, np.float32)
-        st = _lib.require_gpu().fastembedr_cuda_umap_knn_spectral(
-            idx_cm.ctypes.data, dist_cm.ctypes.data, n, k, knn_index_offset(idx), epochs, int(negative_sample_rate),
-            float(learning_rate), float(min_dist), float(repulsion_strength), rounds, float(init_scale),
-            int(seed) & 0xFFFFFFFF, out.ctypes.data)
+        h_idx, h_dist, rows, offset = _host_knn(idx, distances)
+        lib = _lib.require_gpu()
+        fit = lib.fastembedr_cuda_umap_knn_spectral_rows if rows else lib.fastembedr_cuda_umap_knn_spectral
+        st = fit(h_idx.ctypes.data, h_dist.ctypes.data, n, k, offset, epochs, int(negative_sample_rate),
+                 float(learning_rate), float(min_dist), float(repulsion_strength), rounds, float(init_scale),
+                 int(seed) & 0xFFFFFFFF, out.ctypes.data)
         _lib.check(st, "CUDA UMAP")
         config = dict(method="umap", backend="cuda", n=n, k=k, n_epochs=epochs, min_dist=float(min_dist),
                       negative_sample_rate=int(negative_sample_rate), learning_rate=float(learning_rate),
@@ -583,11 +607,10 @@ def umap_knn(indices, distances, init="spectral", n_components=2, seed=42, n_epo
         raise ValueError("init row count must match the KNN graph")
     out = np.zeros((n, 2), np.float32)
     lib = _lib.require_gpu()
-    idx_cm, dist_cm = _colmajor(idx, np.int32), _colmajor(distances, np.float32)
-    st = lib.fastembedr_cuda_umap_from_knn(idx_cm.ctypes.data, dist_cm.ctypes.data, y0.ctypes.data, n, k,
-                                           knn_index_offset(idx), epochs, int(negative_sample_rate),
-                                           float(learning_rate), float(min_dist), float(repulsion_strength),
-                                           int(seed) & 0xFFFFFFFF, out.ctypes.data)
+    h_idx, h_dist, rows, offset = _host_knn(idx, distances)
+    fit = lib.fastembedr_cuda_umap_from_knn_rows if rows else lib.fastembedr_cuda_umap_from_knn
+    st = fit(h_idx.ctypes.data, h_dist.ctypes.data, y0.ctypes.data, n, k, offset, epochs, int(negative_sample_rate),
+             float(learning_rate), float(min_dist), float(repulsion_strength), int(seed) & 0xFFFFFFFF, out.ctypes.data)
     _lib.check(st, "CUDA UMAP")
     config = dict(method="umap", backend="cuda", n=n, k=k, n_epochs=epochs, min_dist=float(min_dist),
                   negative_sample_rate=int(negative_sample_rate), learning_rate=float(learning_rate),
@@ -654,15 +677,19 @@ def transform_tsne(reference_layout, knn, k=None, perplexity=5.0, initialization
             raise ValueError("`Y_init` must have one row per query and the same columns as `reference_layout`.")
         init = 1
     out = np.zeros((2, nq), np.float64)  # column-major n_query x 2
-    ref_cm, idx_cm, dist_cm = _colmajor(ref, np.float64), _colmajor(idx, np.int32), _colmajor(dist, np.float64)
+    ref_cm = _colmajor(ref, np.float64)
+    h_idx, rows = _host_matrix(idx, np.int32)
+    h_dist, dist_rows = _host_matrix(dist, np.float64)
+    if rows != dist_rows:
+        h_idx, h_dist, rows = np.ascontiguousarray(h_idx), np.ascontiguousarray(h_dist), True
     y0_cm = _colmajor(y0, np.float64)
     lib = _lib.require_gpu()
-    st = lib.fastembedr_cuda_transform_tsne(ref_cm.ctypes.data, n_ref, idx_cm.ctypes.data, dist_cm.ctypes.data, nq, kk,
-                                            y0_cm.ctypes.data if init else None, init, initialization.encode(),
-                                            perplexity, n_iter, early, float(learning_rate),
-                                            float(early_exaggeration), float(exaggeration), float(initial_momentum),
-                                            float(final_momentum), float(max_grad_norm), float(max_step_norm),
-                                            n_negatives, threshold, int(seed), out.ctypes.data)
+    place = lib.fastembedr_cuda_transform_tsne_rows if rows else lib.fastembedr_cuda_transform_tsne
+    st = place(ref_cm.ctypes.data, n_ref, h_idx.ctypes.data, h_dist.ctypes.data, nq, kk,
+               y0_cm.ctypes.data if init else None, init, initialization.encode(), perplexity, n_iter, early,
+               float(learning_rate), float(early_exaggeration), float(exaggeration), float(initial_momentum),
+               float(final_momentum), float(max_grad_norm), float(max_step_norm), n_negatives, threshold, int(seed),
+               out.ctypes.data)
     _lib.check(st, "CUDA t-SNE transform")
     n_neg_eff = min(n_negatives, n_ref)
     exact = n_ref <= max(threshold, 1) or n_neg_eff >= n_ref
@@ -715,13 +742,16 @@ class TransformServer:
         self._shape = {}
 
     def submit(self, indices, distances) -> int:
-        idx = _colmajor(np.asarray(indices), np.int32)
-        dist = _colmajor(np.asarray(distances), np.float32)
+        idx, rows = _host_matrix(indices, np.int32)
+        dist, dist_rows = _host_matrix(distances, np.float32)
         if idx.shape != dist.shape or idx.ndim != 2:
             raise ValueError("KNN `indices` and `distances` must have the same dimensions.")
+        if rows != dist_rows:
+            idx, dist, rows = np.ascontiguousarray(idx), np.ascontiguousarray(dist), True
         rid = C.c_ulonglong()
-        st = self._lib.fastembedr_transform_server_submit(self._h, idx.ctypes.data, dist.ctypes.data, idx.shape[0],
-                                                          idx.shape[1], C.byref(rid))
+        submit = (self._lib.fastembedr_transform_server_submit_rows if rows
+                  else self._lib.fastembedr_transform_server_submit)
+        st = submit(self._h, idx.ctypes.data, dist.ctypes.data, idx.shape[0], idx.shape[1], C.byref(rid))
         _lib.check(st, "CUDA t-SNE transform request")
         self._shape[rid.value] = idx.shape[0]
         return rid.value

@@ -24,6 +24,7 @@
 #include <climits>
 #include <cmath>
 #include <cstring>
+#include <limits>
 #include <mutex>
 #include <random>
 #include <string>
@@ -77,11 +78,44 @@ void gf2_power(long long n, std::uint32_t* out) {
 }
 }  // namespace
 
+// Lane l's matrix is the step matrix to the power l n / 32: each from the one before by one of the two
+// powers that occur as differences.
 XorshiftJump xorshift_jump_table(int n_negatives) {
   XorshiftJump t;
-  for (int lane = 0; lane < 32; ++lane) gf2_power((long long)lane * n_negatives / 32, t.col[lane]);
+  std::uint32_t low[32], high[32];
+  const long long base = n_negatives / 32;
+  gf2_power(base, low);
+  gf2_power(base + 1, high);
+  gf2_power(0, t.col[0]);
+  for (int lane = 1; lane < 32; ++lane) {
+    const long long step = (long long)lane * n_negatives / 32 - (long long)(lane - 1) * n_negatives / 32;
+    gf2_mul(step == base ? low : high, t.col[lane - 1], t.col[lane]);
+  }
   return t;
 }
+
+// Labels and distances of host queries, as resolve_reference_index_offset and the range checks of the
+// reference (src/tsne_neighbors.cpp:1371-1382, :2175-2185): returns the offset.
+template <typename DistT>
+int check_query_knn(const int* idx, const DistT* dist, std::size_t items, int n_ref) {
+  int lo = INT_MAX, hi = INT_MIN;
+  bool bad = false;
+  for (std::size_t t = 0; t < items; ++t) {
+    lo = std::min(lo, idx[t]);
+    hi = std::max(hi, idx[t]);
+  }
+  for (std::size_t t = 0; t < items; ++t) bad |= !(dist[t] >= DistT(0) && dist[t] <= std::numeric_limits<DistT>::max());
+  const int offset = lo >= 1 && hi <= n_ref ? 1 : 0;
+  if (!bad && lo - offset >= 0 && hi - offset < n_ref) return offset;
+  for (std::size_t t = 0; t < items; ++t) {  // the first offence names the error
+    const int r = idx[t] - offset;
+    if (r < 0 || r >= n_ref) throw Error("KNN indices are out of range for `reference_layout`.");
+    if (!std::isfinite(dist[t]) || dist[t] < DistT(0)) throw Error("KNN distances must be finite and non-negative.");
+  }
+  return offset;
+}
+template int check_query_knn<float>(const int*, const float*, std::size_t, int);
+template int check_query_knn<double>(const int*, const double*, std::size_t, int);
 
 std::size_t transform_query_bytes(int k) {
   return (std::size_t)k * (sizeof(float2) + sizeof(float)) + 2 * sizeof(float4) + 2 * sizeof(double) + 64;
@@ -647,13 +681,13 @@ int transform_chunk(long long n_query, const TransformParams& tp, int k) {
 
 }  // namespace fe
 
-extern "C" int fastembedr_cuda_transform_tsne(const double* reference_layout, int n_reference, const int* indices,
-                                              const double* distances, int n_query, int k, const double* y_init,
-                                              int init, const char* initialization, double perplexity, int n_iter,
-                                              int early_exaggeration_iter, double learning_rate,
-                                              double early_exaggeration, double exaggeration, double initial_momentum,
-                                              double final_momentum, double max_grad_norm, double max_step_norm,
-                                              int n_negatives, int exact_repulsion_threshold, int seed, double* out) {
+namespace {
+int transform_tsne(const double* reference_layout, int n_reference, const int* indices, const double* distances,
+                   bool rows, int n_query, int k, const double* y_init, int init, const char* initialization,
+                   double perplexity, int n_iter, int early_exaggeration_iter, double learning_rate,
+                   double early_exaggeration, double exaggeration, double initial_momentum, double final_momentum,
+                   double max_grad_norm, double max_step_norm, int n_negatives, int exact_repulsion_threshold,
+                   int seed, double* out) {
   return fe::guarded([&] {
     if (!reference_layout || !indices || !distances || !out || (init && !y_init))
       throw fe::Error("null CUDA t-SNE transform pointer");
@@ -666,20 +700,8 @@ extern "C" int fastembedr_cuda_transform_tsne(const double* reference_layout, in
         n_reference, n_negatives, exact_repulsion_threshold, perplexity, n_iter, early_exaggeration_iter,
         learning_rate, early_exaggeration, exaggeration, initial_momentum, final_momentum, max_grad_norm,
         max_step_norm, mode == 3 ? 0 : mode, seed);
-    // resolve_reference_index_offset and the range checks of src/tsne_neighbors.cpp:1371-1382, :2175-2185
     const long long items = (long long)n_query * k;
-    int lo = INT_MAX, hi = INT_MIN;
-    for (long long t = 0; t < items; ++t) {
-      lo = std::min(lo, indices[t]);
-      hi = std::max(hi, indices[t]);
-    }
-    const int offset = (lo >= 1 && hi <= n_reference) ? 1 : 0;
-    for (long long t = 0; t < items; ++t) {
-      const int r = indices[t] - offset;
-      if (r < 0 || r >= n_reference) throw fe::Error("KNN indices are out of range for `reference_layout`.");
-      if (!std::isfinite(distances[t]) || distances[t] < 0.0)
-        throw fe::Error("KNN distances must be finite and non-negative.");
-    }
+    const int offset = fe::check_query_knn(indices, distances, (std::size_t)items, n_reference);
     std::vector<double> random_init;
     if (mode == 3) {
       random_init.resize(2 * (std::size_t)n_query);
@@ -719,10 +741,13 @@ extern "C" int fastembedr_cuda_transform_tsne(const double* reference_layout, in
     if (have_init)
       FE_CUDA(cudaMemcpyAsync(d_init, y_init, sizeof(double) * 2 * n_query, cudaMemcpyHostToDevice, s));
     fe::TransformSegment seg{d_idx, nullptr, d_dist, have_init ? d_init : nullptr, d_nb, d_p, d_state, d_opt,
-                             d_out, 0, n_query, k, offset};
+                             d_out, 0, n_query, k, offset, rows ? 1 : 0};
     FE_CUDA(cudaMemcpyAsync(d_seg, &seg, sizeof(seg), cudaMemcpyHostToDevice, s));
-    const fe::XorshiftJump jump = fe::xorshift_jump_table(tp.n_negatives);
-    FE_CUDA(cudaMemcpyAsync(d_jump, &jump, sizeof(jump), cudaMemcpyHostToDevice, s));
+    fe::XorshiftJump jump;
+    if (!tp.exact) {  // the exact sweep draws no samples
+      jump = fe::xorshift_jump_table(tp.n_negatives);
+      FE_CUDA(cudaMemcpyAsync(d_jump, &jump, sizeof(jump), cudaMemcpyHostToDevice, s));
+    }
     fe::transform_upload_reference(d_ref_cm, n_reference, d_ref, d_ref_d, s);
     fe::transform_prepare(d_ref, d_ref_d, d_seg, 1, n_query, k, tp, s);
     const int chunk = fe::transform_chunk(n_query, tp, k);
@@ -731,4 +756,31 @@ extern "C" int fastembedr_cuda_transform_tsne(const double* reference_layout, in
     FE_CUDA(cudaMemcpyAsync(out, d_out, sizeof(double) * 2 * n_query, cudaMemcpyDeviceToHost, s));
     FE_CUDA(cudaStreamSynchronize(s));
   });
+}
+}  // namespace
+
+extern "C" int fastembedr_cuda_transform_tsne(const double* reference_layout, int n_reference, const int* indices,
+                                              const double* distances, int n_query, int k, const double* y_init,
+                                              int init, const char* initialization, double perplexity, int n_iter,
+                                              int early_exaggeration_iter, double learning_rate,
+                                              double early_exaggeration, double exaggeration, double initial_momentum,
+                                              double final_momentum, double max_grad_norm, double max_step_norm,
+                                              int n_negatives, int exact_repulsion_threshold, int seed, double* out) {
+  return transform_tsne(reference_layout, n_reference, indices, distances, false, n_query, k, y_init, init, initialization,
+                        perplexity, n_iter, early_exaggeration_iter, learning_rate, early_exaggeration, exaggeration,
+                        initial_momentum, final_momentum, max_grad_norm, max_step_norm, n_negatives,
+                        exact_repulsion_threshold, seed, out);
+}
+
+extern "C" int fastembedr_cuda_transform_tsne_rows(const double* reference_layout, int n_reference, const int* indices,
+                                              const double* distances, int n_query, int k, const double* y_init,
+                                              int init, const char* initialization, double perplexity, int n_iter,
+                                              int early_exaggeration_iter, double learning_rate,
+                                              double early_exaggeration, double exaggeration, double initial_momentum,
+                                              double final_momentum, double max_grad_norm, double max_step_norm,
+                                              int n_negatives, int exact_repulsion_threshold, int seed, double* out) {
+  return transform_tsne(reference_layout, n_reference, indices, distances, true, n_query, k, y_init, init, initialization,
+                        perplexity, n_iter, early_exaggeration_iter, learning_rate, early_exaggeration, exaggeration,
+                        initial_momentum, final_momentum, max_grad_norm, max_step_norm, n_negatives,
+                        exact_repulsion_threshold, seed, out);
 }

@@ -52,6 +52,10 @@ struct XorshiftJump {
 };
 XorshiftJump xorshift_jump_table(int n_negatives);
 
+// Checks a host KNN into n_ref references (throws) and returns its 0- or 1-based offset.
+template <typename DistT>
+int check_query_knn(const int* idx, const DistT* dist, std::size_t items, int n_ref);
+
 // Bytes of device memory one query of width k needs in a segment (excluding inputs).
 std::size_t transform_query_bytes(int k);
 

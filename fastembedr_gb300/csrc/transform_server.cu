@@ -99,8 +99,9 @@ using Clock = std::chrono::steady_clock;
 struct Request {
   unsigned long long id = 0;
   int nq = 0, k = 0, offset = 0;
-  std::vector<int> idx;        // column-major n_query x k
-  std::vector<float> dist;     // column-major n_query x k
+  bool rows = false;           // the KNN is row-major
+  std::vector<int> idx;        // n_query x k
+  std::vector<float> dist;     // n_query x k
   std::vector<double> init;    // column-major n_query x 2 (random start), or empty
   std::vector<double> result;  // column-major n_query x 2
   Clock::time_point submitted, finished;
@@ -218,6 +219,7 @@ class TransformServer {
       sg.nq = r->nq;
       sg.k = r->k;
       sg.offset = r->offset;
+      sg.row_major = r->rows ? 1 : 0;
       FE_CUDA(cudaMemcpyAsync(const_cast<int*>(sg.idx), h_idx, items * sizeof(int), cudaMemcpyHostToDevice, s));
       FE_CUDA(cudaMemcpyAsync(const_cast<float*>(sg.dist_f), h_dist, items * sizeof(float), cudaMemcpyHostToDevice,
                               s));
@@ -517,9 +519,8 @@ extern "C" int fastembedr_transform_server_create(const double* reference_layout
   });
 }
 
-extern "C" int fastembedr_transform_server_submit(fastembedr_transform_server* server, const int* indices,
-                                                  const float* distances, int n_query, int k,
-                                                  unsigned long long* request_id) {
+static int submit_request(fastembedr_transform_server* server, const int* indices, const float* distances, bool rows,
+                          int n_query, int k, unsigned long long* request_id) {
   return fe::guarded([&] {
     fe::TransformServer* sv = impl(server);
     if (!indices || !distances || !request_id) throw fe::Error("null CUDA t-SNE transform request pointer");
@@ -528,20 +529,10 @@ extern "C" int fastembedr_transform_server_submit(fastembedr_transform_server* s
     const std::size_t items = (std::size_t)n_query * k;
     r->nq = n_query;
     r->k = k;
+    r->rows = rows;
+    r->offset = fe::check_query_knn(indices, distances, items, sv->n_ref);
     r->idx.assign(indices, indices + items);
     r->dist.assign(distances, distances + items);
-    int lo = INT_MAX, hi = INT_MIN;
-    for (int v : r->idx) {
-      lo = std::min(lo, v);
-      hi = std::max(hi, v);
-    }
-    r->offset = (lo >= 1 && hi <= sv->n_ref) ? 1 : 0;
-    for (std::size_t t = 0; t < items; ++t) {
-      const int ref = r->idx[t] - r->offset;
-      if (ref < 0 || ref >= sv->n_ref) throw fe::Error("KNN indices are out of range for `reference_layout`.");
-      if (!std::isfinite(r->dist[t]) || r->dist[t] < 0.0f)
-        throw fe::Error("KNN distances must be finite and non-negative.");
-    }
     if (sv->init_mode == 3) {
       r->init.resize(2 * (std::size_t)n_query);
       fe::transform_random_init(sv->tp.seed, 0, n_query, r->init.data());
@@ -561,6 +552,18 @@ extern "C" int fastembedr_transform_server_submit(fastembedr_transform_server* s
     }
     sv->cv_work.notify_one();
   });
+}
+
+extern "C" int fastembedr_transform_server_submit(fastembedr_transform_server* server, const int* indices,
+                                                  const float* distances, int n_query, int k,
+                                                  unsigned long long* request_id) {
+  return submit_request(server, indices, distances, false, n_query, k, request_id);
+}
+
+extern "C" int fastembedr_transform_server_submit_rows(fastembedr_transform_server* server, const int* indices,
+                                                       const float* distances, int n_query, int k,
+                                                       unsigned long long* request_id) {
+  return submit_request(server, indices, distances, true, n_query, k, request_id);
 }
 
 extern "C" int fastembedr_transform_server_wait(fastembedr_transform_server* server, unsigned long long request_id,

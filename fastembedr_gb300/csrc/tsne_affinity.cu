@@ -53,16 +53,102 @@ void knn_flags_check(unsigned flags) {
   if (flags & 2u) throw Error("KNN distances must be finite and non-negative.");
 }
 
-void validate_knn(const int* d_idx, const float* d_dist, int n, int k, int offset, cudaStream_t s) {
-  unsigned* d_flags = nullptr;
-  FE_CUDA(cudaMallocAsync(&d_flags, sizeof(unsigned), s));
-  FE_CUDA(cudaMemsetAsync(d_flags, 0, sizeof(unsigned), s));
-  validate_knn_async(d_idx, d_dist, n, k, offset, d_flags, s);
-  unsigned flags = 0u;
-  FE_CUDA(cudaMemcpyAsync(&flags, d_flags, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
+// Smallest and largest label, and whether a distance is bad, in state[0 .. 2].
+__global__ void scan_knn_kernel(const int* __restrict__ idx, const float* __restrict__ dist, long long total,
+                                int* __restrict__ state) {
+  int lo = INT_MAX, hi = INT_MIN;
+  bool bad = false;
+  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
+       t += (long long)gridDim.x * blockDim.x) {
+    const int v = idx[t];
+    lo = min(lo, v);
+    hi = max(hi, v);
+    const float d = dist[t];
+    bad |= !isfinite(d) || d < 0.0f;
+  }
+  lo = __reduce_min_sync(0xffffffffu, lo);
+  hi = __reduce_max_sync(0xffffffffu, hi);
+  bad = __any_sync(0xffffffffu, bad);
+  if ((threadIdx.x & 31) == 0) {
+    atomicMin(state, lo);
+    atomicMax(state + 1, hi);
+    if (bad) atomicOr(state + 2, 1);
+  }
+}
+
+int validate_knn(const int* d_idx, const float* d_dist, int n, int k, int offset, cudaStream_t s) {
+  int* d_state = nullptr;
+  int h[3] = {INT_MAX, INT_MIN, 0};
+  FE_CUDA(cudaMallocAsync(&d_state, sizeof(h), s));
+  FE_CUDA(cudaMemcpyAsync(d_state, h, sizeof(h), cudaMemcpyHostToDevice, s));
+  const long long total = (long long)n * k;
+  scan_knn_kernel<<<std::max(1, std::min(ceil_div(total, 256), sm_count() * 8)), 256, 0, s>>>(d_idx, d_dist, total,
+                                                                                              d_state);
+  FE_LAUNCH("scan_knn_kernel");
+  FE_CUDA(cudaMemcpyAsync(h, d_state, sizeof(h), cudaMemcpyDeviceToHost, s));
   FE_CUDA(cudaStreamSynchronize(s));
-  FE_CUDA(cudaFreeAsync(d_flags, s));
-  knn_flags_check(flags);
+  FE_CUDA(cudaFreeAsync(d_state, s));
+  if (offset == kDetectLabels) offset = h[0] >= 1 && h[1] <= n ? 1 : 0;
+  const bool range = (long long)h[0] - offset < 0 || (long long)h[1] - offset >= n;
+  knn_flags_check((range ? 1u : 0u) | (h[2] ? 2u : 0u));
+  return offset;
+}
+
+// in: n x p row-major -> out: column-major, 32 x 32 tiles.
+template <typename In, typename Out>
+__global__ void __launch_bounds__(256)
+transpose_kernel(const In* __restrict__ in, int n, int p, Out* __restrict__ out) {
+  __shared__ Out tile[32][33];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const long long r0 = blockIdx.x * 32LL;
+  const int c0 = blockIdx.y * 32;
+#pragma unroll
+  for (int u = 0; u < 32; u += 8)
+    if (r0 + ty + u < n && c0 + tx < p) tile[ty + u][tx] = (Out)in[(r0 + ty + u) * p + c0 + tx];
+  __syncthreads();
+#pragma unroll
+  for (int u = 0; u < 32; u += 8)
+    if (r0 + tx < n && c0 + ty + u < p) out[(long long)(c0 + ty + u) * n + r0 + tx] = tile[tx][ty + u];
+}
+
+template <typename In, typename Out>
+void transpose(const In* in, int n, int p, Out* out, cudaStream_t s) {
+  if (ceil_div(p, 32) > 65535) throw Error("too many columns");
+  transpose_kernel<<<dim3(ceil_div(n, 32), ceil_div(p, 32)), 256, 0, s>>>(in, n, p, out);
+  FE_LAUNCH("transpose_kernel");
+}
+
+void upload_knn(int* d_idx, float* d_dist, const int* idx, const float* dist, int n, int k, bool rows,
+                cudaStream_t s) {
+  const std::size_t items = (std::size_t)n * k;
+  if (!rows || k == 1) {
+    fe::upload(d_idx, idx, sizeof(int) * items, s);
+    fe::upload(d_dist, dist, sizeof(float) * items, s);
+    return;
+  }
+  int* r_idx = nullptr;
+  float* r_dist = nullptr;
+  Arena tmp;
+  tmp.reserve(&r_idx, items);
+  tmp.reserve(&r_dist, items);
+  tmp.commit("row-major KNN input");
+  fe::upload(r_idx, idx, sizeof(int) * items, s);
+  transpose(r_idx, n, k, d_idx, s);
+  fe::upload(r_dist, dist, sizeof(float) * items, s);
+  transpose(r_dist, n, k, d_dist, s);
+  FE_CUDA(cudaStreamSynchronize(s));
+}
+
+void upload_rows_as_columns(float* d_out, const void* values, bool is_double, int n, int p, cudaStream_t s) {
+  const std::size_t bytes = (std::size_t)n * p * (is_double ? sizeof(double) : sizeof(float));
+  unsigned char* raw = nullptr;
+  Arena tmp;
+  tmp.reserve(&raw, bytes);
+  tmp.commit("row-major data input");
+  fe::upload(raw, values, bytes, s);
+  if (is_double) transpose(reinterpret_cast<const double*>(raw), n, p, d_out, s);
+  else transpose(reinterpret_cast<const float*>(raw), n, p, d_out, s);
+  FE_CUDA(cudaStreamSynchronize(s));
 }
 
 // ---------------------------------------------------------------- bisection

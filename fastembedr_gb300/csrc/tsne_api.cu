@@ -169,7 +169,7 @@ struct TsneJob {
     cudaStream_t s = stream.s;
     configure_adaptive(false);
     order_after_legacy_stream(s);  // d_idx / d_dist may be the caller's buffers
-    validate_knn(d_idx, d_dist, n, k, offset, s);
+    offset = validate_knn(d_idx, d_dist, n, k, offset, s);
     {
       float* d_p = nullptr;
       Arena tmp;
@@ -405,19 +405,21 @@ void check_tsne_args(const void* idx, const void* dist, const float* init, int h
     throw Error("invalid CUDA openTSNE FFT-grid dimensions or parameters");
 }
 
-// The PCA start of host data (column-major n x p, float or double) on the GPU, as a host
+// The PCA start of host data (n x p, column-major, or row-major when rows; float or double) on the GPU, as a host
 // row-major n x 2 init.
-std::vector<float> pca_start(const void* values, bool is_double, int n, int p, cudaStream_t s) {
+std::vector<float> pca_start(const void* values, bool is_double, bool rows, int n, int p, cudaStream_t s) {
   const std::size_t items = (std::size_t)n * p;
   float* X = nullptr;
   double* raw = nullptr;
   float2* init = nullptr;
   Arena a;
   a.reserve(&X, items);
-  if (is_double) a.reserve(&raw, items);
+  if (is_double && !rows) a.reserve(&raw, items);
   a.reserve(&init, n);
   a.commit("device PCA input");
-  if (is_double) {
+  if (rows) {
+    upload_rows_as_columns(X, values, is_double, n, p, s);
+  } else if (is_double) {
     fe::upload(raw, values, sizeof(double) * items, s);
     double_to_float_kernel<<<std::max(1, std::min(ceil_div((long long)items, 256), sm_count() * 8)), 256, 0, s>>>(
         raw, X, (long long)items);
@@ -437,7 +439,7 @@ int run_tsne_from_knn(const int* indices, const DistT* distances, bool on_device
                       int n, int k, int n_components, float perplexity, int early_iter, int n_iter, float early_exag,
                       float exag, float lr, int lr_auto, float m0, float m1, float min_gain, float max_step,
                       unsigned seed, int offset, float* out, const void* pca_values = nullptr,
-                      bool pca_double = false, int pca_p = 0) {
+                      bool pca_double = false, int pca_p = 0, bool rows = false) {
   return guarded([&] {
     check_tsne_args(indices, distances, init, has_init, n, k, n_components, perplexity, early_iter, n_iter,
                     early_exag, exag, lr, lr_auto, m0, m1, min_gain, out);
@@ -448,7 +450,7 @@ int run_tsne_from_knn(const int* indices, const DistT* distances, bool on_device
     if (on_device) order_after_legacy_stream(s);
     std::vector<float> pca_init;
     if (!has_init && pca_values) {
-      pca_init = pca_start(pca_values, pca_double, n, pca_p, s);
+      pca_init = pca_start(pca_values, pca_double, false, n, pca_p, s);
       init = pca_init.data();
       has_init = 1;
     }
@@ -462,16 +464,16 @@ int run_tsne_from_knn(const int* indices, const DistT* distances, bool on_device
     if (!on_device && !std::is_same<DistT, float>::value) in.reserve(&d_raw, items);
     in.commit("CUDA openTSNE KNN input");
     const int* idx_ptr = on_device ? indices : d_idx;
-    if (!on_device) fe::upload(d_idx, indices, sizeof(int) * items, s);
     const float* dist_ptr = nullptr;
     if constexpr (std::is_same<DistT, float>::value) {
       if (on_device) {
         dist_ptr = distances;
       } else {
-        fe::upload(d_dist, distances, sizeof(float) * items, s);
+        upload_knn(d_idx, d_dist, indices, distances, n, k, rows, s);
         dist_ptr = d_dist;
       }
     } else {
+      if (!on_device) fe::upload(d_idx, indices, sizeof(int) * items, s);
       const DistT* src = distances;
       if (!on_device) {
         fe::upload(d_raw, distances, sizeof(DistT) * items, s);
@@ -526,6 +528,18 @@ int fastembedr_cuda_opentsne_fft_from_knn_float(const int* indices, const float*
                                       seed, index_offset, out);
 }
 
+int fastembedr_cuda_opentsne_fft_from_knn_rows_float(const int* indices, const float* distances, const float* init,
+                                                     int has_init, int n, int k, int n_components, float perplexity,
+                                                     int early_iter, int n_iter, float early_exag, float exag,
+                                                     float lr, int lr_auto, float m0, float m1, float min_gain,
+                                                     float max_step, unsigned int seed, int index_offset,
+                                                     float* out) {
+  return fe::run_tsne_from_knn<float>(indices, distances, false, init, has_init, n, k, n_components, perplexity,
+                                      early_iter, n_iter, early_exag, exag, lr, lr_auto, m0, m1, min_gain, max_step,
+                                      seed, index_offset < 0 ? fe::kDetectLabels : index_offset, out, nullptr, false, 0,
+                                      true);
+}
+
 int fastembedr_cuda_opentsne_fft_from_knn(const int* indices, const double* distances, const float* init,
                                           int has_init, int n, int k, int n_components, float perplexity,
                                           int early_iter, int n_iter, float early_exag, float exag, float lr,
@@ -568,13 +582,21 @@ int fastembedr_cuda_opentsne_fft_from_device_knn_float_pca_float(
                                       seed, index_offset, out, pca_init_values, false, pca_init_p);
 }
 
-int fastembedr_cuda_tsne_pca_init(const void* values, int is_double, int n, int p, float* out) {
+static int pca_init(const void* values, bool is_double, bool rows, int n, int p, float* out) {
   return fe::guarded([&] {
     if (!values || !out) throw fe::Error("null host pointer");
     fe::Stream st;
-    const std::vector<float> h = fe::pca_start(values, is_double != 0, n, p, st.s);
+    const std::vector<float> h = fe::pca_start(values, is_double, rows, n, p, st.s);
     std::copy(h.begin(), h.end(), out);
   });
+}
+
+int fastembedr_cuda_tsne_pca_init(const void* values, int is_double, int n, int p, float* out) {
+  return pca_init(values, is_double != 0, false, n, p, out);
+}
+
+int fastembedr_cuda_tsne_pca_init_rows(const void* values, int is_double, int n, int p, float* out) {
+  return pca_init(values, is_double != 0, true, n, p, out);
 }
 
 int fastembedr_cuda_tsne_affinities(const int* indices, const float* distances, int n, int k, float perplexity,

@@ -1170,7 +1170,7 @@ void umap_spectral_job(const int* d_idx, const float* d_dist, int n, int k, int 
   job.alloc(n);
   cudaStream_t s = job.stream.s;
   order_after_legacy_stream(s);  // d_idx / d_dist may be the caller's device buffers
-  validate_knn(d_idx, d_dist, n, k, offset, s);
+  offset = validate_knn(d_idx, d_dist, n, k, offset, s);
   UmapGraph g;
   umap_build_graph(d_idx, d_dist, n, k, offset, g, s);
   if (binary) {
@@ -1209,7 +1209,7 @@ void umap_knn_spectral_job(const int* d_idx, const float* d_dist, int n, int k, 
   job.alloc(n);
   cudaStream_t s = job.stream.s;
   order_after_legacy_stream(s);
-  validate_knn(d_idx, d_dist, n, k, offset, s);
+  offset = validate_knn(d_idx, d_dist, n, k, offset, s);
   UmapGraph g;
   umap_build_graph(d_idx, d_dist, n, k, offset, g, s);
   SpectralDraws pre = early->get();
@@ -1348,10 +1348,10 @@ int fastembedr_cuda_umap_graph_from_knn(const int* indices, const float* distanc
   });
 }
 
-int fastembedr_cuda_umap_from_knn_profile(const int* indices, const float* distances, const float* init, int n,
-                                          int k, int index_offset, int n_epochs, int negative_sample_rate,
-                                          float learning_rate, float min_dist, float repulsion_strength,
-                                          unsigned int seed, float* out, float* graph_ms, float* sgd_ms) {
+static int umap_from_knn(const int* indices, const float* distances, bool rows, const float* init, int n, int k,
+                         int index_offset, int n_epochs, int negative_sample_rate, float learning_rate,
+                         float min_dist, float repulsion_strength, unsigned int seed, float* out, float* graph_ms,
+                         float* sgd_ms) {
   return fe::guarded([&] {
     if (!indices || !distances || !init || !out) throw fe::Error("null UMAP input pointer");
     if (n < 2 || k < 1 || n_epochs < 1 || negative_sample_rate < 0 || !(learning_rate > 0.0f) || min_dist < 0.0f ||
@@ -1367,8 +1367,7 @@ int fastembedr_cuda_umap_from_knn_profile(const int* indices, const float* dista
     a.reserve(&d_idx, items);
     a.reserve(&d_dist, items);
     a.commit("UMAP input");
-    fe::upload(d_idx, indices, sizeof(int) * items, s);
-    fe::upload(d_dist, distances, sizeof(float) * items, s);
+    fe::upload_knn(d_idx, d_dist, indices, distances, n, k, rows, s);
     FE_CUDA(cudaMemcpyAsync(job.y, init, sizeof(float) * 2 * n, cudaMemcpyHostToDevice, s));
     cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
     const bool timed = graph_ms || sgd_ms;
@@ -1382,9 +1381,9 @@ int fastembedr_cuda_umap_from_knn_profile(const int* indices, const float* dista
       }
     } guard{ev};
     if (timed) FE_CUDA(cudaEventRecord(ev[0], s));
-    fe::validate_knn(d_idx, d_dist, n, k, index_offset, s);
+    const int offset = fe::validate_knn(d_idx, d_dist, n, k, index_offset, s);
     fe::UmapGraph g;
-    fe::umap_build_graph(d_idx, d_dist, n, k, index_offset, g, s);
+    fe::umap_build_graph(d_idx, d_dist, n, k, offset, g, s);
     if (timed) FE_CUDA(cudaEventRecord(ev[1], s));
     double av = 0.0, bv = 0.0;
     fe::umap_ab_params(1.0, min_dist, &av, &bv);
@@ -1672,10 +1671,10 @@ int fastembedr_cuda_umap_spectral_init_csr(const int* offsets, const int* neighb
   });
 }
 
-int fastembedr_cuda_umap_knn_spectral(const int* indices, const float* distances, int n, int k, int index_offset,
-                                      int n_epochs, int negative_sample_rate, float learning_rate, float min_dist,
-                                      float repulsion_strength, int spectral_n_iter, double init_scale,
-                                      unsigned int seed, float* out) {
+static int umap_knn_spectral(const int* indices, const float* distances, bool rows, int n, int k, int index_offset,
+                             int n_epochs, int negative_sample_rate, float learning_rate, float min_dist,
+                             float repulsion_strength, int spectral_n_iter, double init_scale, unsigned int seed,
+                             float* out) {
   return fe::guarded([&] {
     if (!indices || !distances || !out) throw fe::Error("null host pointer");
     if (n < 2 || k < 1 || n_epochs < 1 || negative_sample_rate < 0 || !(learning_rate > 0.0f) || min_dist < 0.0f ||
@@ -1690,12 +1689,28 @@ int fastembedr_cuda_umap_knn_spectral(const int* indices, const float* distances
     a.reserve(&d_idx, items);
     a.reserve(&d_dist, items);
     a.commit("UMAP input");
-    fe::upload(d_idx, indices, sizeof(int) * items, st.s);
-    fe::upload(d_dist, distances, sizeof(float) * items, st.s);
+    fe::upload_knn(d_idx, d_dist, indices, distances, n, k, rows, st.s);
     FE_CUDA(cudaStreamSynchronize(st.s));
     fe::umap_knn_spectral_job(d_idx, d_dist, n, k, index_offset, n_epochs, negative_sample_rate, learning_rate,
                               min_dist, repulsion_strength, spectral_n_iter, init_scale, seed, nullptr, out, &draws);
   });
+}
+
+int fastembedr_cuda_umap_knn_spectral(const int* indices, const float* distances, int n, int k, int index_offset,
+                                      int n_epochs, int negative_sample_rate, float learning_rate, float min_dist,
+                                      float repulsion_strength, int spectral_n_iter, double init_scale,
+                                      unsigned int seed, float* out) {
+  return umap_knn_spectral(indices, distances, false, n, k, index_offset, n_epochs, negative_sample_rate,
+                           learning_rate, min_dist, repulsion_strength, spectral_n_iter, init_scale, seed, out);
+}
+
+int fastembedr_cuda_umap_knn_spectral_rows(const int* indices, const float* distances, int n, int k, int index_offset,
+                                           int n_epochs, int negative_sample_rate, float learning_rate,
+                                           float min_dist, float repulsion_strength, int spectral_n_iter,
+                                           double init_scale, unsigned int seed, float* out) {
+  return umap_knn_spectral(indices, distances, true, n, k, index_offset < 0 ? fe::kDetectLabels : index_offset,
+                           n_epochs, negative_sample_rate, learning_rate, min_dist, repulsion_strength,
+                           spectral_n_iter, init_scale, seed, out);
 }
 
 int fastembedr_cuda_spectral_init_from_knn(const int* indices, const double* distances, int n, int k,
@@ -1764,9 +1779,24 @@ int fastembedr_cuda_umap_from_device_knn_spectral_float(const int* device_indice
 int fastembedr_cuda_umap_from_knn(const int* indices, const float* distances, const float* init, int n, int k,
                                   int index_offset, int n_epochs, int negative_sample_rate, float learning_rate,
                                   float min_dist, float repulsion_strength, unsigned int seed, float* out) {
-  return fastembedr_cuda_umap_from_knn_profile(indices, distances, init, n, k, index_offset, n_epochs,
-                                               negative_sample_rate, learning_rate, min_dist, repulsion_strength, seed,
-                                               out, nullptr, nullptr);
+  return umap_from_knn(indices, distances, false, init, n, k, index_offset, n_epochs, negative_sample_rate,
+                       learning_rate, min_dist, repulsion_strength, seed, out, nullptr, nullptr);
+}
+
+int fastembedr_cuda_umap_from_knn_profile(const int* indices, const float* distances, const float* init, int n,
+                                          int k, int index_offset, int n_epochs, int negative_sample_rate,
+                                          float learning_rate, float min_dist, float repulsion_strength,
+                                          unsigned int seed, float* out, float* graph_ms, float* sgd_ms) {
+  return umap_from_knn(indices, distances, false, init, n, k, index_offset, n_epochs, negative_sample_rate,
+                       learning_rate, min_dist, repulsion_strength, seed, out, graph_ms, sgd_ms);
+}
+
+int fastembedr_cuda_umap_from_knn_rows(const int* indices, const float* distances, const float* init, int n, int k,
+                                       int index_offset, int n_epochs, int negative_sample_rate, float learning_rate,
+                                       float min_dist, float repulsion_strength, unsigned int seed, float* out) {
+  return umap_from_knn(indices, distances, true, init, n, k, index_offset < 0 ? fe::kDetectLabels : index_offset,
+                       n_epochs, negative_sample_rate, learning_rate, min_dist, repulsion_strength, seed, out, nullptr,
+                       nullptr);
 }
 
 }  // extern "C"

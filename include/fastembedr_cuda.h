@@ -52,6 +52,17 @@ int fastembedr_cuda_opentsne_fft_from_knn_float(const int* indices, const float*
                                                 float max_step_norm, unsigned int seed, int index_offset,
                                                 float* out);
 
+/* The same on row-major n x k host arrays (no reference counterpart: its host language is column-major).
+ * index_offset < 0 detects the labels as the package does: 1-based when all lie in [1, n]. */
+int fastembedr_cuda_opentsne_fft_from_knn_rows_float(const int* indices, const float* distances, const float* init,
+                                                     int has_init, int n, int k, int n_components, float perplexity,
+                                                     int early_exaggeration_iter, int n_iter,
+                                                     float early_exaggeration, float exaggeration,
+                                                     float learning_rate, int learning_rate_auto,
+                                                     float initial_momentum, float final_momentum, float min_gain,
+                                                     float max_step_norm, unsigned int seed, int index_offset,
+                                                     float* out);
+
 /* replaces fastembedr_cuda_opentsne_fft_from_knn (double distances), src/embedding_cuda_kernels.cpp:6178-6205 */
 int fastembedr_cuda_opentsne_fft_from_knn(const int* indices, const double* distances, const float* init,
                                           int has_init, int n, int k, int n_components, float perplexity,
@@ -93,6 +104,8 @@ int fastembedr_cuda_opentsne_fft_from_device_knn_float_pca_float(
 /* The PCA start alone (no reference counterpart as an entry point): host column-major n x p data
  * (is_double: double, else float) -> out, host row-major n x 2 floats. */
 int fastembedr_cuda_tsne_pca_init(const void* values, int is_double, int n, int p, float* out);
+/* The same on row-major n x p data. */
+int fastembedr_cuda_tsne_pca_init_rows(const void* values, int is_double, int n, int p, float* out);
 
 /* ---------------------------------------------------------------- UMAP */
 
@@ -142,6 +155,12 @@ int fastembedr_cuda_umap_knn_spectral(const int* indices, const float* distances
                                       float repulsion_strength, int spectral_n_iter, double init_scale,
                                       unsigned int seed, float* out);
 
+/* The same on row-major n x k host arrays; index_offset < 0 detects the labels. */
+int fastembedr_cuda_umap_knn_spectral_rows(const int* indices, const float* distances, int n, int k, int index_offset,
+                                           int n_epochs, int negative_sample_rate, float learning_rate,
+                                           float min_dist, float repulsion_strength, int spectral_n_iter,
+                                           double init_scale, unsigned int seed, float* out);
+
 /* find_ab_params (src/fast_knn_umap.cpp:437-497), the curve a, b that the reference's bridges
  * compute on the host before calling the fused UMAP entry points below (host code, no GPU). */
 void fastembedr_umap_find_ab_params(double spread, double min_dist, double* a, double* b);
@@ -188,6 +207,10 @@ int fastembedr_cuda_umap_from_device_knn_spectral_float(const int* device_indice
 int fastembedr_cuda_umap_from_knn(const int* indices, const float* distances, const float* init, int n, int k,
                                   int index_offset, int n_epochs, int negative_sample_rate, float learning_rate,
                                   float min_dist, float repulsion_strength, unsigned int seed, float* out);
+/* The same on row-major n x k host arrays; index_offset < 0 detects the labels. */
+int fastembedr_cuda_umap_from_knn_rows(const int* indices, const float* distances, const float* init, int n, int k,
+                                       int index_offset, int n_epochs, int negative_sample_rate, float learning_rate,
+                                       float min_dist, float repulsion_strength, unsigned int seed, float* out);
 /* No reference counterpart: many UMAP instances in one job. Each instance's fuzzy graph is built
  * on its own and appended (vertices offset by the instance's first point); every epoch is one
  * launch over all edges (negatives drawn inside the edge's own instance, Philox keyed by the
@@ -268,6 +291,15 @@ int fastembedr_cuda_transform_tsne(const double* reference_layout, int n_referen
                                    double max_grad_norm, double max_step_norm, int n_negatives,
                                    int exact_repulsion_threshold, int seed, double* out);
 
+/* The same with row-major indices and distances (the layouts stay column-major). */
+int fastembedr_cuda_transform_tsne_rows(const double* reference_layout, int n_reference, const int* indices,
+                                        const double* distances, int n_query, int k, const double* y_init, int init,
+                                        const char* initialization, double perplexity, int n_iter,
+                                        int early_exaggeration_iter, double learning_rate, double early_exaggeration,
+                                        double exaggeration, double initial_momentum, double final_momentum,
+                                        double max_grad_norm, double max_step_norm, int n_negatives,
+                                        int exact_repulsion_threshold, int seed, double* out);
+
 /* replaces fastembedr_cuda_landmark_tsne_from_device_knn, src/embedding_cuda_kernels.cpp:3572-3686
  * (project_landmark_model's CUDA route, landmark_tsne_transform_cuda_gpu_cpp,
  * src/embedding_cuda_bridge.cpp:584-612). device_indices / device_distances: device pointers,
@@ -311,6 +343,10 @@ int fastembedr_transform_server_create(const double* reference_layout, int n_ref
  * (1- or 0-based). The arrays are copied before the call returns. */
 int fastembedr_transform_server_submit(fastembedr_transform_server* server, const int* indices, const float* distances,
                                        int n_query, int k, unsigned long long* request_id);
+/* The same with a row-major KNN. */
+int fastembedr_transform_server_submit_rows(fastembedr_transform_server* server, const int* indices,
+                                            const float* distances, int n_query, int k,
+                                            unsigned long long* request_id);
 /* Wait up to timeout_ms (< 0: no limit). Returns 0 when done (out: column-major n_query x 2
  * doubles, latency_ms: submit to result on the host; a non-NULL out consumes the request),
  * 2 while still queued or running, 1 on error. */
