@@ -23,11 +23,13 @@
 #include <map>
 #include <memory>
 #include <type_traits>
+#include <optional>
 #include <vector>
 
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_segmented_radix_sort.cuh>
 
+#include "umap_curve.cuh"
 #include "../../include/fastembedr_cuda.h"
 #include "philox.cuh"
 #include "sort.cuh"
@@ -815,59 +817,136 @@ __global__ void umap_sanitize_kernel(float2* __restrict__ y, int n, unsigned* __
 }
 
 // find_ab_params CPU policy (src/fast_knn_umap.cpp:437-497): hard-coded values for the package's
-// spreads/min_dists, otherwise the grid search + gradient refinement of that function.
-void umap_ab_params(double spread, double min_dist, double* a, double* b) {
-  if (std::fabs(spread - 1.0) < 1e-12 && std::fabs(min_dist - 0.01) < 1e-12) {
-    *a = 1.895605865596314;
-    *b = 0.8006377738365004;
-    return;
+// spreads/min_dists, otherwise the grid search + gradient refinement of that function (here for host callers; the
+// jobs fit on the GPU, UmapCurve).
+bool umap_tabulated_ab(double spread, double min_dist, double* a, double* b) {
+  constexpr double kTable[3][3] = {{0.01, 1.895605865596314, 0.8006377738365004},
+                                   {0.1, 1.5769434601962196, 0.8950608781227859},
+                                   {0.5, 0.5830300199018228, 1.3341669931033755}};
+  for (const auto& row : kTable)
+    if (std::fabs(spread - 1.0) < 1e-12 && std::fabs(min_dist - row[0]) < 1e-12) {
+      *a = row[1];
+      *b = row[2];
+      return true;
+    }
+  return false;
+}
+
+// The points of the fit, and its two stages as the reference computes them.
+struct UmapCurvePoints {
+  double xs[kCurvePoints], ys[kCurvePoints];
+  UmapCurvePoints(double spread, double min_dist) {
+    for (int i = 0; i < kCurvePoints; ++i) {
+      xs[i] = (spread * 3.0) * (double)i / 299.0;
+      ys[i] = xs[i] < min_dist ? 1.0 : std::exp(-(xs[i] - min_dist) / spread);
+    }
   }
-  if (std::fabs(spread - 1.0) < 1e-12 && std::fabs(min_dist - 0.1) < 1e-12) {
+  double loss(double av, double bv) const {
+    double sum = 0.0;
+    for (int i = 0; i < kCurvePoints; ++i) {
+      const double e = 1.0 / (1.0 + av * std::pow(xs[i], 2.0 * bv)) - ys[i];
+      sum += e * e;
+    }
+    return sum;
+  }
+  // The grid point of least loss (the first of equals) among those that `skip` does not rule out.
+  template <typename Skip>
+  void search(Skip skip, double* a, double* b) const {
+    double best = INFINITY;
+    int k = 0;
     *a = 1.5769434601962196;
     *b = 0.8950608781227859;
-    return;
-  }
-  if (std::fabs(spread - 1.0) < 1e-12 && std::fabs(min_dist - 0.5) < 1e-12) {
-    *a = 0.5830300199018228;
-    *b = 1.3341669931033755;
-    return;
-  }
-  double xs[300], ys[300];
-  for (int i = 0; i < 300; ++i) {
-    xs[i] = (spread * 3.0) * (double)i / 299.0;
-    ys[i] = xs[i] < min_dist ? 1.0 : std::exp(-(xs[i] - min_dist) / spread);
-  }
-  double ba = 1.5769434601962196, bb = 0.8950608781227859, best = INFINITY;
-  for (double la = -4.0; la <= 4.0001; la += 0.2)
-    for (double bv = 0.25; bv <= 2.0001; bv += 0.05) {
-      const double av = std::exp(la);
-      double loss = 0.0;
-      for (int i = 0; i < 300; ++i) {
-        const double e = 1.0 / (1.0 + av * std::pow(xs[i], 2.0 * bv)) - ys[i];
-        loss += e * e;
+    for (double la = -4.0; la <= 4.0001; la += 0.2)
+      for (double bv = 0.25; bv <= 2.0001; bv += 0.05, ++k) {
+        if (skip(k)) continue;
+        const double av = std::exp(la), l = loss(av, bv);
+        if (l < best) {
+          best = l;
+          *a = av;
+          *b = bv;
+        }
       }
-      if (loss < best) {
-        best = loss;
-        ba = av;
-        bb = bv;
-      }
-    }
-  for (int it = 0; it < 80; ++it) {
-    double ga = 0.0, gb = 0.0;
-    for (int i = 0; i < 300; ++i) {
-      const double x = std::max(xs[i], 1e-6);
-      const double x2b = std::pow(x, 2.0 * bb);
-      const double den = 1.0 + ba * x2b;
-      const double e = 1.0 / den - ys[i];
-      ga += e * (-x2b / (den * den));
-      gb += e * (-(ba * x2b * 2.0 * std::log(x)) / (den * den));
-    }
-    ba = std::max(1e-4, ba - 0.01 * ga);
-    bb = std::max(0.1, bb - 0.01 * gb);
   }
-  *a = ba;
-  *b = bb;
+  void descend(double* a, double* b) const {
+    double ba = *a, bb = *b, lx[kCurvePoints];
+    for (int i = 0; i < kCurvePoints; ++i) lx[i] = std::log(std::max(xs[i], 1e-6));
+    for (int it = 0; it < 80; ++it) {
+      double ga = 0.0, gb = 0.0;
+      for (int i = 0; i < kCurvePoints; ++i) {
+        const double x2b = std::pow(std::max(xs[i], 1e-6), 2.0 * bb);
+        const double den = 1.0 + ba * x2b;
+        const double e = 1.0 / den - ys[i];
+        ga += e * (-x2b / (den * den));
+        gb += e * (-(ba * x2b * 2.0 * lx[i]) / (den * den));
+      }
+      ba = std::max(1e-4, ba - 0.01 * ga);
+      bb = std::max(0.1, bb - 0.01 * gb);
+    }
+    *a = ba;
+    *b = bb;
+  }
+};
+
+void umap_ab_params(double spread, double min_dist, double* a, double* b) {
+  if (umap_tabulated_ab(spread, min_dist, a, b)) return;
+  const UmapCurvePoints points(spread, min_dist);
+  points.search([](int) { return false; }, a, b);
+  points.descend(a, b);
 }
+
+// The curve parameters of a job, the values of umap_ab_params: tabulated, or fitted beside the job's uploads and
+// graph build. The GPU evaluates the grid; a host thread takes the points whose loss is within rounding of the
+// least (one, but for ties), decides among them with the host's own sums, and descends: its 80 steps can
+// amplify a last bit into the second digit (min_dist 0.99), so they stay the host's.
+class UmapCurve {
+ public:
+  UmapCurve(double spread, double min_dist) {
+    double a = 0.0, b = 0.0;
+    if (umap_tabulated_ab(spread, min_dist, &a, &b)) {
+      values_ = std::make_pair(a, b);
+      return;
+    }
+    stream_.emplace();
+    arena_.reserve(&loss_, kCurveGrid);
+    arena_.commit("UMAP curve fit");
+    curve_grid_losses(spread, min_dist, loss_, stream_->s);
+    int device = 0;
+    FE_CUDA(cudaGetDevice(&device));
+    fit_ = std::async(std::launch::async, [this, spread, min_dist, device] {
+      FE_CUDA(cudaSetDevice(device));
+      std::vector<double> loss(kCurveGrid);
+      FE_CUDA(cudaMemcpyAsync(loss.data(), loss_, sizeof(double) * loss.size(), cudaMemcpyDeviceToHost, stream_->s));
+      FE_CUDA(cudaStreamSynchronize(stream_->s));
+      double least = INFINITY;
+      for (double l : loss)
+        if (l < least) least = l;
+      const double limit = least * (1.0 + 1e-9);
+      const UmapCurvePoints points(spread, min_dist);
+      double a = 0.0, b = 0.0;
+      points.search([&](int k) { return !(loss[k] <= limit); }, &a, &b);
+      points.descend(&a, &b);
+      return std::make_pair(a, b);
+    });
+  }
+  ~UmapCurve() {
+    if (fit_.valid()) fit_.wait();  // it uses the buffer and the stream
+    if (stream_) cudaStreamSynchronize(stream_->s);
+  }
+  UmapCurve(const UmapCurve&) = delete;
+  UmapCurve& operator=(const UmapCurve&) = delete;
+  void get(double* a, double* b) {
+    if (fit_.valid()) values_ = fit_.get();
+    *a = values_.first;
+    *b = values_.second;
+  }
+
+ private:
+  std::pair<double, double> values_{0.0, 0.0};
+  double* loss_ = nullptr;
+  Arena arena_;
+  std::optional<Stream> stream_;
+  std::future<std::pair<double, double>> fit_;
+};
 
 // Optimizer state of one UMAP instance.
 // Sort keys of the period-ordered edge list: the bits of epochs_per_sample (non-negative floats,
@@ -1207,6 +1286,8 @@ void umap_knn_spectral_job(const int* d_idx, const float* d_dist, int n, int k, 
   }
   UmapJob job;
   job.alloc(n);
+  std::optional<UmapCurve> curve;
+  if (y_out && n_epochs > 0) curve.emplace(1.0, min_dist);
   cudaStream_t s = job.stream.s;
   order_after_legacy_stream(s);
   offset = validate_knn(d_idx, d_dist, n, k, offset, s);
@@ -1226,7 +1307,7 @@ void umap_knn_spectral_job(const int* d_idx, const float* d_dist, int n, int k, 
     FE_LAUNCH("umap_start_to_layout_kernel");
     if (n_epochs > 0) {
       double av = 0.0, bv = 0.0;
-      umap_ab_params(1.0, min_dist, &av, &bv);
+      curve->get(&av, &bv);
       const UmapParams p{n, n_epochs, nsr, seed, lr, (float)av, (float)bv, rep};
       job.run(g.heads, g.neighbors, g.eps, g.nnz, p);
     }
@@ -1359,6 +1440,7 @@ static int umap_from_knn(const int* indices, const float* distances, bool rows, 
       throw fe::Error("invalid CUDA UMAP parameters");
     fe::UmapJob job;
     job.alloc(n);
+    fe::UmapCurve curve(1.0, min_dist);
     cudaStream_t s = job.stream.s;
     const std::size_t items = (std::size_t)n * k;
     int* d_idx = nullptr;
@@ -1386,7 +1468,7 @@ static int umap_from_knn(const int* indices, const float* distances, bool rows, 
     fe::umap_build_graph(d_idx, d_dist, n, k, offset, g, s);
     if (timed) FE_CUDA(cudaEventRecord(ev[1], s));
     double av = 0.0, bv = 0.0;
-    fe::umap_ab_params(1.0, min_dist, &av, &bv);
+    curve.get(&av, &bv);
     const fe::UmapParams p{n, n_epochs, negative_sample_rate, seed, learning_rate, (float)av, (float)bv,
                            repulsion_strength};
     job.run(g.heads, g.neighbors, g.eps, g.nnz, p);
@@ -1438,6 +1520,7 @@ void umap_batch_job(int n_instances, const int* sizes, const std::vector<const i
   const int n = vb[n_instances];
   UmapJob job;
   job.alloc(n);
+  UmapCurve curve(1.0, min_dist);
   cudaStream_t s = job.stream.s;
   long long n_edges = 0;
   // Every instance's fuzzy graph is built in one reused workspace and written straight into the
@@ -1515,7 +1598,7 @@ void umap_batch_job(int n_instances, const int* sizes, const std::vector<const i
                             cudaMemcpyHostToDevice, s));
   FE_CUDA(cudaStreamSynchronize(s));
   double av = 0.0, bv = 0.0;
-  umap_ab_params(1.0, min_dist, &av, &bv);
+  curve.get(&av, &bv);
   const UmapParams p{n, n_epochs, negative_sample_rate, seed, learning_rate, (float)av, (float)bv,
                      repulsion_strength};
   job.edge_begin = d_eb;
@@ -1578,6 +1661,14 @@ int fastembedr_cuda_umap_batch_from_knn_rows(int n_instances, const int* sizes, 
       if (!iu[b] || !du[b] || !yu[b] || !ou[b]) throw fe::Error("null UMAP batch pointer");
     fe::umap_batch_job(n_instances, sizes, iu, du, yu, ou, true, k, index_offset, n_epochs, negative_sample_rate,
                        learning_rate, min_dist, repulsion_strength, seed, sgd_ms);
+  });
+}
+
+int fastembedr_cuda_umap_find_ab_params(double spread, double min_dist, double* a, double* b) {
+  return fe::guarded([&] {
+    if (!a || !b) throw fe::Error("null UMAP curve output");
+    fe::UmapCurve curve(spread, min_dist);
+    curve.get(a, b);
   });
 }
 

@@ -164,6 +164,8 @@ int fastembedr_cuda_umap_knn_spectral_rows(const int* indices, const float* dist
 /* find_ab_params (src/fast_knn_umap.cpp:437-497), the curve a, b that the reference's bridges
  * compute on the host before calling the fused UMAP entry points below (host code, no GPU). */
 void fastembedr_umap_find_ab_params(double spread, double min_dist, double* a, double* b);
+/* The same fitted on the GPU, as the KNN entry points do beside their graph build (the same values). */
+int fastembedr_cuda_umap_find_ab_params(double spread, double min_dist, double* a, double* b);
 
 /* No reference counterpart (diagnostic, host code, no GPU): 1 when the multi-threaded normal draws
  * of the spectral start reproduce std::normal_distribution<double> on std::mt19937 bit for bit on
