@@ -42,6 +42,12 @@ struct Blocks {
   static constexpr int PAIRS = T >= 64 ? 1 : 64 / T;  // row passes: 3 x PAIRS x T threads
   static constexpr int COLS = T >= 64 ? 1 : 64 / T;   // column pass: 4 x COLS x T threads
   static constexpr int KROWS = 3 * PAIRS;             // kernel rows of a block of the row pass
+  // Blocks per SM that the registers must leave room for. Up to M = 512 the eight values of a thread fit 64 registers
+  // and twice the warps hide the barriers and exchanges (32 instances of G = 256, ten iterations: 3.72 -> 3.40 ms; one
+  // instance is bound by latency and runs the same). M = 1024 spills at 64 (one instance: 0.7% slower), 2048 needs two
+  // blocks of 512 threads to fill an SM.
+  static constexpr int ROW_BLOCKS = LOGM == 11 ? 2 : LOGM <= 9 ? 5 : 1;
+  static constexpr int COL_BLOCKS = LOGM == 11 ? 2 : LOGM <= 9 ? 4 : 1;
 };
 
 // Kernel rows dy of one block: forward FFTs of (q, q^2) at columns c (offset c or c - M, zero beyond
@@ -82,7 +88,7 @@ __device__ __forceinline__ void kernel_rows(float2* sbuf, int row0, int nodes, i
 // cleared for the next scatter. A spectra to arow, separated B half spectra to brow, the rows of a
 // pair side by side (places 2 p and 2 p + 1 of a column). blockIdx.y: member of the grid class.
 template <int LOGM>
-__global__ void __launch_bounds__(3 * Blocks<LOGM>::PAIRS* FftPlan<LOGM>::T, LOGM == 11 ? 2 : 1)
+__global__ void __launch_bounds__(3 * Blocks<LOGM>::PAIRS* FftPlan<LOGM>::T, Blocks<LOGM>::ROW_BLOCKS)
 rows_forward_kernel(const TsneInstance* __restrict__ inst, const int* __restrict__ members, int grid, int nodes, int ld,
                     const float2* __restrict__ tw, const GridState* __restrict__ cur, int charge_blocks,
                     float2* __restrict__ arow, float2* __restrict__ brow, float2* __restrict__ krow) {
@@ -148,7 +154,7 @@ rows_forward_kernel(const TsneInstance* __restrict__ inst, const int* __restrict
 // columns (Z + n up to the 1 / M^2 scale) are formed on the values in registers and the first
 // three transformed back in place. The sum is kept in two floats (48 bits).
 template <int LOGM>
-__global__ void __launch_bounds__(4 * Blocks<LOGM>::COLS* FftPlan<LOGM>::T, LOGM == 11 ? 2 : 1)
+__global__ void __launch_bounds__(4 * Blocks<LOGM>::COLS* FftPlan<LOGM>::T, Blocks<LOGM>::COL_BLOCKS)
 columns_convolve_kernel(float2* __restrict__ arow, float2* __restrict__ brow, const float2* __restrict__ krow,
                         int nodes, int ld, const float2* __restrict__ tw, double* __restrict__ zpart) {
   using P = FftPlan<LOGM>;
@@ -245,7 +251,7 @@ columns_convolve_kernel(float2* __restrict__ arow, float2* __restrict__ brow, co
 // an instance instead finalises Z = sum_k |F_mass|^2 Kq / M^2 - n (the reference's
 // sum_i q_grid(y_i) - n).
 template <int LOGM>
-__global__ void __launch_bounds__(3 * Blocks<LOGM>::PAIRS* FftPlan<LOGM>::T, LOGM == 11 ? 2 : 1)
+__global__ void __launch_bounds__(3 * Blocks<LOGM>::PAIRS* FftPlan<LOGM>::T, Blocks<LOGM>::ROW_BLOCKS)
 rows_inverse_kernel(const float2* __restrict__ arow, const float2* __restrict__ brow,
                     const TsneInstance* __restrict__ inst, const int* __restrict__ members, int grid, int nodes, int ld,
                     const float2* __restrict__ tw, const double* __restrict__ zpart, int zblocks,
