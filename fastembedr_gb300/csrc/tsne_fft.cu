@@ -86,16 +86,17 @@ __device__ __forceinline__ void kernel_rows(float2* sbuf, int row0, int nodes, i
 // Row pass. Blocks from charge_blocks on take kernel rows (see above). The others take charge rows in
 // pairs (p, p + npairs), npairs = ld / 2: forward FFTs of A of both rows and of m + i m'; the rows are
 // cleared for the next scatter. A spectra to arow, separated B half spectra to brow, the rows of a
-// pair side by side (places 2 p and 2 p + 1 of a column). blockIdx.y: member of the grid class.
+// pair side by side (places 2 p and 2 p + 1 of a column). blockIdx.y: member of the grid class
+// (`first` is member 0, so that a single instance waits for one load less).
 template <int LOGM>
 __global__ void __launch_bounds__(3 * Blocks<LOGM>::PAIRS* FftPlan<LOGM>::T, Blocks<LOGM>::ROW_BLOCKS)
-rows_forward_kernel(const TsneInstance* __restrict__ inst, const int* __restrict__ members, int grid, int nodes, int ld,
-                    const float2* __restrict__ tw, const GridState* __restrict__ cur, int charge_blocks,
+rows_forward_kernel(long long* __restrict__ charges, const int* __restrict__ members, int first, int grid, int nodes,
+                    int ld, const float2* __restrict__ tw, const GridState* __restrict__ cur, int charge_blocks,
                     float2* __restrict__ arow, float2* __restrict__ brow, float2* __restrict__ krow) {
   using P = FftPlan<LOGM>;
   constexpr int M = P::M, HM = M / 2, NP = Blocks<LOGM>::PAIRS, THREADS = 3 * NP * P::T;
   extern __shared__ float2 sbuf[];
-  const int b = members[blockIdx.y];
+  const int b = blockIdx.y == 0 ? first : members[blockIdx.y];
   if ((int)blockIdx.x >= charge_blocks) {
     kernel_rows<LOGM>(sbuf, ((int)blockIdx.x - charge_blocks) * Blocks<LOGM>::KROWS, nodes, ld, tw, cur[b].h,
                       krow + (long long)blockIdx.y * (HM + 1) * ld);
@@ -103,7 +104,7 @@ rows_forward_kernel(const TsneInstance* __restrict__ inst, const int* __restrict
   }
   const int g = threadIdx.x / P::T, tid = threadIdx.x % P::T;
   const int npairs = ld / 2, pair0 = blockIdx.x * NP, s = g % 3, r1 = pair0 + g / 3, r2 = r1 + npairs;
-  long long* __restrict__ charges = inst[b].charges;
+  charges += (long long)blockIdx.y * grid * grid * kChargeStride;
   arow += (long long)blockIdx.y * M * ld;
   brow += (long long)blockIdx.y * (HM + 1) * ld;
   const float inv_q = cur[b].inv_qscale;
@@ -253,14 +254,15 @@ columns_convolve_kernel(float2* __restrict__ arow, float2* __restrict__ brow, co
 template <int LOGM>
 __global__ void __launch_bounds__(3 * Blocks<LOGM>::PAIRS* FftPlan<LOGM>::T, Blocks<LOGM>::ROW_BLOCKS)
 rows_inverse_kernel(const float2* __restrict__ arow, const float2* __restrict__ brow,
-                    const TsneInstance* __restrict__ inst, const int* __restrict__ members, int grid, int nodes, int ld,
+                    float4* __restrict__ potential, const TsneInstance* __restrict__ inst,
+                    const int* __restrict__ members, int first, int grid, int nodes, int ld,
                     const float2* __restrict__ tw, const double* __restrict__ zpart, int zblocks,
                     GridState* __restrict__ cur) {
   using P = FftPlan<LOGM>;
   constexpr int M = P::M, HM = M / 2, NP = Blocks<LOGM>::PAIRS, THREADS = 3 * NP * P::T;
   extern __shared__ float2 sbuf[];
-  const int b = members[blockIdx.y];
   if (blockIdx.x == gridDim.x - 1) {
+    const int b = blockIdx.y == 0 ? first : members[blockIdx.y];
     __shared__ double s_z[THREADS / 32];
     double z = 0.0;
     for (int t = threadIdx.x; t < zblocks; t += THREADS) z += zpart[(long long)blockIdx.y * zblocks + t];
@@ -277,7 +279,7 @@ rows_inverse_kernel(const float2* __restrict__ arow, const float2* __restrict__ 
     return;
   }
   const int g = threadIdx.x / P::T, tid = threadIdx.x % P::T, npairs = ld / 2, pair0 = blockIdx.x * NP;
-  float4* __restrict__ potential = inst[b].potential;
+  potential += (long long)blockIdx.y * grid * grid;
   arow += (long long)blockIdx.y * M * ld;
   brow += (long long)blockIdx.y * (HM + 1) * ld;
   // in batches whose loads are all in flight before the first is stored
@@ -366,8 +368,8 @@ struct Pass {
   static void rows_forward(const TsneDevice& d, const GridClass& c, cudaStream_t s) {
     const int charge = ceil_div(c.ld / 2, B::PAIRS);
     rows_forward_kernel<LOGM><<<dim3(charge + ceil_div(c.nodes, B::KROWS), c.count), 3 * B::PAIRS * P::T,
-                                3 * B::PAIRS * kSeq, s>>>(d.d_inst, c.members, c.grid, c.nodes, c.ld, c.twiddle,
-                                                          d.cur, charge, c.arow, c.brow, c.krow);
+                                3 * B::PAIRS * kSeq, s>>>(c.charges, c.members, c.first, c.grid, c.nodes, c.ld,
+                                                          c.twiddle, d.cur, charge, c.arow, c.brow, c.krow);
     FE_LAUNCH("rows_forward_kernel");
   }
   static void columns(const TsneDevice&, const GridClass& c, cudaStream_t s) {
@@ -377,8 +379,9 @@ struct Pass {
   }
   static void rows_inverse(const TsneDevice& d, const GridClass& c, cudaStream_t s) {
     rows_inverse_kernel<LOGM><<<dim3(ceil_div(c.ld / 2, B::PAIRS) + 1, c.count), 3 * B::PAIRS * P::T,
-                                3 * B::PAIRS * kSeq, s>>>(c.arow, c.brow, d.d_inst, c.members, c.grid, c.nodes,
-                                                          c.ld, c.twiddle, c.zpart, c.col_blocks, d.cur);
+                                3 * B::PAIRS * kSeq, s>>>(c.arow, c.brow, c.potential, d.d_inst, c.members, c.first,
+                                                          c.grid, c.nodes, c.ld, c.twiddle, c.zpart, c.col_blocks,
+                                                          d.cur);
     FE_LAUNCH("rows_inverse_kernel");
   }
 };

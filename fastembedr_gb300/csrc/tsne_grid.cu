@@ -62,6 +62,12 @@ __device__ __forceinline__ Stencil<TAPS> make_stencil(float x, float x0, float i
   return s;
 }
 
+// (instance, first slot) of this point block. A single instance needs no table (null): its blocks
+// follow one another, and the kernels that a small layout waits for have one load less in their chain.
+__device__ __forceinline__ int2 point_block(const int2* __restrict__ blocks) {
+  return blocks ? blocks[blockIdx.x] : make_int2(0, (int)blockIdx.x * kPointBlock);
+}
+
 // ---------------------------------------------------------------- layout statistics
 // Fixed-order reduction of the per-block partials into the grid of the next iteration
 // (the bounding-square rule of src/tsne_neighbors.cpp:1168-1184).
@@ -86,22 +92,28 @@ __device__ void finish_layout_stats(const StepPartial* __restrict__ part, int nb
   mxx = warp_max(mxx);
   mny = warp_min(mny);
   mxy = warp_max(mxy);
-  if (nblocks > 1) {
+  // (warps without a partial stay off the FP64 pipe: a warp's two sums hold it for 190 cycles)
+  if (nblocks > 1 && (int)(threadIdx.x & ~31u) < nblocks) {
     sx = warp_sum(sx);
     sy = warp_sum(sy);
   }
   if ((threadIdx.x & 31) == 0) s_stat[threadIdx.x >> 5] = StepPartial{mnx, mxx, mny, mxy, sx, sy};
   __syncthreads();
+  // warps without a partial hold the neutral values
+  const int warps = min((int)(blockDim.x / 32), (nblocks + 31) / 32);
+  if (threadIdx.x == 32 || threadIdx.x == 64) {  // the means, beside the box
+    const bool is_x = threadIdx.x == 32;
+    double sum = is_x ? s_stat[0].sum_x : s_stat[0].sum_y;
+    for (int w = 1; w < warps; ++w) sum += is_x ? s_stat[w].sum_x : s_stat[w].sum_y;
+    (is_x ? next->mean_x : next->mean_y) = sum / (double)n;
+  }
   if (threadIdx.x == 0) {
     StepPartial p = s_stat[0];
-    // warps without a partial hold the neutral values
-    for (int w = 1; w < (int)(blockDim.x / 32) && w * 32 < nblocks; ++w) {
+    for (int w = 1; w < warps; ++w) {
       p.min_x = fminf(p.min_x, s_stat[w].min_x);
       p.max_x = fmaxf(p.max_x, s_stat[w].max_x);
       p.min_y = fminf(p.min_y, s_stat[w].min_y);
       p.max_y = fmaxf(p.max_y, s_stat[w].max_y);
-      p.sum_x += s_stat[w].sum_x;
-      p.sum_y += s_stat[w].sum_y;
     }
     const float min_x = p.min_x, max_x = p.max_x, min_y = p.min_y, max_y = p.max_y;
     GridState g;
@@ -124,10 +136,6 @@ __device__ void finish_layout_stats(const StepPartial* __restrict__ part, int nb
     }
     g.inv_h = 1.0f / g.h;
     g.inv_box = 1.0f / g.box;
-    g.mean_x = p.sum_x / (double)n;
-    g.mean_y = p.sum_y / (double)n;
-    g.z = 0.0;
-    g.inv_z = 0.0f;
     // |mass| and |mass * d| summed over any subset of points stay below 1.5625 n max(half, 1)
     // (stencil weights sum to 1 in absolute value for bilinear, 1.5625 for Lagrange; |d| <= half):
     // scale so that bound stays below 2^62.
@@ -144,7 +152,21 @@ __device__ void finish_layout_stats(const StepPartial* __restrict__ part, int nb
     frexpf(tbound, &et);
     g.tile_shift = (62 - e) - (30 - et);  // >= 0: et <= e
     g.tscale = ldexpf(1.0f, 30 - et);
-    *next = g;
+    next->x0 = g.x0;
+    next->y0 = g.y0;
+    next->h = g.h;
+    next->inv_h = g.inv_h;
+    next->box = g.box;
+    next->inv_box = g.inv_box;
+    next->cx = g.cx;
+    next->cy = g.cy;
+    next->z = 0.0;
+    next->inv_z = 0.0f;
+    next->nodes = g.nodes;
+    next->qscale = g.qscale;
+    next->inv_qscale = g.inv_qscale;
+    next->tscale = g.tscale;
+    next->tile_shift = g.tile_shift;
   }
 }
 
@@ -249,27 +271,30 @@ __device__ __forceinline__ void red_add_i64(long long* p, long long v) {
 template <int TAPS>
 __global__ void __launch_bounds__(256)
 scatter_kernel(const float2* __restrict__ y, const TsneInstance* __restrict__ inst, const int2* __restrict__ blocks,
-               GridState* __restrict__ cur, const GridState* __restrict__ next) {
+               GridState* __restrict__ cur, const GridState* __restrict__ next, int n) {
   constexpr int NV = TAPS * TAPS * 3;
-  __shared__ int tile[kScatterTile * kScatterTile * 3];
+  __shared__ __align__(16) int tile[kScatterTile * kScatterTile * 3];
   __shared__ int s_box[4];
-  const int2 bl = blocks[blockIdx.x];
+  const int2 bl = point_block(blocks);
+  const int i = bl.y + threadIdx.x;
+  // the point is requested beside the instance and grid records (clamped as in the update)
+  const float2 own = y[min(i, n - 1)];
   const TsneInstance I = inst[bl.x];
   const int grid = I.grid;
   long long* __restrict__ charges = I.charges;
   const GridState g = next[bl.x];
-  if (bl.y == I.pt_begin && threadIdx.x == 0) cur[bl.x] = g;
   const int lane = threadIdx.x & 31;
-  for (int t = threadIdx.x; t < kScatterTile * kScatterTile * 3; t += blockDim.x) tile[t] = 0;
+  for (int t = threadIdx.x; t < kScatterTile * kScatterTile * 3 / 4; t += blockDim.x)
+    reinterpret_cast<int4*>(tile)[t] = make_int4(0, 0, 0, 0);
   if (threadIdx.x == 0) {
     s_box[0] = INT_MAX;
     s_box[1] = INT_MAX;
     s_box[2] = -1;
     s_box[3] = -1;
   }
-  const int i = bl.y + threadIdx.x;
+  if (bl.y == I.pt_begin && threadIdx.x == 0) cur[bl.x] = g;
   const bool valid = i < I.pt_begin + I.n;
-  const float2 p = valid ? y[i] : make_float2(g.cx, g.cy);
+  const float2 p = valid ? own : make_float2(g.cx, g.cy);
   const Stencil<TAPS> sx = make_stencil<TAPS>(p.x, g.x0, g.inv_h, g.inv_box, g.nodes);
   const Stencil<TAPS> sy = make_stencil<TAPS>(p.y, g.y0, g.inv_h, g.inv_box, g.nodes);
   const float dx = p.x - g.cx, dy = p.y - g.cy;
@@ -302,11 +327,16 @@ scatter_kernel(const float2* __restrict__ y, const TsneInstance* __restrict__ in
   }
   const bool head = valid && ((heads >> lane) & 1u);
   __syncthreads();
-  if (head) {
-    atomicMin(&s_box[0], sx.base);
-    atomicMin(&s_box[1], sy.base);
-    atomicMax(&s_box[2], sx.base);
-    atomicMax(&s_box[3], sy.base);
+  // the block's anchors: a reduction per warp first (32 lanes on one address would take turns)
+  const int x_lo = __reduce_min_sync(0xffffffffu, head ? sx.base : INT_MAX);
+  const int y_lo = __reduce_min_sync(0xffffffffu, head ? sy.base : INT_MAX);
+  const int x_hi = __reduce_max_sync(0xffffffffu, head ? sx.base : -1);
+  const int y_hi = __reduce_max_sync(0xffffffffu, head ? sy.base : -1);
+  if (lane == 0 && x_hi >= 0) {
+    atomicMin(&s_box[0], x_lo);
+    atomicMin(&s_box[1], y_lo);
+    atomicMax(&s_box[2], x_hi);
+    atomicMax(&s_box[3], y_hi);
   }
   __syncthreads();
   const int ox = s_box[0], oy = s_box[1];
@@ -649,7 +679,7 @@ update_kernel(float2* __restrict__ y, const float2* __restrict__ attr, float2* _
               const GridState* __restrict__ cur, GridState* __restrict__ next, StepPartial* __restrict__ part,
               unsigned* __restrict__ counter, int n, int mode, float lr, float mom, float min_gain, float max_step,
               float2* __restrict__ out_rep) {
-  const int2 bl = blocks[blockIdx.x];
+  const int2 bl = point_block(blocks);
   const int i = bl.y + threadIdx.x;
   // the point's state is requested beside the instance and grid records (clamped: the last block of
   // the last instance may reach past the end)
@@ -869,6 +899,7 @@ void build_grid_classes(TsneDevice& d, const std::vector<int>& grids) {
     k.fft = 2 * k.grid;
     k.log_fft = log2_ceil(k.fft);
     k.count = (int)members[c].size();
+    k.first = members[c][0];
     fft_class_layout(k);
     const std::size_t m = k.fft, ld = k.ld;
     d.grid_arena.reserve(&k.charges, (std::size_t)k.count * k.grid * k.grid * kChargeStride);
@@ -1018,11 +1049,13 @@ void tsne_device_init(TsneDevice& d, const float* d_init, cudaStream_t s) {
   FE_LAUNCH("layout_stats_kernel");
 }
 
+static const int2* block_table(const TsneDevice& d) { return d.inst.size() == 1 ? nullptr : d.blocks; }
+
 void tsne_grid_stage(TsneDevice& d, cudaStream_t s) {
   if (d.mode == kInterpBilinear)
-    scatter_kernel<2><<<d.nblocks, kPointBlock, 0, s>>>(d.y, d.d_inst, d.blocks, d.cur, d.next);
+    scatter_kernel<2><<<d.nblocks, kPointBlock, 0, s>>>(d.y, d.d_inst, block_table(d), d.cur, d.next, d.n);
   else
-    scatter_kernel<3><<<d.nblocks, kPointBlock, 0, s>>>(d.y, d.d_inst, d.blocks, d.cur, d.next);
+    scatter_kernel<3><<<d.nblocks, kPointBlock, 0, s>>>(d.y, d.d_inst, block_table(d), d.cur, d.next, d.n);
   FE_LAUNCH("scatter_kernel");
   fft_convolve(d, s);
 }
@@ -1088,11 +1121,11 @@ bool tsne_tune_attractive(TsneDevice& d, const DeviceCsr& P, float exag, cudaStr
 
 void tsne_update_stage(TsneDevice& d, float lr, float mom, float min_gain, float max_step, cudaStream_t s) {
   if (d.mode == kInterpBilinear)
-    update_kernel<2, false><<<d.nblocks, kStepThreads, 0, s>>>(d.y, d.attr, d.gains, d.update, d.d_inst, d.blocks,
+    update_kernel<2, false><<<d.nblocks, kStepThreads, 0, s>>>(d.y, d.attr, d.gains, d.update, d.d_inst, block_table(d),
                                                                 d.cur, d.next, d.partial, d.counter, d.n, d.mode, lr, mom,
                                                                 min_gain, max_step, nullptr);
   else
-    update_kernel<3, false><<<d.nblocks, kStepThreads, 0, s>>>(d.y, d.attr, d.gains, d.update, d.d_inst, d.blocks,
+    update_kernel<3, false><<<d.nblocks, kStepThreads, 0, s>>>(d.y, d.attr, d.gains, d.update, d.d_inst, block_table(d),
                                                                 d.cur, d.next, d.partial, d.counter, d.n, d.mode, lr, mom,
                                                                 min_gain, max_step, nullptr);
   FE_LAUNCH("update_kernel");
@@ -1115,11 +1148,11 @@ void tsne_forces(TsneDevice& d, const DeviceCsr& P, float exag, float* d_attr, f
   FE_CUDA(cudaMemcpyAsync(d_attr, d.attr, sizeof(float2) * d.n, cudaMemcpyDeviceToDevice, s));
   float2* r = reinterpret_cast<float2*>(d_rep);
   if (d.mode == kInterpBilinear)
-    update_kernel<2, true><<<d.nblocks, kStepThreads, 0, s>>>(d.y, d.attr, d.gains, d.update, d.d_inst, d.blocks,
+    update_kernel<2, true><<<d.nblocks, kStepThreads, 0, s>>>(d.y, d.attr, d.gains, d.update, d.d_inst, block_table(d),
                                                                d.cur, d.next, d.partial, d.counter, d.n, d.mode, 0.0f,
                                                                0.0f, 0.0f, 0.0f, r);
   else
-    update_kernel<3, true><<<d.nblocks, kStepThreads, 0, s>>>(d.y, d.attr, d.gains, d.update, d.d_inst, d.blocks,
+    update_kernel<3, true><<<d.nblocks, kStepThreads, 0, s>>>(d.y, d.attr, d.gains, d.update, d.d_inst, block_table(d),
                                                                d.cur, d.next, d.partial, d.counter, d.n, d.mode, 0.0f,
                                                                0.0f, 0.0f, 0.0f, r);
   FE_LAUNCH("update_kernel(diagnostic)");

@@ -57,6 +57,7 @@ struct GridClass {
   int grid = 0, nodes = 0, fft = 0, log_fft = 0;
   int count = 0;
   int* members = nullptr;     // device: the class's instance indices
+  int first = 0;               // members[0]
   int ld = 0;                  // rows of a column of the spectra: nodes rounded up to even
   int col_blocks = 0;          // blocks of the column pass
   int twiddles = 0;
