@@ -1,0 +1,30 @@
+// Normal draws of the std::mt19937 stream on the GPU.
+#pragma once
+
+#include <cstddef>
+#include <cstdint>
+
+#include "common.cuh"
+
+namespace fe {
+
+// out[i] = scale * draw i of N(0, sd) from a freshly seeded std::mt19937, in the order of
+// std::normal_distribution (Marsaglia's polar method; see normal_stream.cuh), for an even count. The words and the
+// accepted points are those of the host stream; logarithm and root are CUDA's (within a unit in the last place of the
+// host's). *enough is set to 1 when the words sufficed (they do but for one seed in far more than 10^9).
+class MtNormalBlock {
+ public:
+  MtNormalBlock(std::uint32_t seed, std::size_t count, double sd, double scale);
+  ~MtNormalBlock();
+  // Copies the draws to dst on stream s, after them; false when the words did not suffice.
+  bool copy_to(double* dst, cudaStream_t s);
+
+ private:
+  Stream stream_;
+  Arena arena_;
+  double* out_ = nullptr;
+  int* enough_ = nullptr;
+  std::size_t count_;
+};
+
+}  // namespace fe

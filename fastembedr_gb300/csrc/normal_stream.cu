@@ -96,6 +96,10 @@ void NormalStream::fill_polar(std::mt19937& g, double* out, std::size_t count, d
   }
 }
 
+void NormalStream::skip(std::mt19937& g, std::size_t pairs) {
+  for (std::size_t i = 0; i < pairs; ++i) polar_point(g);
+}
+
 bool NormalStream::self_check() {
   const std::uint32_t seeds[] = {1u, 42u, 2026u};
   for (std::uint32_t seed : seeds) {

@@ -21,6 +21,8 @@ class NormalStream {
   double next(std::mt19937& g);
   // out[i] = next(g) * scale for i < count
   void fill(std::mt19937& g, double* out, std::size_t count, double scale);
+  // Advances the engine past `pairs` pairs of the polar path, without their values.
+  static void skip(std::mt19937& g, std::size_t pairs);
   // whether the polar path reproduces std::normal_distribution here (and is used)
   static bool polar_path();
 

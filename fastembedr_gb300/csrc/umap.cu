@@ -1281,7 +1281,9 @@ void umap_knn_spectral_job(const int* d_idx, const float* d_dist, int n, int k, 
   // the GPU validates the KNN and builds the graph
   std::future<SpectralDraws> own;
   if (!early) {
-    own = std::async(std::launch::async, spectral_draws, n, (int)seed);
+    int device = 0;
+    FE_CUDA(cudaGetDevice(&device));
+    own = std::async(std::launch::async, spectral_draws, n, (int)seed, device, false);
     early = &own;
   }
   UmapJob job;
@@ -1685,7 +1687,9 @@ int fastembedr_cuda_umap_spectral_init_from_knn(const int* indices, const float*
   return fe::guarded([&] {
     if (!indices || !distances || !out) throw fe::Error("null host pointer");
     if (n < 2 || k < 1 || spectral_n_iter < 1) throw fe::Error("invalid spectral initialization parameters");
-    auto draws = std::async(std::launch::async, fe::spectral_draws, n, seed);
+    int device = 0;
+    FE_CUDA(cudaGetDevice(&device));
+    auto draws = std::async(std::launch::async, fe::spectral_draws, n, seed, device, false);
     fe::Stream st;
     const std::size_t items = (std::size_t)n * k;
     int* d_idx = nullptr;
@@ -1771,7 +1775,9 @@ static int umap_knn_spectral(const int* indices, const float* distances, bool ro
     if (n < 2 || k < 1 || n_epochs < 1 || negative_sample_rate < 0 || !(learning_rate > 0.0f) || min_dist < 0.0f ||
         !(repulsion_strength > 0.0f) || spectral_n_iter < 1)
       throw fe::Error("invalid CUDA UMAP parameters");
-    auto draws = std::async(std::launch::async, fe::spectral_draws, n, (int)seed);
+    int device = 0;
+    FE_CUDA(cudaGetDevice(&device));
+    auto draws = std::async(std::launch::async, fe::spectral_draws, n, (int)seed, device, false);
     fe::Stream st;
     const std::size_t items = (std::size_t)n * k;
     int* d_idx = nullptr;

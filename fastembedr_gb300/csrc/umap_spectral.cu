@@ -11,8 +11,8 @@
 // (scale_embedding_max_abs_and_jitter, :2705-2730), then the optional scale_embedding_sdev
 // (:2681-2703).
 //
-// The random draws are made on the host in the reference's order (the column redraw of a
-// vanishing Gram-Schmidt column included) and uploaded; every arithmetic step runs on the GPU in
+// The random draws are made in the reference's order (on the host, or the start block of a large layout on
+// the GPU; the column redraw of a vanishing Gram-Schmidt column included); every arithmetic step runs on the GPU in
 // FP64 with the reference's operation order and no contraction (__d*_rn). Sums over points are
 // reduced in a fixed block order, so results are deterministic and differ from the sequential
 // CPU sums by rounding only.
@@ -885,19 +885,29 @@ __global__ void sp_rescale_kernel(double* __restrict__ col, int n, const double*
 
 }  // namespace
 
-SpectralDraws spectral_draws(int n, int seed) {
+SpectralDraws spectral_draws(int n, int seed, int device, bool on_host) {
   SpectralDraws d;
-  d.rng.seed((std::uint32_t)seed);
+  d.n = n;
   const int B = std::min(n - 1, kSpBlock);
   if (B < 2) return d;
-  d.block.resize((std::size_t)n * B);
-  d.normal.fill(d.rng, d.block.data(), d.block.size(), 10000.0);
-  d.jitter = std::async(std::launch::async, [ahead = d.rng, n]() mutable {
-               NormalStream jitter(0.0, 1e-4);
-               std::vector<double> v(2 * (std::size_t)n);
-               jitter.fill(ahead, v.data(), v.size(), 1.0);
-               return v;
-             }).share();
+  const std::size_t count = (std::size_t)n * B;
+  std::mt19937 rng((std::uint32_t)seed);
+  // (an odd count leaves a value in the host stream; a polar path that is not the library's has no twin)
+  const bool on_device = !on_host && n >= kSpectralDeviceDraws && count % 2 == 0 && NormalStream::polar_path();
+  if (on_device) {
+    FE_CUDA(cudaSetDevice(device));
+    d.device = std::make_shared<MtNormalBlock>((std::uint32_t)seed, count, 1e-4, 10000.0);
+  } else {
+    d.block.resize(count);
+    d.normal.fill(rng, d.block.data(), count, 10000.0);
+  }
+  d.tail = std::async(std::launch::async, [rng, n, skip = on_device ? count / 2 : 0]() mutable {
+             NormalStream::skip(rng, skip);
+             SpectralTail t{rng, std::vector<double>(2 * (std::size_t)n)};
+             NormalStream jitter(0.0, 1e-4);
+             jitter.fill(rng, t.jitter.data(), t.jitter.size(), 1.0);
+             return t;
+           }).share();
   return d;
 }
 
@@ -950,10 +960,17 @@ void umap_spectral_start(const int* offsets, const int* neighbors, const float* 
     FE_CUDA(cudaMemcpyAsync(grid, &g0, sizeof(SpGrid), cudaMemcpyHostToDevice, s));
     SpectralDraws local;
     SpectralDraws* dr = pre;
-    if (!dr || dr->block.size() != (std::size_t)n * B) {
-      local = spectral_draws(n, seed);
+    int dev = 0, coop = 0;
+    FE_CUDA(cudaGetDevice(&dev));
+    if (!dr || dr->n != n) {
+      local = spectral_draws(n, seed, dev);
       dr = &local;
     }
+    if (dr->device && !dr->device->copy_to(q, s)) {
+      local = spectral_draws(n, seed, dev, true);
+      dr = &local;
+    }
+    std::mt19937 live;  // the stream after the block, from the first redraw on
     bool redrawn = false;
 
     // The subspace iteration as cooperative launches: the initial orthonormalisation (round -1) and
@@ -969,11 +986,10 @@ void umap_spectral_start(const int* offsets, const int* neighbors, const float* 
     int per_sm = 0;
     FE_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, rounds, kSpRoundThreads, smem));
     if (per_sm * sm_count() < parts) throw Error("the spectral start's subspace iteration cannot be made resident");
-    int dev = 0, coop = 0;
-    FE_CUDA(cudaGetDevice(&dev));
     FE_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
     if (!coop) throw Error("the device does not support cooperative launches");
-    FE_CUDA(cudaMemcpyAsync(q, dr->block.data(), sizeof(double) * dr->block.size(), cudaMemcpyHostToDevice, s));
+    if (!dr->device)
+      FE_CUDA(cudaMemcpyAsync(q, dr->block.data(), sizeof(double) * dr->block.size(), cudaMemcpyHostToDevice, s));
     int r0 = -1, from = 0, mult = 0;
     for (;;) {
       int r_end = spectral_n_iter;
@@ -990,9 +1006,10 @@ void umap_spectral_start(const int* offsets, const int* neighbors, const float* 
       if (g1.status < 0) break;
       const int rr = g1.status / 16 - 1, f = g1.status % 16;
       if (rr < -1 || rr >= spectral_n_iter || f < 0 || f >= B) throw Error("spectral start: invalid redraw status");
+      if (!redrawn) live = dr->tail.get().rng;
       redrawn = true;
       host.resize(n);
-      dr->normal.fill(dr->rng, host.data(), host.size(), 10000.0);
+      dr->normal.fill(live, host.data(), host.size(), 10000.0);
       // the later columns back to their post-multiply values where the pass had started on them, then
       // the redrawn column
       double* m = ((rr + 1) & 1) ? z : q;
@@ -1024,9 +1041,9 @@ void umap_spectral_start(const int* offsets, const int* neighbors, const float* 
     if (redrawn) {
       NormalStream jitter(0.0, 1e-4);
       fresh.resize(2 * (std::size_t)n);
-      jitter.fill(dr->rng, fresh.data(), fresh.size(), 1.0);
+      jitter.fill(live, fresh.data(), fresh.size(), 1.0);
     }
-    const std::vector<double>& jv = redrawn ? fresh : dr->jitter.get();
+    const std::vector<double>& jv = redrawn ? fresh : dr->tail.get().jitter;
     FE_CUDA(cudaMemcpyAsync(jit, jv.data(), sizeof(double) * jv.size(), cudaMemcpyHostToDevice, s));
     sp_expand_kernel<<<gb, kSpThreads, 0, s>>>(out, n, pc, nb, jit);
     FE_LAUNCH("sp_expand_kernel");

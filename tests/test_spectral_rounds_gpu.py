@@ -1,6 +1,7 @@
 """The subspace iteration of the CPU spectral start at the edges of its row split: fewer rows than a warp, one and two
 warps per block (152 blocks of 32 rows hold 4,864), one and two tiles (77,824 rows), rows in the global buffers (more
-than 524,552), and fewer points than the block has columns."""
+than 524,552), fewer points than the block has columns, and both sides of the line (8,192) from which the start
+block is drawn on the GPU."""
 import numpy as np
 import pytest
 
@@ -25,7 +26,7 @@ def ring(n, rng):
 # the projected matrix (1e-16 sqrt(n) at most) over the gap of the Ritz values, which for 8 random directions is
 # above 1e-4 but for rare draws: 1e-9 of the layout's 10, and four decades of room for the division by the largest
 # coordinate and the rounds' own amplification.
-@pytest.mark.parametrize("n,iters", [(5, 3), (31, 3), (33, 3), (4864, 3), (4865, 3), (77824, 2), (77825, 2), (100001, 2),
+@pytest.mark.parametrize("n,iters", [(5, 3), (31, 3), (33, 3), (4864, 3), (4865, 3), (8191, 3), (8192, 3), (30001, 2), (77824, 2), (77825, 2), (100001, 2),
                                      (560000, 1)])
 def test_spectral_rounds_edges(n, iters):
     off, nb, w = ring(n, np.random.default_rng(n))
