@@ -315,8 +315,9 @@ scatter_kernel(const float2* __restrict__ y, const TsneInstance* __restrict__ in
     // suffix sums restricted to contiguous runs [lane, next head)
     const unsigned above = heads & ~((2u << lane) - 1u);
     const int run_end = above ? __ffs(above) - 1 : 32;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
+    // no further than the longest run (the levels beyond add nothing)
+    const int longest = __reduce_max_sync(0xffffffffu, run_end - lane);
+    for (int off = 1; off < longest; off <<= 1) {
       const bool take = lane + off < run_end;
 #pragma unroll
       for (int c = 0; c < NV; ++c) {
