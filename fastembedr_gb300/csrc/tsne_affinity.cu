@@ -4,8 +4,8 @@
 // Reference behaviour followed (fastEmbedR):
 //   - index/distance validation and messages: src/tsne_neighbors.cpp:630-640
 //   - per-row bisection: src/tsne_neighbors.cpp:532-614 (control flow, tolerance 1e-5,
-//     200 iterations, uniform fallback) evaluated with FP32 exp and FP64 sums as in the
-//     FP64 test oracle tests/testthat/helper-tsne-reference.R:1-54
+//     200 iterations, uniform fallback) evaluated in two floats, so that it takes the
+//     steps of the FP64 test oracle tests/testthat/helper-tsne-reference.R:1-54
 //   - symmetrisation: src/tsne_neighbors.cpp:616-724 (self edges skipped, duplicate
 //     directed edges summed in double, value = float(sum) * float(0.5 / total))
 //
