@@ -257,7 +257,9 @@ layout_stats_kernel(const float2* __restrict__ ynew, const TsneInstance* __restr
 //   2. run heads accumulate into a kTile x kTile node tile in shared memory anchored at the block's
 //      lowest anchor, in 32-bit fixed point (the run sums rounded to a multiple of 1 / tscale,
 //      about 2^-30 of the largest sum a block can make; native 32-bit shared atomics); heads
-//      outside the tile add to the grid directly in 64-bit fixed point (x qscale);
+//      outside the tile add to the grid directly in 64-bit fixed point (x qscale), four lanes a node, so that its
+//      three sums leave the SM as one request (a lane per head kept the few SMs of a small layout busy with
+//      12 requests a point: twenty iterations at 2,000 points 785 -> 673 us, at 100,000 3.22 -> 3.14 ms);
 //   3. the tile is flushed with one 64-bit integer atomic per touched node and value, the tile sum
 //      shifted up to the grid's scale (exact: both scales are powers of two).
 // Integer sums do not depend on the order in which atomics arrive, so the charges (and the
@@ -275,6 +277,7 @@ scatter_kernel(const float2* __restrict__ y, const TsneInstance* __restrict__ in
   constexpr int NV = TAPS * TAPS * 3;
   __shared__ __align__(16) int tile[kScatterTile * kScatterTile * 3];
   __shared__ int s_box[4];
+  __shared__ float4 s_beyond[kPointBlock / 32][32];
   const int2 bl = point_block(blocks);
   const int i = bl.y + threadIdx.x;
   // the point is requested beside the instance and grid records (clamped as in the update)
@@ -341,32 +344,42 @@ scatter_kernel(const float2* __restrict__ y, const TsneInstance* __restrict__ in
   }
   __syncthreads();
   const int ox = s_box[0], oy = s_box[1];
-  if (head) {
-    const int tx = sx.base - ox, ty = sy.base - oy;
-    if (tx + TAPS <= kScatterTile && ty + TAPS <= kScatterTile) {
+  const int tx = sx.base - ox, ty = sy.base - oy;
+  const bool in_tile = tx + TAPS <= kScatterTile && ty + TAPS <= kScatterTile;
+  if (head && in_tile) {
 #pragma unroll
-      for (int a = 0; a < TAPS; ++a)
+    for (int a = 0; a < TAPS; ++a)
 #pragma unroll
-        for (int b = 0; b < TAPS; ++b) {
-          int* t = tile + ((ty + a) * kScatterTile + tx + b) * 3;
-          const int c = (a * TAPS + b) * 3;
-          atomicAdd(t, __float2int_rn(v[c] * g.tscale));
-          atomicAdd(t + 1, __float2int_rn(v[c + 1] * g.tscale));
-          atomicAdd(t + 2, __float2int_rn(v[c + 2] * g.tscale));
-        }
-    } else {
-#pragma unroll
-      for (int a = 0; a < TAPS; ++a) {
-        long long* row = charges + ((long long)(sy.base + a) * grid + sx.base) * kChargeStride;
-#pragma unroll
-        for (int b = 0; b < TAPS; ++b) {
-          const int c = (a * TAPS + b) * 3;
-          red_add_i64(row + b * kChargeStride, __float2ll_rn(v[c] * g.qscale));
-          red_add_i64(row + b * kChargeStride + 1, __float2ll_rn(v[c + 1] * g.qscale));
-          red_add_i64(row + b * kChargeStride + 2, __float2ll_rn(v[c + 2] * g.qscale));
-        }
+      for (int b = 0; b < TAPS; ++b) {
+        int* t = tile + ((ty + a) * kScatterTile + tx + b) * 3;
+        const int c = (a * TAPS + b) * 3;
+        atomicAdd(t, __float2int_rn(v[c] * g.tscale));
+        atomicAdd(t + 1, __float2int_rn(v[c + 1] * g.tscale));
+        atomicAdd(t + 2, __float2int_rn(v[c + 2] * g.tscale));
       }
-    }
+  }
+  // Heads beyond the tile, node by node: four lanes take one node's three sums, which lie in one 32-byte
+  // sector and leave the SM as one request (a lane per head sent three).
+  const unsigned beyond = __ballot_sync(0xffffffffu, head && !in_tile);
+  if (beyond) {
+    float4* mine = s_beyond[threadIdx.x >> 5];
+    const int rank = __popc(beyond & ((1u << lane) - 1u)), count = 4 * __popc(beyond);
+#pragma unroll
+    for (int a = 0; a < TAPS; ++a)
+#pragma unroll
+      for (int b = 0; b < TAPS; ++b) {
+        const int c = (a * TAPS + b) * 3;
+        if (head && !in_tile)
+          mine[rank] = make_float4(v[c], v[c + 1], v[c + 2],
+                                   __int_as_float(((sy.base + a) * grid + sx.base + b) * kChargeStride));
+        __syncwarp();
+        for (int t = lane; t < count; t += 32) {
+          const float* e = reinterpret_cast<const float*>(mine + (t >> 2));
+          const int u = t & 3;
+          if (u < 3) red_add_i64(charges + __float_as_int(e[3]) + u, __float2ll_rn(e[u] * g.qscale));
+        }
+        __syncwarp();
+      }
   }
   __syncthreads();
   if (s_box[2] < 0) return;  // no valid point in this block
