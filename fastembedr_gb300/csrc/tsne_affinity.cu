@@ -209,11 +209,9 @@ row_probabilities_kernel(const float* __restrict__ dist, int n, int k, double lo
       float* sf = stile + rr * stride;
       const float m2 = __fmul_rn(min_d, min_d);
       const Float2Sum min2{m2, __fmaf_rn(min_d, min_d, -m2)};
-      // squares near the smallest floats have no room for a low part: FP64 for such a row
-      const bool tiny = max_f < 1.0e-28f;
       const double dmin2 = (double)min_d * (double)min_d;
-      for (int j = 0; j < k; ++j)
-        sf[j] = tiny ? (float)((double)d[j] * (double)d[j] - dmin2) : shifted_square(d[j], min2).hi;
+      // (max_f is above 1e-7 here, so a square that counts has room for its low part)
+      for (int j = 0; j < k; ++j) sf[j] = shifted_square(d[j], min2).hi;
       const Float2Sum target = split(-log_perplexity);
       double beta = 1.0, beta_min = -DBL_MAX, beta_max = DBL_MAX;
       double beta_eval = beta;
@@ -255,7 +253,7 @@ row_probabilities_kernel(const float* __restrict__ dist, int n, int k, double lo
         beta_eval = beta;
         sum_eval = sp;
         double dd = value(diff);
-        if (exact_eval && (tiny || fabs(fabs(dd) - 1e-5) < 1e-10)) {
+        if (exact_eval && fabs(fabs(dd) - 1e-5) < 1e-10) {
           double xp = 0.0, xw = 0.0;
           for (int j = 0; j < k; ++j) {
             const double s = (double)d[j] * (double)d[j] - dmin2, p = exp(-beta * s);
@@ -282,7 +280,6 @@ row_probabilities_kernel(const float* __restrict__ dist, int n, int k, double lo
       for (int j = 0; j < k; ++j) {
         Float2Sum p{0.0f, 0.0f};
         if (!exact_eval) p.hi = expf(nb * sf[j]);
-        else if (tiny) p = split(exp(-beta_eval * ((double)d[j] * (double)d[j] - dmin2)));
         else p = exp_two(mul(shifted_square(d[j], min2), b2), exp_table);
         const Float2Sum v = mul(inv, p);
         d[j] = __fadd_rn(v.hi, v.lo);
