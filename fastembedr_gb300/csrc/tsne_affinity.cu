@@ -165,7 +165,11 @@ void upload_rows_as_columns(float* d_out, const void* values, bool is_double, in
 // of each step's entropy were four fifths of the time (100,000 rows of 45: 1.19 -> 0.26 ms; the
 // rest is FP32 exp and Kahan sums). The probabilities overwrite the row's distances and the CTA stores
 // them row-major with coalesced writes.
+// A step with beta beyond kFloatBeta is FP64 altogether, as are the probabilities at such a beta: where more
+// neighbours tie at the smallest distance than the perplexity, the entropy stays above the target, beta is
+// doubled out of the float range, and 0 times an infinite float is NaN.
 constexpr int kBisectRows = 128;
+constexpr double kFloatBeta = 1.0e30;
 
 __device__ __forceinline__ Float2Sum shifted_square(float d, Float2Sum min2) {
   const float p = __fmul_rn(d, d);
@@ -217,52 +221,62 @@ row_probabilities_kernel(const float* __restrict__ dist, int n, int k, double lo
       double beta_eval = beta;
       Float2Sum sum_eval{1.0f, 0.0f}, ent{0.0f, 0.0f};
       bool exact_eval = false;
-      for (int it = 0; it < 200; ++it) {
-        const float nb = (float)(-beta);
-        const Float2Sum b2 = split(beta);
-        float ps = 0.0f, pc = 0.0f, ws = 0.0f, wc = 0.0f;
+      // sum of the exponentials at b in FP64; *diff: distance of the entropy from the target
+      auto evaluate = [&](double b, double* diff) -> double {
+        double xp = 0.0, xw = 0.0;
         for (int j = 0; j < k; ++j) {
-          const float sj = sf[j];
-          const float p = expf(nb * sj);
-          const float yp = p - pc;
-          const float tp = ps + yp;
-          pc = (tp - ps) - yp;
-          ps = tp;
-          const float yw = sj * p - wc;
-          const float tw = ws + yw;
-          wc = (tw - ws) - yw;
-          ws = tw;
+          const double s = (double)d[j] * (double)d[j] - dmin2, p = exp(-b * s);
+          xp += p;
+          xw += s * p;
         }
-        Float2Sum sp = two_sum(ps, -pc), sw = two_sum(ws, -wc);
-        ent = add(divide(mul(sw, b2), sp), log_two(sp, log_table));
-        Float2Sum diff = add(ent, target);
-        exact_eval = false;
-        // The stop test is the only decision FP32 exp can flip: re-evaluate near its boundary.
-        if (fabsf(fabsf(diff.hi) - 1e-5f) < 1e-6f) {
-          sp = sw = Float2Sum{0.0f, 0.0f};
+        *diff = b * xw / xp + log(xp) - log_perplexity;
+        return xp;
+      };
+      double wide_sum = 0.0;  // of the last step, where that was FP64
+      for (int it = 0; it < 200; ++it) {
+        double dd = 0.0;
+        if (beta > kFloatBeta) {
+          wide_sum = evaluate(beta, &dd);
+          ent = split(dd + log_perplexity);
+        } else {
+          wide_sum = 0.0;
+          const float nb = (float)(-beta);
+          const Float2Sum b2 = split(beta);
+          float ps = 0.0f, pc = 0.0f, ws = 0.0f, wc = 0.0f;
           for (int j = 0; j < k; ++j) {
-            const Float2Sum s = shifted_square(d[j], min2);
-            const Float2Sum p = exp_two(mul(s, Float2Sum{-b2.hi, -b2.lo}), exp_table);
-            sp = add(sp, p);
-            sw = add(sw, mul(s, p));
+            const float sj = sf[j];
+            const float p = expf(nb * sj);
+            const float yp = p - pc;
+            const float tp = ps + yp;
+            pc = (tp - ps) - yp;
+            ps = tp;
+            const float yw = sj * p - wc;
+            const float tw = ws + yw;
+            wc = (tw - ws) - yw;
+            ws = tw;
           }
+          Float2Sum sp = two_sum(ps, -pc), sw = two_sum(ws, -wc);
           ent = add(divide(mul(sw, b2), sp), log_two(sp, log_table));
-          diff = add(ent, target);
-          exact_eval = true;
+          Float2Sum diff = add(ent, target);
+          exact_eval = false;
+          // The stop test is the only decision FP32 exp can flip: re-evaluate near its boundary.
+          if (fabsf(fabsf(diff.hi) - 1e-5f) < 1e-6f) {
+            sp = sw = Float2Sum{0.0f, 0.0f};
+            for (int j = 0; j < k; ++j) {
+              const Float2Sum s = shifted_square(d[j], min2);
+              const Float2Sum p = exp_two(mul(s, Float2Sum{-b2.hi, -b2.lo}), exp_table);
+              sp = add(sp, p);
+              sw = add(sw, mul(s, p));
+            }
+            ent = add(divide(mul(sw, b2), sp), log_two(sp, log_table));
+            diff = add(ent, target);
+            exact_eval = true;
+          }
+          sum_eval = sp;
+          dd = value(diff);
+          if (exact_eval && fabs(fabs(dd) - 1e-5) < 1e-10) sum_eval = split(evaluate(beta, &dd));
         }
         beta_eval = beta;
-        sum_eval = sp;
-        double dd = value(diff);
-        if (exact_eval && fabs(fabs(dd) - 1e-5) < 1e-10) {
-          double xp = 0.0, xw = 0.0;
-          for (int j = 0; j < k; ++j) {
-            const double s = (double)d[j] * (double)d[j] - dmin2, p = exp(-beta * s);
-            xp += p;
-            xw += s * p;
-          }
-          dd = beta * xw / xp + log(xp) - log_perplexity;
-          sum_eval = split(xp);
-        }
         if (fabs(dd) < 1e-5) break;
         if (dd > 0.0) {
           beta_min = beta;
@@ -278,6 +292,10 @@ row_probabilities_kernel(const float* __restrict__ dist, int n, int k, double lo
       const float nb = (float)(-beta_eval);
       const Float2Sum b2 = split(-beta_eval);
       for (int j = 0; j < k; ++j) {
+        if (wide_sum > 0.0) {
+          d[j] = (float)(exp(-beta_eval * ((double)d[j] * (double)d[j] - dmin2)) / wide_sum);
+          continue;
+        }
         Float2Sum p{0.0f, 0.0f};
         if (!exact_eval) p.hi = expf(nb * sf[j]);
         else p = exp_two(mul(shifted_square(d[j], min2), b2), exp_table);
