@@ -167,9 +167,11 @@ void upload_rows_as_columns(float* d_out, const void* values, bool is_double, in
 // them row-major with coalesced writes.
 // A step with beta beyond kFloatBeta is FP64 altogether, as are the probabilities at such a beta: where more
 // neighbours tie at the smallest distance than the perplexity, the entropy stays above the target, beta is
-// doubled out of the float range, and 0 times an infinite float is NaN.
+// doubled out of the float range, and 0 times an infinite float is NaN. So is a row with squares beyond kFloatSquare: the
+// sums of its squares may leave the float range.
 constexpr int kBisectRows = 128;
 constexpr double kFloatBeta = 1.0e30;
+constexpr float kFloatSquare = 1.0e30f;
 
 __device__ __forceinline__ Float2Sum shifted_square(float d, Float2Sum min2) {
   const float p = __fmul_rn(d, d);
@@ -232,10 +234,11 @@ row_probabilities_kernel(const float* __restrict__ dist, int n, int k, double lo
         *diff = b * xw / xp + log(xp) - log_perplexity;
         return xp;
       };
+      const bool far = !(max_f <= kFloatSquare);
       double wide_sum = 0.0;  // of the last step, where that was FP64
       for (int it = 0; it < 200; ++it) {
         double dd = 0.0;
-        if (beta > kFloatBeta) {
+        if (far || beta > kFloatBeta) {
           wide_sum = evaluate(beta, &dd);
           ent = split(dd + log_perplexity);
         } else {

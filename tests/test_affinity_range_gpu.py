@@ -1,9 +1,9 @@
-"""Perplexity search of rows whose precision leaves the float range: more neighbours tied at the smallest distance than
-the perplexity, where the entropy never reaches the target and the precision is doubled 200 times.
+"""Perplexity search of rows whose precision leaves the float range (more neighbours tied at the smallest distance than
+the perplexity, where the entropy never reaches the target and the precision is doubled 200 times), and of rows whose
+squared distances nearly do.
 
-Reference: the FP64 search of the oracle. Both end at the same precision, far beyond the float range, where the tied
-neighbours share the mass and the others have none; a probability is rounded to float once: 2^-24 of itself, 2^-23
-allowed.
+Reference: the FP64 search of the oracle. Both take the same steps; a probability is rounded to float once: 2^-24 of
+itself, 2^-23 allowed.
 """
 import numpy as np
 import pytest
@@ -33,3 +33,19 @@ def test_more_ties_than_the_perplexity(k, ties, perplexity, smallest):
     assert np.isfinite(got["val"]).all() and np.isfinite(got["total_mass"])
     fit = api.tsne_knn(_ring(n, k), dist, perplexity=perplexity, n_iter=5, early_exaggeration_iter=5)
     assert np.isfinite(fit.layout).all()
+
+
+# On both sides of 1e15, from where a row is searched in FP64, and up to 1.8e19, where a float's square overflows (such a
+# row is uniform by the zero-spread test, which is in float as the reference's) and sums of several squares do before.
+# Below the line the exponentials are FP32: an exponent x errs by 3 x 2^-24, which moves a probability p = exp(-x) / sum by
+# less than 0.37 x 3 x 2^-24 of 1.
+@pytest.mark.parametrize("lo,hi", [(2e14, 5e14), (8e14, 2e15), (1e18, 1.8e19)])
+def test_squares_beyond_the_float_range(lo, hi):
+    n, k = 500, 30
+    rng = np.random.default_rng(7)
+    dist = np.sort(rng.uniform(lo, hi, (n, k)), 1).astype(np.float32)
+    got = api.tsne_affinities(_ring(n, k), dist, 10.0, index_offset=0)
+    want, _ = O.row_p_f64(dist, 10.0)
+    fp64 = dist.max(1) > 1.001e15
+    np.testing.assert_allclose(got["p_directed"][fp64], want[fp64], rtol=2.0 ** -23)
+    np.testing.assert_allclose(got["p_directed"][~fp64], want[~fp64], rtol=2.0 ** -22, atol=2.0 ** -23)
