@@ -15,8 +15,8 @@
 // Here every step runs on the GPU: column means; C from exact products in two-float sums (tiles of C x
 // row slices, partials summed in a fixed order in FP64); a cyclic Jacobi eigendecomposition on one
 // block in two-float arithmetic (round-robin ordering: the p/2 disjoint rotations of a step are applied
-// together); scores in two-float; the sign rule; and the reference's scaling. The data are read scaled by
-// the power of two that brings their largest magnitude near 1, so that no product leaves the float range.
+// together); scores in two-float; the sign rule; and the reference's scaling. The centred data
+// are scaled by the power of two that brings their largest magnitude near 1, so that no product leaves the float range.
 #include <algorithm>
 #include <cfloat>
 #include <cmath>
@@ -35,28 +35,31 @@ constexpr int kJacobiSweeps = 30;
 constexpr int kPcaMaxFeatures = 1024;
 constexpr int kJacobiSharedFeatures = 152;  // 152 x 152 two-float values: 185 KB of shared memory
 
-// Exponent of the power of two the data are divided by (`bits`: the largest magnitude's).
+// Exponent of the power of two the centred data are divided by (`bits`: their largest magnitude's).
 __device__ __forceinline__ int data_exponent(int bits) {
   const float top = __int_as_float(bits);
   return top > 0.0f ? min(max(ilogbf(top), -100), 126) : 0;
 }
 
-// part[column][slice] = sum of the slice's rows of the column, status[0] set on a non-finite value,
-// status[1] = bits of the largest magnitude. 200,000 x 50: one FP64 sum per block of a column took 389 us,
+// part[column][slice] = sum of the slice's rows of the column, range[column][slice] = their smallest and largest
+// value, status[0] set on a non-finite value. 200,000 x 50: one FP64 sum per block of a column took 389 us,
 // 19 us now.
 __global__ void __launch_bounds__(256)
-pca_sum_kernel(const float* __restrict__ X, int n, double* __restrict__ part, int* __restrict__ status) {
+pca_sum_kernel(const float* __restrict__ X, int n, double* __restrict__ part, float2* __restrict__ range,
+               int* __restrict__ status) {
   __shared__ double s_sum[8];
+  __shared__ float2 s_range[8];
   const float* col = X + (long long)blockIdx.x * n;
   const int first = blockIdx.y * 256 + threadIdx.x, stride = gridDim.y * 256;
   Float2Sum s{0.0f, 0.0f};
-  float top = 0.0f;
+  float lo = FLT_MAX, hi = -FLT_MAX;
   bool finite = true;
 #pragma unroll 4
   for (int i = first; i < n; i += stride) {
     const float v = col[i];
     finite &= isfinite(v);
-    top = fmaxf(top, fabsf(v));
+    lo = fminf(lo, v);
+    hi = fmaxf(hi, v);
     s = add(s, v);
   }
   double t = value(s);
@@ -65,26 +68,42 @@ pca_sum_kernel(const float* __restrict__ X, int n, double* __restrict__ part, in
     for (int i = first; i < n; i += stride) t += (double)col[i];
   }
   if (!finite) atomicExch(status, 1);
-  const int bits = __reduce_max_sync(0xffffffffu, __float_as_int(top));
   t = warp_sum(t);
+  lo = warp_min(lo);
+  hi = warp_max(hi);
   if ((threadIdx.x & 31) == 0) {
-    if (bits > 0) atomicMax(status + 1, bits);
     s_sum[threadIdx.x >> 5] = t;
+    s_range[threadIdx.x >> 5] = make_float2(lo, hi);
   }
   __syncthreads();
   if (threadIdx.x == 0) {
     t = 0.0;
-    for (int w = 0; w < 8; ++w) t += s_sum[w];
+    for (int w = 0; w < 8; ++w) {
+      t += s_sum[w];
+      lo = fminf(lo, s_range[w].x);
+      hi = fmaxf(hi, s_range[w].y);
+    }
     part[blockIdx.x * gridDim.y + blockIdx.y] = t;
+    range[blockIdx.x * gridDim.y + blockIdx.y] = make_float2(lo, hi);
   }
 }
 
-__global__ void pca_mean_kernel(const double* __restrict__ part, int p, int slices, int n, float* __restrict__ mean) {
+// The columns' means; status[1] = bits of the largest magnitude of the centred data. (Of the data themselves it would
+// be a constant column's: one of 1e23 beside columns of spread 1 would leave these no bits.)
+__global__ void pca_mean_kernel(const double* __restrict__ part, const float2* __restrict__ range, int p, int slices,
+                                int n, float* __restrict__ mean, int* __restrict__ status) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= p) return;
   double t = 0.0;
-  for (int y = 0; y < slices; ++y) t += part[c * slices + y];
-  mean[c] = (float)(t / (double)n);
+  float lo = FLT_MAX, hi = -FLT_MAX;
+  for (int y = 0; y < slices; ++y) {
+    t += part[c * slices + y];
+    lo = fminf(lo, range[c * slices + y].x);
+    hi = fmaxf(hi, range[c * slices + y].y);
+  }
+  const float m = (float)(t / (double)n);
+  mean[c] = m;
+  atomicMax(status + 1, __float_as_int(fmaxf(fabsf(lo - m), fabsf(hi - m))));
 }
 
 // partial[slice][a][b] = sum over the slice's rows of u_a u_b, u = (X - mean) / 2^e, for the block's 16 x 16
@@ -530,12 +549,14 @@ void pca_tsne_start(const float* X, int n, int p, float2* init, cudaStream_t s) 
   const bool shared = p <= kJacobiSharedFeatures;
   double *sums = nullptr, *partial = nullptr, *C = nullptr, *sign = nullptr, *moments = nullptr;
   float *mean = nullptr, *tangents = nullptr;
+  float2* range = nullptr;
   Float2Sum *work = nullptr, *V = nullptr;
   double2* sc = nullptr;
   ArgMax* am = nullptr;
-  int* status = nullptr;  // non-finite data, bits of the largest magnitude
+  int* status = nullptr;  // non-finite data, bits of the largest centred magnitude
   Arena w;
   w.reserve(&sums, (std::size_t)p * mslices);
+  w.reserve(&range, (std::size_t)p * mslices);
   w.reserve(&mean, p);
   w.reserve(&partial, (std::size_t)slices * p * p);
   w.reserve(&C, (std::size_t)p * p);
@@ -549,9 +570,9 @@ void pca_tsne_start(const float* X, int n, int p, float2* init, cudaStream_t s) 
   w.reserve(&moments, 4 * (std::size_t)mblocks);
   w.commit("device PCA initialization");
   FE_CUDA(cudaMemsetAsync(status, 0, 2 * sizeof(int), s));
-  pca_sum_kernel<<<dim3(p, mslices), 256, 0, s>>>(X, n, sums, status);
+  pca_sum_kernel<<<dim3(p, mslices), 256, 0, s>>>(X, n, sums, range, status);
   FE_LAUNCH("pca_sum_kernel");
-  pca_mean_kernel<<<ceil_div(p, 128), 128, 0, s>>>(sums, p, mslices, n, mean);
+  pca_mean_kernel<<<ceil_div(p, 128), 128, 0, s>>>(sums, range, p, mslices, n, mean, status);
   FE_LAUNCH("pca_mean_kernel");
   int h_bad = 0;
   FE_CUDA(cudaMemcpyAsync(&h_bad, status, sizeof(int), cudaMemcpyDeviceToHost, s));
