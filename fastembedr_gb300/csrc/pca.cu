@@ -15,7 +15,7 @@
 // Here every step runs on the GPU: column means; C from exact products in two-float sums (tiles of C x
 // row slices, partials summed in a fixed order in FP64); a cyclic Jacobi eigendecomposition on one
 // block in two-float arithmetic (round-robin ordering: the p/2 disjoint rotations of a step are applied
-// together); scores in two-float; the sign rule; and the reference's scaling. The centred data
+// together) and one FP64 refinement of the two leading eigenvectors; scores in two-float; the sign rule; and the reference's scaling. The centred data
 // are scaled by the power of two that brings their largest magnitude near 1, so that no product leaves the float range.
 #include <algorithm>
 #include <cfloat>
@@ -227,16 +227,15 @@ __device__ __forceinline__ void jacobi_rotate(Float2Sum& x, Float2Sum& y, Float2
   x = u;
 }
 
-// The two leading eigenvectors of the symmetric p x p matrix C by cyclic Jacobi, one block. Only the upper
+// The eigenvalues of the symmetric p x p matrix C by cyclic Jacobi, one block, and the rotations. Only the upper
 // triangle of A is kept (m x m, m = p rounded up to even; in shared memory, or in `work` beyond
 // kJacobiSharedFeatures). Round-robin ordering: step t pairs position 0 with position m - 1 and the others
 // around a circle; a step's m/2 disjoint rotations are applied together, J^T A J as one update of the 2 x 2
-// blocks of (pair, pair). The eigenvectors are the product of all rotations: their tangents are kept
-// (`tangents`, kJacobiSweeps (m - 1) m / 2 floats) and, at the end, applied in reverse to the unit vectors of the
-// two largest eigenvalues, one warp each, instead of carrying all of V along. A tangent is FP32: an
-// angle a little off leaves a little of the entry to the next sweep. Stops when the off-diagonal mass is below
-// 1e-26 of the diagonal mass (entries below 2^-43 of the spectrum), or after kJacobiSweeps sweeps.
-// vectors[c * p + i]: component c.
+// blocks of (pair, pair). The eigenvectors are the product of all rotations, whose tangents are kept
+// (`tangents`, kJacobiSweeps (m - 1) m / 2 floats) for the kernel below, instead of carrying all of V along. A tangent
+// is FP32: an angle a little off leaves a little of the entry to the next sweep. Stops when the off-diagonal mass is
+// below 1e-26 of the diagonal mass (entries below 2^-43 of the spectrum), or after kJacobiSweeps sweeps.
+// lambda: the eigenvalues; info: the indices of the two largest, and the number of steps.
 //
 // p = 50: 1907 us with A and V in FP64 in global memory, 480 us now, bound by the latency of the two
 // dependent phases of a step; the whole start of 5,000 x 150: 90.8 ms, 6.4 now; x 300, with A in global
@@ -244,13 +243,11 @@ __device__ __forceinline__ void jacobi_rotate(Float2Sum& x, Float2Sum& y, Float2
 template <bool kShared>
 __global__ void __launch_bounds__(kJacobiThreads)
 pca_jacobi_kernel(const double* __restrict__ C, int p, Float2Sum* __restrict__ work, float* __restrict__ tangents,
-                  Float2Sum* __restrict__ vectors) {
+                  double* __restrict__ lambda, int* __restrict__ info) {
   extern __shared__ Float2Sum s_a[];
   __shared__ int2 s_pair[kJacobiThreads];
   __shared__ float4 s_rot[kJacobiThreads];  // c, s
-  __shared__ Float2Sum s_vec[2][kPcaMaxFeatures];
   __shared__ float s_red[2][kJacobiThreads / 32];
-  __shared__ int s_order[2];
   __shared__ bool s_done;
   Float2Sum* A = kShared ? s_a : work;
   const int m = p + (p & 1), half = m / 2;
@@ -348,17 +345,28 @@ pca_jacobi_kernel(const double* __restrict__ C, int p, Float2Sum* __restrict__ w
       if (above(i, b0)) b0 = i;
     for (int i = 0; i < p; ++i)
       if (i != b0 && (b1 < 0 || above(i, b1))) b1 = i;
-    s_order[0] = b0;
-    s_order[1] = b1;
+    info[0] = b0;
+    info[1] = b1;
+    info[2] = steps;
   }
-  __syncthreads();
+  for (int i = threadIdx.x; i < p; i += blockDim.x) lambda[i] = value(A[i * m + i]) / unit;
+}
+
+// All eigenvectors, vectors[v * p + i]: the rotations applied in reverse to the unit vectors, a warp for each of a
+// block's two. x <- J x for each step's J, (x_i, x_j) <- (c x_i + s x_j, -s x_i + c x_j); the block computes the
+// rotations of as many steps as it has threads for.
+__global__ void __launch_bounds__(kJacobiThreads)
+pca_vectors_kernel(const float* __restrict__ tangents, int p, const int* __restrict__ info,
+                   Float2Sum* __restrict__ vectors) {
+  __shared__ int2 s_pair[kJacobiThreads];
+  __shared__ float4 s_rot[kJacobiThreads];
+  __shared__ Float2Sum s_vec[2][kPcaMaxFeatures];
+  const int m = p + (p & 1), half = m / 2, first = 2 * (int)blockIdx.x;
   const int comp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (comp < 2)
-    for (int i = lane; i < m; i += 32) s_vec[comp][i] = Float2Sum{i == s_order[comp] ? 1.0f : 0.0f, 0.0f};
-  // x <- J x for each step's J, (x_i, x_j) <- (c x_i + s x_j, -s x_i + c x_j); the block computes the
-  // rotations of as many steps as it has threads for, two warps apply them
+    for (int i = lane; i < m; i += 32) s_vec[comp][i] = Float2Sum{i == first + comp ? 1.0f : 0.0f, 0.0f};
   const int batch = kJacobiThreads / half;
-  for (int last = steps; last > 0; last -= batch) {
+  for (int last = info[2]; last > 0; last -= batch) {
     const int count = min(batch, last), g = threadIdx.x / half, k = threadIdx.x - g * half;
     if (g < count) {
       const int done = last - 1 - g;
@@ -383,7 +391,73 @@ pca_jacobi_kernel(const double* __restrict__ C, int p, Float2Sum* __restrict__ w
     }
     __syncthreads();
   }
-  for (int i = threadIdx.x; i < 2 * p; i += blockDim.x) vectors[i] = s_vec[i / p][i % p];
+  for (int i = threadIdx.x; i < 2 * p; i += blockDim.x) {
+    const int v = i / p;
+    if (first + v < p) vectors[(long long)(first + v) * p + i % p] = s_vec[v][i % p];
+  }
+}
+
+// One step of Ogita and Aishima's refinement (2018) for the two leading eigenvectors x_c: with S = X^T C X and
+// R = I - X^T X in FP64, x_c gains sum over i of e_ic x_i, e_ic = (S_ic + lambda_c R_ic) / (lambda_c - lambda_i), or
+// R_ic / 2 for an eigenvalue that cannot be told from lambda_c. It squares the error, which in two floats is some 1e-13
+// over the gap of the eigenvalues: with a gap of 1e-7 of the largest, a start of 151 features was off by 5e-7 of its
+// largest coordinate, 7e-8 now (6e-8 is the rounding to float).
+// y[c * p + r] = (C x_c)_r, a warp per r.
+__global__ void __launch_bounds__(256)
+pca_product_kernel(const double* __restrict__ C, const Float2Sum* __restrict__ X, int p, const int* __restrict__ info,
+                   double* __restrict__ y) {
+  const int r = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (r >= p) return;
+  for (int c = 0; c < 2; ++c) {
+    const Float2Sum* x = X + (long long)info[c] * p;
+    double t = 0.0;
+    for (int i = lane; i < p; i += 32) t += C[(long long)r * p + i] * value(x[i]);
+    t = warp_sum(t);
+    if (lane == 0) y[c * p + r] = t;
+  }
+}
+// e[c * p + i] = e_ic, a warp per i.
+__global__ void __launch_bounds__(256)
+pca_correction_kernel(const Float2Sum* __restrict__ X, const double* __restrict__ y, int p,
+                      const double* __restrict__ lambda, const int* __restrict__ info, double* __restrict__ e) {
+  const int i = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (i >= p) return;
+  const Float2Sum* x = X + (long long)i * p;
+  for (int c = 0; c < 2; ++c) {
+    const Float2Sum* xc = X + (long long)info[c] * p;
+    double s = 0.0, r = 0.0;
+    for (int j = lane; j < p; j += 32) {
+      const double v = value(x[j]);
+      s += v * y[c * p + j];
+      r += v * value(xc[j]);
+    }
+    s = warp_sum(s);
+    r = (i == info[c] ? 1.0 : 0.0) - warp_sum(r);
+    const double gap = lambda[info[c]] - lambda[i];
+    if (lane == 0)
+      e[c * p + i] = fabs(gap) > 1e-12 * fabs(lambda[info[0]]) ? (s + lambda[info[c]] * r) / gap : 0.5 * r;
+  }
+}
+// vectors[c * p + i] = component c; block: 32 coordinates, eight warps share the sum.
+__global__ void __launch_bounds__(256)
+pca_refine_kernel(const Float2Sum* __restrict__ X, const double* __restrict__ e, int p, const int* __restrict__ info,
+                  Float2Sum* __restrict__ vectors) {
+  __shared__ double s_sum[8][2][32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, i = blockIdx.x * 32 + lane;
+  double t[2] = {0.0, 0.0};
+  if (i < p)
+    for (int j = warp; j < p; j += 8) {
+      const double v = value(X[(long long)j * p + i]);
+      t[0] += e[j] * v;
+      t[1] += e[p + j] * v;
+    }
+  s_sum[warp][0][lane] = t[0];
+  s_sum[warp][1][lane] = t[1];
+  __syncthreads();
+  if (warp >= 2 || i >= p) return;
+  double sum = 0.0;
+  for (int w = 0; w < 8; ++w) sum += s_sum[w][warp][lane];
+  vectors[warp * p + i] = split(value(X[(long long)info[warp] * p + i]) + sum);
 }
 
 struct ArgMax {
@@ -548,11 +622,13 @@ void pca_tsne_start(const float* X, int n, int p, float2* init, cudaStream_t s) 
   const std::size_t m = p + (p & 1);
   const bool shared = p <= kJacobiSharedFeatures;
   double *sums = nullptr, *partial = nullptr, *C = nullptr, *sign = nullptr, *moments = nullptr;
+  double *lambda = nullptr, *y = nullptr, *e = nullptr;
   float *mean = nullptr, *tangents = nullptr;
   float2* range = nullptr;
-  Float2Sum *work = nullptr, *V = nullptr;
+  Float2Sum *work = nullptr, *all = nullptr, *V = nullptr;
   double2* sc = nullptr;
   ArgMax* am = nullptr;
+  int* info = nullptr;
   int* status = nullptr;  // non-finite data, bits of the largest centred magnitude
   Arena w;
   w.reserve(&sums, (std::size_t)p * mslices);
@@ -562,6 +638,11 @@ void pca_tsne_start(const float* X, int n, int p, float2* init, cudaStream_t s) 
   w.reserve(&C, (std::size_t)p * p);
   w.reserve(&work, shared ? 1 : m * m);
   w.reserve(&tangents, kJacobiSweeps * (m - 1) * (m / 2));
+  w.reserve(&lambda, p);
+  w.reserve(&info, 3);
+  w.reserve(&all, (std::size_t)p * p);
+  w.reserve(&y, 2 * (std::size_t)p);
+  w.reserve(&e, 2 * (std::size_t)p);
   w.reserve(&V, 2 * (std::size_t)p);
   w.reserve(&sc, n);
   w.reserve(&am, 2 * (std::size_t)sblocks);
@@ -586,11 +667,19 @@ void pca_tsne_start(const float* X, int n, int p, float2* init, cudaStream_t s) 
   if (shared) {
     const int smem = (int)(m * m * sizeof(Float2Sum));
     FE_CUDA(cudaFuncSetAttribute(pca_jacobi_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    pca_jacobi_kernel<true><<<1, kJacobiThreads, smem, s>>>(C, p, work, tangents, V);
+    pca_jacobi_kernel<true><<<1, kJacobiThreads, smem, s>>>(C, p, work, tangents, lambda, info);
   } else {
-    pca_jacobi_kernel<false><<<1, kJacobiThreads, 0, s>>>(C, p, work, tangents, V);
+    pca_jacobi_kernel<false><<<1, kJacobiThreads, 0, s>>>(C, p, work, tangents, lambda, info);
   }
   FE_LAUNCH("pca_jacobi_kernel");
+  pca_vectors_kernel<<<ceil_div(p, 2), kJacobiThreads, 0, s>>>(tangents, p, info, all);
+  FE_LAUNCH("pca_vectors_kernel");
+  pca_product_kernel<<<ceil_div(p, 8), 256, 0, s>>>(C, all, p, info, y);
+  FE_LAUNCH("pca_product_kernel");
+  pca_correction_kernel<<<ceil_div(p, 8), 256, 0, s>>>(all, y, p, lambda, info, e);
+  FE_LAUNCH("pca_correction_kernel");
+  pca_refine_kernel<<<ceil_div(p, 32), 256, 0, s>>>(all, e, p, info, V);
+  FE_LAUNCH("pca_refine_kernel");
   pca_scores_kernel<<<sblocks, 256, 0, s>>>(X, mean, status, n, p, V, sc, am);
   FE_LAUNCH("pca_scores_kernel");
   pca_sign_kernel<<<1, 64, 0, s>>>(sc, am, sblocks, sign);
