@@ -135,6 +135,15 @@ int sm_count() {
   return sms;
 }
 
+void allow_dynamic_shared(const void* kernel) {
+  int dev = 0, most = 0;
+  FE_CUDA(cudaGetDevice(&dev));
+  FE_CUDA(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+  cudaFuncAttributes a{};
+  FE_CUDA(cudaFuncGetAttributes(&a, kernel));
+  FE_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)a.sharedSizeBytes));
+}
+
 }  // namespace fe
 
 void fe::order_after_legacy_stream(cudaStream_t s) {
