@@ -72,6 +72,7 @@ SIGNATURES = {
     "fastembedr_tsne_plan_kl": (I, [vp, C.POINTER(D)]),
     "fastembedr_cuda_umap_spectral_init_from_knn": (I, [vp, vp, I, I, I, I, D, I, vp]),
     "fastembedr_cuda_umap_spectral_init_csr": (I, [vp, vp, vp, I, I, D, I, vp]),
+    "fastembedr_cuda_umap_spectral_init_csr_blocks": (I, [vp, vp, vp, I, I, D, I, I, vp]),
     "fastembedr_cuda_umap_knn_spectral": (I, [vp, vp, I, I, I, I, I, F, F, F, I, D, U, vp]),
     "fastembedr_umap_find_ab_params": (None, [D, D, C.POINTER(D), C.POINTER(D)]),
     "fastembedr_cuda_umap_find_ab_params": (I, [D, D, C.POINTER(D), C.POINTER(D)]),

@@ -1707,6 +1707,13 @@ int fastembedr_cuda_umap_spectral_init_from_knn(const int* indices, const float*
 
 int fastembedr_cuda_umap_spectral_init_csr(const int* offsets, const int* neighbors, const float* weights, int n,
                                            int spectral_n_iter, double init_scale, int seed, double* out) {
+  return fastembedr_cuda_umap_spectral_init_csr_blocks(offsets, neighbors, weights, n, spectral_n_iter, init_scale, seed,
+                                                       0, out);
+}
+
+int fastembedr_cuda_umap_spectral_init_csr_blocks(const int* offsets, const int* neighbors, const float* weights, int n,
+                                                  int spectral_n_iter, double init_scale, int seed, int max_blocks,
+                                                  double* out) {
   return fe::guarded([&] {
     if (!offsets || !neighbors || !weights || !out) throw fe::Error("null host pointer");
     if (n < 1 || spectral_n_iter < 1) throw fe::Error("invalid spectral initialization parameters");
@@ -1759,7 +1766,7 @@ int fastembedr_cuda_umap_spectral_init_csr(const int* offsets, const int* neighb
       fe::upload(d_nb, nb0.data(), sizeof(int) * nnz, s);
       fe::upload(d_w, weights, sizeof(float) * nnz, s);
     }
-    fe::umap_spectral_start(d_off, d_nb, d_w, n, nnz, spectral_n_iter, init_scale, seed, d_out, s);
+    fe::umap_spectral_start(d_off, d_nb, d_w, n, nnz, spectral_n_iter, init_scale, seed, d_out, s, nullptr, max_blocks);
     FE_CUDA(cudaMemcpyAsync(out, d_out, sizeof(double) * 2 * (std::size_t)n, cudaMemcpyDeviceToHost, s));
     FE_CUDA(cudaStreamSynchronize(s));
   });

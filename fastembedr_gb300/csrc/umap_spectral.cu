@@ -127,7 +127,7 @@ __global__ void sp_normalise_trivial_kernel(double* __restrict__ triv, int n, co
 // multiplies them and keeps their B values in shared memory through the pass (as long as kSpSharedRows hold
 // them; in the global buffers beyond). Blocks exchange sums without a barrier: a partial is published with the
 // exchange's number in the same words, and whoever needs the sum polls for all partials and adds them in
-// block order. `points` and `nparts` follow from n alone, so the sums do not depend on the launch.
+// block order. `points` and `nparts` follow from n and the number of SMs, so the sums do not depend on the launch.
 // Columns written during the launch are read through L2 (__ldcg): another block may have written them, and L1
 // is not coherent.
 //
@@ -144,12 +144,12 @@ __global__ void sp_normalise_trivial_kernel(double* __restrict__ triv, int n, co
 
 constexpr long long kSpWaitCycles = 4000000000LL;  // about 2 s at the SM clock
 constexpr int kSpRoundThreads = 512;
-constexpr int kSpParts = 152;         // blocks, at most (one per SM)
+constexpr int kSpParts = 152;         // blocks, at most (one per SM, or as many as there are SMs)
 constexpr int kSpSharedRows = 3456;   // rows of a block in shared memory: 64 bytes each, 216 KB
 
-// Tiles of a block and rows per tile: every SM has its share, of a warp's width at least.
-int sp_tiles(int n) { return ceil_div(n, kSpParts * kSpRoundThreads); }
-int sp_points(int n) { return std::max(32, ceil_div(n, kSpParts * sp_tiles(n))); }
+// Tiles of a block and rows per tile for at most `blocks` blocks: each has its share, of a warp's width at least.
+int sp_tiles(int n, int blocks) { return ceil_div(n, (long long)blocks * kSpRoundThreads); }
+int sp_points(int n, int blocks) { return std::max(32, ceil_div(n, (long long)blocks * sp_tiles(n, blocks))); }
 
 struct SpGrid {
   int error;   // 1: a wait gave up
@@ -913,7 +913,7 @@ SpectralDraws spectral_draws(int n, int seed, int device, bool on_host) {
 
 void umap_spectral_start(const int* offsets, const int* neighbors, const float* weights, int n, long long nnz,
                          int spectral_n_iter, double init_scale, int seed, double* out, cudaStream_t s,
-                         SpectralDraws* pre) {
+                         SpectralDraws* pre, int max_blocks) {
   if (n < 1 || spectral_n_iter < 1) throw Error("invalid spectral initialization parameters");
   std::mt19937 rng((std::uint32_t)seed);
   std::uniform_real_distribution<double> uniform(-10.0, 10.0);
@@ -976,10 +976,11 @@ void umap_spectral_start(const int* offsets, const int* neighbors, const float* 
     // The subspace iteration as cooperative launches: the initial orthonormalisation (round -1) and
     // spectral_n_iter rounds. A launch that stops at a vanished column is resumed from it after the host redraws
     // the column from the stream, as the reference redraws and repeats it.
-    int points = sp_points(n);
-    const int parts = ceil_div(n, points * sp_tiles(n));
-    int tiles = sp_tiles(n);
-    const bool shared = tiles * points <= kSpSharedRows;
+    int blocks = std::min(kSpParts, sm_count());
+    if (max_blocks > 0) blocks = std::min(blocks, max_blocks);
+    int points = sp_points(n, blocks), tiles = sp_tiles(n, blocks);
+    const int parts = ceil_div(n, (long long)points * tiles);
+    const bool shared = (long long)tiles * points <= kSpSharedRows;
     const int smem = shared ? kSpBlock * tiles * points * (int)sizeof(double) : 0;
     const void* rounds = shared ? (const void*)sp_rounds_kernel<true> : (const void*)sp_rounds_kernel<false>;
     allow_dynamic_shared(rounds);

@@ -38,9 +38,10 @@ SpectralDraws spectral_draws(int n, int seed, int device, bool on_host = false);
 // ascending per row, no self entries, w_ij == w_ji) into out: device, column-major n x 2 doubles.
 // spectral_n_iter rounds, seed for the std::mt19937 stream of the reference, init_scale > 0
 // rescales every column to that standard deviation (NaN: no rescaling). Synchronises s.
-// `pre` (may be null): the draws of spectral_draws(n, seed), made ahead.
+// `pre` (may be null): the draws of spectral_draws(n, seed), made ahead. max_blocks > 0: no more blocks in the rounds
+// than that (otherwise one per SM).
 void umap_spectral_start(const int* offsets, const int* neighbors, const float* weights, int n, long long nnz,
                          int spectral_n_iter, double init_scale, int seed, double* out, cudaStream_t s,
-                         SpectralDraws* pre = nullptr);
+                         SpectralDraws* pre = nullptr, int max_blocks = 0);
 
 }  // namespace fe

@@ -146,6 +146,11 @@ int fastembedr_cuda_umap_spectral_init_from_knn(const int* indices, const float*
  * is). out: host, column-major n x 2 doubles. */
 int fastembedr_cuda_umap_spectral_init_csr(const int* offsets, const int* neighbors, const float* weights, int n,
                                            int spectral_n_iter, double init_scale, int seed, double* out);
+/* The same with at most max_blocks blocks in the subspace iteration (0: one per SM), as on a device, or a share of one,
+ * with that many SMs: the sums over points are split differently. */
+int fastembedr_cuda_umap_spectral_init_csr_blocks(const int* offsets, const int* neighbors, const float* weights, int n,
+                                                  int spectral_n_iter, double init_scale, int seed, int max_blocks,
+                                                  double* out);
 /* No reference counterpart: umap_knn(backend = "cuda") with the start above computed on the GPU
  * instead of the CPU (R/umap_core_helpers.R:205-243 then fastembedr_cuda_umap_optimize_coo): KNN ->
  * fuzzy graph -> spectral start -> n_epochs SGD epochs (min_dist through find_ab_params), one
