@@ -7,6 +7,7 @@
 // and the call 5.0 -> 4.1 ms.
 #include <climits>
 
+#include "../../include/fastembedr_cuda.h"
 #include "mt_normal.cuh"
 
 namespace fe {
@@ -64,11 +65,16 @@ __device__ __forceinline__ double canonical(std::uint32_t lo, std::uint32_t hi) 
   return r >= 1.0 ? 0.99999999999999988897769753748 : r;
 }
 
-__device__ __forceinline__ PolarPoint polar_point(uint4 w) {
+// The square of the radius is rounded as the host rounds it, or a point next to the unit circle could be accepted by one
+// and not by the other, which would shift every later draw, and its logarithm, of 1 - r2, would be off by far more than r2.
+using Radius = NormalStream::Radius;
+__device__ __forceinline__ PolarPoint polar_point(uint4 w, Radius radius) {
   PolarPoint p;
   p.x = 2.0 * canonical(w.x, w.y) - 1.0;
   p.y = 2.0 * canonical(w.z, w.w) - 1.0;
-  p.r2 = p.x * p.x + p.y * p.y;
+  const double xx = __dmul_rn(p.x, p.x), yy = __dmul_rn(p.y, p.y);
+  p.r2 = radius == Radius::kFusedX ? __fma_rn(p.x, p.x, yy)
+                                   : radius == Radius::kFusedY ? __fma_rn(p.y, p.y, xx) : __dadd_rn(xx, yy);
   p.accepted = p.r2 <= 1.0 && p.r2 != 0.0;
   return p;
 }
@@ -96,19 +102,19 @@ __device__ __forceinline__ int block_prefix(int v, int& total) {
 }
 
 __global__ void __launch_bounds__(kPointThreads)
-polar_count_kernel(const uint4* __restrict__ words, int candidates, int* __restrict__ counts) {
+polar_count_kernel(const uint4* __restrict__ words, int candidates, Radius radius, int* __restrict__ counts) {
   const int first = blockIdx.x * kPerBlock + threadIdx.x * kPerThread;
   int mine = 0;
   for (int u = 0; u < kPerThread; ++u)
-    if (first + u < candidates) mine += polar_point(words[first + u]).accepted;
+    if (first + u < candidates) mine += polar_point(words[first + u], radius).accepted;
   int total = 0;
   block_prefix(mine, total);
   if (threadIdx.x == 0) counts[blockIdx.x] = total;
 }
 
 __global__ void __launch_bounds__(kPointThreads)
-polar_fill_kernel(const uint4* __restrict__ words, int candidates, const int* __restrict__ counts, long long pairs,
-                  double sd, double scale, double2* __restrict__ out, int* __restrict__ enough) {
+polar_fill_kernel(const uint4* __restrict__ words, int candidates, Radius radius, const int* __restrict__ counts,
+                  long long pairs, double sd, double scale, double2* __restrict__ out, int* __restrict__ enough) {
   int before = 0, unused = 0;
   for (int b = threadIdx.x; b < (int)blockIdx.x; b += kPointThreads) before += counts[b];
   block_prefix(before, before);
@@ -118,7 +124,7 @@ polar_fill_kernel(const uint4* __restrict__ words, int candidates, const int* __
 #pragma unroll
   for (int u = 0; u < kPerThread; ++u) {
     p[u].accepted = false;
-    if (first + u < candidates) p[u] = polar_point(words[first + u]);
+    if (first + u < candidates) p[u] = polar_point(words[first + u], radius);
     mine += p[u].accepted;
   }
   long long at = before + block_prefix(mine, unused);
@@ -135,10 +141,12 @@ polar_fill_kernel(const uint4* __restrict__ words, int candidates, const int* __
 
 }  // namespace
 
-MtNormalBlock::MtNormalBlock(std::uint32_t seed, std::size_t count, double sd, double scale) : count_(count) {
+MtNormalBlock::MtNormalBlock(std::uint32_t seed, std::size_t count, double sd, double scale, long long max_points)
+    : count_(count) {
   const long long pairs = (long long)(count / 2);
   // pi / 4 of the points are accepted, with a standard deviation of half the root of their number: 2% and 4,096 more
-  const long long points = (long long)((double)pairs * 1.2733 * 1.02) + 4096;
+  const long long enough = (long long)((double)pairs * 1.2733 * 1.02) + 4096;
+  const long long points = max_points > 0 ? std::min(enough, max_points) : enough;
   const long long states = (points * 4 + kState - 1) / kState;
   if (states * (kState / 4) > INT_MAX / 2) throw Error("too many draws for one block");
   const int candidates = (int)(states * (kState / 4)), blocks = ceil_div(candidates, kPerBlock);
@@ -154,9 +162,10 @@ MtNormalBlock::MtNormalBlock(std::uint32_t seed, std::size_t count, double sd, d
   mt_words_kernel<<<1, kWordThreads, 0, s>>>(seed, (int)states, words);
   FE_LAUNCH("mt_words_kernel");
   const uint4* quads = reinterpret_cast<const uint4*>(words);
-  polar_count_kernel<<<blocks, kPointThreads, 0, s>>>(quads, candidates, counts);
+  const Radius radius = NormalStream::radius_rounding();
+  polar_count_kernel<<<blocks, kPointThreads, 0, s>>>(quads, candidates, radius, counts);
   FE_LAUNCH("polar_count_kernel");
-  polar_fill_kernel<<<blocks, kPointThreads, 0, s>>>(quads, candidates, counts, pairs, sd, scale,
+  polar_fill_kernel<<<blocks, kPointThreads, 0, s>>>(quads, candidates, radius, counts, pairs, sd, scale,
                                                      reinterpret_cast<double2*>(out_), enough_);
   FE_LAUNCH("polar_fill_kernel");
 }
@@ -173,3 +182,23 @@ bool MtNormalBlock::copy_to(double* dst, cudaStream_t s) {
 }
 
 }  // namespace fe
+
+extern "C" int fastembedr_cuda_normal_draws(unsigned int seed, long long count, long long max_points, double* device,
+                                            double* host, int* enough) {
+  return fe::guarded([&] {
+    if (!device || !host || !enough) throw fe::Error("null output of the normal draws");
+    if (count < 2 || count % 2 != 0) throw fe::Error("the normal draws come in pairs");
+    std::mt19937 rng(seed);
+    fe::NormalStream stream(0.0, 1e-4);
+    stream.fill(rng, host, (std::size_t)count, 10000.0);
+    fe::Stream st;
+    fe::Arena a;
+    double* d = nullptr;
+    a.reserve(&d, (std::size_t)count);
+    a.commit("normal draws");
+    fe::MtNormalBlock block(seed, (std::size_t)count, 1e-4, 10000.0, max_points);
+    *enough = block.copy_to(d, st.s) ? 1 : 0;
+    if (*enough) FE_CUDA(cudaMemcpyAsync(device, d, sizeof(double) * count, cudaMemcpyDeviceToHost, st.s));
+    FE_CUDA(cudaStreamSynchronize(st.s));
+  });
+}

@@ -5,16 +5,18 @@
 #include <cstdint>
 
 #include "common.cuh"
+#include "normal_stream.cuh"
 
 namespace fe {
 
 // out[i] = scale * draw i of N(0, sd) from a freshly seeded std::mt19937, in the order of
 // std::normal_distribution (Marsaglia's polar method; see normal_stream.cuh), for an even count. The words and the
-// accepted points are those of the host stream; logarithm and root are CUDA's (within a unit in the last place of the
-// host's). *enough is set to 1 when the words sufficed (they do but for one seed in far more than 10^9).
+// accepted points are those of the host stream (NormalStream::radius_rounding() must be known); the logarithm is CUDA's
+// (within a unit in the last place). *enough is set to 1 when the words sufficed (they do but for one seed in far more than 10^9).
 class MtNormalBlock {
  public:
-  MtNormalBlock(std::uint32_t seed, std::size_t count, double sd, double scale);
+  // max_points > 0: words for no more candidate points than that (a test of the case that they do not suffice)
+  MtNormalBlock(std::uint32_t seed, std::size_t count, double sd, double scale, long long max_points = 0);
   ~MtNormalBlock();
   // Copies the draws to dst on stream s, after them; false when the words did not suffice.
   bool copy_to(double* dst, cudaStream_t s);

@@ -131,6 +131,22 @@ bool NormalStream::polar_path() {
   return ok;
 }
 
+NormalStream::Radius NormalStream::radius_rounding() {
+  static const Radius form = [] {
+    std::mt19937 g(1u);
+    bool plain = true, fused_x = true, fused_y = true;
+    for (int i = 0; i < 4096; ++i) {
+      const PolarPoint p = polar_point(g);
+      const volatile double xx = p.x * p.x, yy = p.y * p.y;
+      plain = plain && p.r2 == xx + yy;
+      fused_x = fused_x && p.r2 == std::fma(p.x, p.x, yy);
+      fused_y = fused_y && p.r2 == std::fma(p.y, p.y, xx);
+    }
+    return plain ? Radius::kPlain : fused_x ? Radius::kFusedX : fused_y ? Radius::kFusedY : Radius::kOther;
+  }();
+  return form;
+}
+
 double NormalStream::next(std::mt19937& g) { return polar_path() ? next_polar(g) : std_(g); }
 
 void NormalStream::fill(std::mt19937& g, double* out, std::size_t count, double scale) {

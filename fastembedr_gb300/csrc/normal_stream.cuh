@@ -25,6 +25,9 @@ class NormalStream {
   static void skip(std::mt19937& g, std::size_t pairs);
   // whether the polar path reproduces std::normal_distribution here (and is used)
   static bool polar_path();
+  // How the host's compiler rounds the polar method's x^2 + y^2 (it may fuse a product into the sum).
+  enum class Radius { kPlain, kFusedX, kFusedY, kOther };
+  static Radius radius_rounding();
 
  private:
   double next_polar(std::mt19937& g);

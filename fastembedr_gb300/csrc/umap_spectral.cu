@@ -893,7 +893,8 @@ SpectralDraws spectral_draws(int n, int seed, int device, bool on_host) {
   const std::size_t count = (std::size_t)n * B;
   std::mt19937 rng((std::uint32_t)seed);
   // (an odd count leaves a value in the host stream; a polar path that is not the library's has no twin)
-  const bool on_device = !on_host && n >= kSpectralDeviceDraws && count % 2 == 0 && NormalStream::polar_path();
+  const bool on_device = !on_host && n >= kSpectralDeviceDraws && count % 2 == 0 && NormalStream::polar_path() &&
+                         NormalStream::radius_rounding() != NormalStream::Radius::kOther;
   if (on_device) {
     FE_CUDA(cudaSetDevice(device));
     d.device = std::make_shared<MtNormalBlock>((std::uint32_t)seed, count, 1e-4, 10000.0);

@@ -177,6 +177,11 @@ int fastembedr_cuda_umap_find_ab_params(double spread, double min_dist, double* 
  * this platform (checked once at first use), 0 when the start falls back to drawing through
  * std::normal_distribution itself. Either way the draws equal the reference's. */
 int fastembedr_host_normal_stream_check(void);
+/* No reference counterpart (diagnostic): the first `count` (even) draws of a spectral start's block, normal(0, 1e-4) x 1e4
+ * from std::mt19937(seed), made on the GPU and by the host's stream. max_points > 0 limits the GPU's candidate points;
+ * *enough is 0, and device is not written, when they did not suffice. */
+int fastembedr_cuda_normal_draws(unsigned int seed, long long count, long long max_points, double* device, double* host,
+                                 int* enough);
 
 /* replaces fastembedr_cuda_spectral_init_from_knn, src/embedding_cuda_kernels.cpp:4801-4960
  * (bound by spectral_knn_init_cuda_impl, src/embedding_cuda_impl.cpp:1589-1628): the diffusion
