@@ -18,6 +18,8 @@ class MtNormalBlock {
   // max_points > 0: words for no more candidate points than that (a test of the case that they do not suffice)
   MtNormalBlock(std::uint32_t seed, std::size_t count, double sd, double scale, long long max_points = 0);
   ~MtNormalBlock();
+  // whether a block of that many draws can be made: its candidate points are numbered by an int
+  static bool fits(std::size_t count) { return count / 2 <= (std::size_t)800000000; }
   // Copies the draws to dst on stream s, after them; false when the words did not suffice.
   bool copy_to(double* dst, cudaStream_t s);
 

@@ -893,16 +893,21 @@ SpectralDraws spectral_draws(int n, int seed, int device, bool on_host) {
   const std::size_t count = (std::size_t)n * B;
   std::mt19937 rng((std::uint32_t)seed);
   // (an odd count leaves a value in the host stream; a polar path that is not the library's has no twin)
-  const bool on_device = !on_host && n >= kSpectralDeviceDraws && count % 2 == 0 && NormalStream::polar_path() &&
-                         NormalStream::radius_rounding() != NormalStream::Radius::kOther;
+  const bool on_device = !on_host && n >= kSpectralDeviceDraws && count % 2 == 0 && MtNormalBlock::fits(count) &&
+                         NormalStream::polar_path() && NormalStream::radius_rounding() != NormalStream::Radius::kOther;
   if (on_device) {
     FE_CUDA(cudaSetDevice(device));
-    d.device = std::make_shared<MtNormalBlock>((std::uint32_t)seed, count, 1e-4, 10000.0);
-  } else {
+    try {
+      d.device = std::make_shared<MtNormalBlock>((std::uint32_t)seed, count, 1e-4, 10000.0);
+    } catch (const Error&) {
+      cudaGetLastError();  // no memory for the words: drawn on the host, which needs none
+    }
+  }
+  if (!d.device) {
     d.block.resize(count);
     d.normal.fill(rng, d.block.data(), count, 10000.0);
   }
-  d.tail = std::async(std::launch::async, [rng, n, skip = on_device ? count / 2 : 0]() mutable {
+  d.tail = std::async(std::launch::async, [rng, n, skip = d.device ? count / 2 : 0]() mutable {
              NormalStream::skip(rng, skip);
              SpectralTail t{rng, std::vector<double>(2 * (std::size_t)n)};
              NormalStream jitter(0.0, 1e-4);
