@@ -51,10 +51,19 @@ __global__ void umap_distance_sum_kernel(const float* __restrict__ dist, long lo
     }
   }
   f = warp_sum(f);
+  double s = value(f);
+  if (__any_sync(0xffffffffu, !isfinite(f.hi))) {  // finite distances whose sum leaves the float range
+    s = 0.0;
+    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
+      const float d = dist[t];
+      if (isfinite(d) && d >= 0.0f) s += (double)d;
+    }
+    s = warp_sum(s);
+  }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
   if ((threadIdx.x & 31) == 0) {
-    atomicAdd(acc, value(f));
+    atomicAdd(acc, s);
     atomicAdd(reinterpret_cast<unsigned long long*>(acc + 1), c);
   }
 }
@@ -204,6 +213,12 @@ umap_smooth_knn_kernel(const float* __restrict__ dist, int n, int k, double targ
   double mean = 0.0;
   if (rho > 0.0f && row_count > 0) {
     mean = value(divide(row_sum, Float2Sum{(float)row_count, 0.0f}));
+    if (!isfinite(row_sum.hi)) {  // finite distances whose sum leaves the float range
+      double sum = 0.0;
+      for (int j = 0; j < k; ++j)
+        if (isfinite(d[j]) && d[j] >= 0.0f) sum += (double)d[j];
+      mean = sum / (double)row_count;
+    }
   } else {
     const unsigned long long cnt = reinterpret_cast<const unsigned long long*>(acc)[1];
     mean = cnt > 0 ? acc[0] / (double)cnt : 1.0;
