@@ -468,12 +468,13 @@ __device__ __forceinline__ void ld_stream(const int* pc, const float* pv, int (&
 }
 
 // Lane partials of row [b, e) of the point yi in slot s. Entries of a round outside the row count as
-// the point s itself with value 0, whose term is exactly zero.
+// the point s itself with value 0, whose term is exactly zero. (Positions are unsigned: the round after a row that ends
+// near 2^31 begins beyond it.)
 __device__ __forceinline__ float2 attr_row(const int* __restrict__ col, const float* __restrict__ val,
-                                           const float2* __restrict__ y, int b, int e, int s, float2 yi, int lane) {
+                                           const float2* __restrict__ y, unsigned b, unsigned e, int s, float2 yi, int lane) {
   float ax = 0.0f, ay = 0.0f, kx = 0.0f, ky = 0.0f;
-  for (int c0 = b & ~3; c0 < e; c0 += 128) {
-    const int p = c0 + 4 * lane;
+  for (unsigned c0 = b & ~3u; c0 < e; c0 += 128u) {
+    const unsigned p = c0 + 4u * lane;
     int c[4] = {s, s, s, s};
     float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
     if (p < e) ld_stream(col + p, val + p, c, v);
@@ -849,7 +850,8 @@ __global__ void scatter_points_kernel(const float2* __restrict__ scratch, const 
 // entries each. 1M points x 90 neighbours (115M entries): 575 -> 326 us (540 the first time, out of the caller's
 // order), of 135 for moving the columns once. Shares of some 70 rows even out the row lengths: with 8 blocks
 // per SM the pass took 425 us, a third of it waiting for the longest shares.
-__device__ __forceinline__ int4 relabel_load(const int* __restrict__ col, int2 se, int i) {
+// (positions are unsigned, as in attr_row)
+__device__ __forceinline__ int4 relabel_load(const int* __restrict__ col, uint2 se, unsigned i) {
   int4 v = make_int4(0, 0, 0, 0);
   if (i >= se.x && i + 4 <= se.y) return __ldcs(reinterpret_cast<const int4*>(col + i));
   if (i >= se.x && i < se.y) v.x = col[i];
@@ -858,7 +860,7 @@ __device__ __forceinline__ int4 relabel_load(const int* __restrict__ col, int2 s
   if (i + 3 >= se.x && i + 3 < se.y) v.w = col[i + 3];
   return v;
 }
-__device__ __forceinline__ void relabel_store(int* __restrict__ col, int2 se, int i, int4 v) {
+__device__ __forceinline__ void relabel_store(int* __restrict__ col, uint2 se, unsigned i, int4 v) {
   if (i >= se.x && i + 4 <= se.y) {
     __stcs(reinterpret_cast<int4*>(col + i), v);
     return;
@@ -873,11 +875,14 @@ relabel_rows_kernel(int* __restrict__ col, const int2* __restrict__ slot_rows, i
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int per = (n + (int)gridDim.x - 1) / (int)gridDim.x;
   const int first = (int)blockIdx.x * per, last = min(n, first + per);
-  auto bounds = [&](int r) { return r < last ? slot_rows[r] : make_int2(0, 0); };
-  int2 a = bounds(first + warp), b = bounds(first + warp + 8);
+  auto bounds = [&](int r) {
+    const int2 se = r < last ? slot_rows[r] : make_int2(0, 0);
+    return make_uint2(se.x, se.y);
+  };
+  uint2 a = bounds(first + warp), b = bounds(first + warp + 8);
   for (int r = first + warp; r < last; r += 16) {
-    const int2 an = bounds(r + 16), bn = bounds(r + 24);
-    int ia = (a.x & ~3) + lane * 4, ib = (b.x & ~3) + lane * 4;
+    const uint2 an = bounds(r + 16), bn = bounds(r + 24);
+    unsigned ia = (a.x & ~3u) + lane * 4, ib = (b.x & ~3u) + lane * 4;
     while (__any_sync(0xffffffffu, ia < a.y || ib < b.y)) {
       int4 va = relabel_load(col, a, ia), vb = relabel_load(col, b, ib);
       va = make_int4(delta[va.x], delta[va.y], delta[va.z], delta[va.w]);

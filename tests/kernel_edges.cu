@@ -1,0 +1,53 @@
+// Kernels of the library launched alone, on inputs that its entry points reach at sizes too large for a test.
+#include "../fastembedr_gb300/csrc/tsne_grid.cu"
+
+namespace {
+constexpr long long kEntries = 1LL << 31;  // of P: one more than the largest row bound
+
+// Fills the last `tail` of kEntries entries of a fresh device array from host values.
+template <typename T>
+struct Tail {
+  T* d = nullptr;
+  Tail(const T* host, long long tail) {
+    FE_CUDA(cudaMalloc(&d, sizeof(T) * kEntries));
+    FE_CUDA(cudaMemcpy(d + kEntries - tail, host, sizeof(T) * tail, cudaMemcpyHostToDevice));
+  }
+  ~Tail() { cudaFree(d); }
+};
+template <typename T>
+struct Array {
+  T* d = nullptr;
+  Array(const T* host, long long count) {
+    FE_CUDA(cudaMalloc(&d, sizeof(T) * count));
+    FE_CUDA(cudaMemcpy(d, host, sizeof(T) * count, cudaMemcpyHostToDevice));
+  }
+  ~Array() { cudaFree(d); }
+};
+}  // namespace
+
+// rows: n bounds into the kEntries entries, whose last `tail` are given; col is relabelled in place.
+extern "C" int edge_relabel(const int* rows, int n, int* col, long long tail, const int* delta) {
+  return fe::guarded([&] {
+    Array<int2> r((const int2*)rows, n);
+    Array<int> dl(delta, n);
+    Tail<int> c(col, tail);
+    fe::relabel_rows_kernel<<<1, 256>>>(c.d, r.d, n, dl.d);
+    FE_LAUNCH("relabel_rows_kernel");
+    FE_CUDA(cudaMemcpy(col, c.d + kEntries - tail, sizeof(int) * tail, cudaMemcpyDeviceToHost));
+  });
+}
+
+extern "C" int edge_attractive(const int* rows, int n, const int* col, const float* val, long long tail, const float* y,
+                               float* attr) {
+  return fe::guarded([&] {
+    Array<int2> r((const int2*)rows, n);
+    Array<float2> p((const float2*)y, n), out((const float2*)attr, n);
+    std::vector<unsigned> zero(2 * fe::kAttrCtrStride, 0u);
+    Array<unsigned> ctr(zero.data(), zero.size());
+    Tail<int> c(col, tail);
+    Tail<float> v(val, tail);
+    fe::attractive_kernel<<<1, fe::kAttrThreads>>>(r.d, c.d, v.d, p.d, n, 1.0f, out.d, ctr.d, 1, 1u);
+    FE_LAUNCH("attractive_kernel");
+    FE_CUDA(cudaMemcpy(attr, out.d, sizeof(float2) * n, cudaMemcpyDeviceToHost));
+  });
+}
