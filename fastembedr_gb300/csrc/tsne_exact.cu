@@ -201,8 +201,8 @@ kl_rows_kernel(const int* __restrict__ row_ptr, const int* __restrict__ col, con
   Float2Sum acc{0.0f, 0.0f};
   for (int i = blockIdx.x * 8 + (threadIdx.x >> 5); i < n; i += warps) {
     const float2 yi = inv ? y[inv[i]] : y_rows[i];
-    const int end = row_ptr[i + 1];
-    for (int p = row_ptr[i] + lane; p < end; p += 32) {
+    const unsigned end = row_ptr[i + 1];  // unsigned: the step past a row that ends near 2^31 goes beyond it
+    for (unsigned p = row_ptr[i] + lane; p < end; p += 32) {
       const float2 yj = y[col[p]];
       const float pv = val[p];
       const float dx = yi.x - yj.x, dy = yi.y - yj.y;

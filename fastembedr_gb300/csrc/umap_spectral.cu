@@ -85,7 +85,8 @@ __global__ void sp_degree_kernel(const int* __restrict__ offsets, const float* _
   }
 }
 
-// nw[p] = float(w / sqrt(max(deg_r deg_j, 1e-24))): one warp per row, lanes over its entries.
+// nw[p] = float(w / sqrt(max(deg_r deg_j, 1e-24))): one warp per row, lanes over its entries. (Entries are numbered
+// unsigned where a step may go beyond a row that ends near 2^31.)
 __global__ void __launch_bounds__(kSpThreads)
 sp_adjacency_kernel(const int* __restrict__ offsets, const int* __restrict__ nb, const float* __restrict__ w,
                     const float* __restrict__ deg, int n, float* __restrict__ nw) {
@@ -93,7 +94,7 @@ sp_adjacency_kernel(const int* __restrict__ offsets, const int* __restrict__ nb,
   const int warps = gridDim.x * (blockDim.x >> 5);
   for (int r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); r < n; r += warps) {
     const double dr = (double)deg[r];
-    for (int p = offsets[r] + lane; p < offsets[r + 1]; p += 32) {
+    for (unsigned p = offsets[r] + lane, end = offsets[r + 1]; p < end; p += 32) {
       const double den = __dsqrt_rn(fmax(__dmul_rn(dr, (double)deg[nb[p]]), 1e-24));
       nw[p] = (float)__ddiv_rn((double)w[p], den);
     }
@@ -364,13 +365,14 @@ __device__ void sp_factor(SpShared& sh) {
 // round by shuffles, and every lane gathers its column's 8 values, the next group's before it adds this one's.
 // `step` entries apart.
 __device__ __forceinline__ double sp_row_sum(const int* __restrict__ nb, const float* __restrict__ nw,
-                                             const double* xc, int first, int end, int step, unsigned gmask) {
+                                             const double* xc, unsigned first, unsigned end, unsigned step,
+                                             unsigned gmask) {
   const int c = threadIdx.x & 7;
-  auto entry = [&](int p, int& j, double& w) {
+  auto entry = [&](unsigned p, int& j, double& w) {
     j = p < end ? nb[p] : 0;
     w = p < end ? (double)nw[p] : 0.0;
   };
-  auto gather = [&](int base, int j, double (&v)[8]) {
+  auto gather = [&](unsigned base, int j, double (&v)[8]) {
 #pragma unroll
     for (int t = 0; t < 8; ++t) {
       const int jt = __shfl_sync(gmask, j, t, 8);
@@ -381,7 +383,7 @@ __device__ __forceinline__ double sp_row_sum(const int* __restrict__ nb, const f
   int j;
   entry(first + c, j, w);
   gather(first, j, v);
-  for (int base = first; base < end; base += step) {
+  for (unsigned base = first; base < end; base += step) {
     int jn;
     double wn, vn[8];
     entry(base + step + c, jn, wn);
@@ -410,13 +412,13 @@ __device__ void sp_multiply_rows(const int* __restrict__ offsets, const int* __r
   const double* xc = x + (long long)(c < B ? c : 0) * n;
   for (int g0 = begin + (threadIdx.x >> 5) * 4; g0 < end; g0 += stride) {
     const int g = g0 + slot, r = g < end ? row_of(g) : n;
-    const int p0 = r < n ? offsets[r] : 0, p1 = r < n ? offsets[r + 1] : 0;
+    const unsigned p0 = r < n ? offsets[r] : 0, p1 = r < n ? offsets[r + 1] : 0;
     double acc = sp_row_sum(nb, nw, xc, p0, min(p1, p0 + kSpRowEntries), 8, 0xffu << (slot * 8));
     unsigned longer = __ballot_sync(0xffffffffu, p1 - p0 > kSpRowEntries);
     while (longer) {
       const int who = __ffs(longer) - 1;  // the first lane of a slot
       longer &= ~(0xffu << who);
-      const int q0 = __shfl_sync(0xffffffffu, p0, who) + kSpRowEntries, q1 = __shfl_sync(0xffffffffu, p1, who);
+      const unsigned q0 = __shfl_sync(0xffffffffu, p0, who) + kSpRowEntries, q1 = __shfl_sync(0xffffffffu, p1, who);
       double more = sp_row_sum(nb, nw, xc, q0 + slot * 8, q1, 32, 0xffu << (slot * 8));
       more = __dadd_rn(more, __shfl_xor_sync(0xffffffffu, more, 8));
       more = __dadd_rn(more, __shfl_xor_sync(0xffffffffu, more, 16));

@@ -1,5 +1,7 @@
 // Kernels of the library launched alone, on inputs that its entry points reach at sizes too large for a test.
+#include "../fastembedr_gb300/csrc/tsne_exact.cu"
 #include "../fastembedr_gb300/csrc/tsne_grid.cu"
+#include "../fastembedr_gb300/csrc/umap_spectral.cu"
 
 namespace {
 constexpr long long kEntries = 1LL << 31;  // of P: one more than the largest row bound
@@ -49,5 +51,38 @@ extern "C" int edge_attractive(const int* rows, int n, const int* col, const flo
     fe::attractive_kernel<<<1, fe::kAttrThreads>>>(r.d, c.d, v.d, p.d, n, 1.0f, out.d, ctr.d, 1, 1u);
     FE_LAUNCH("attractive_kernel");
     FE_CUDA(cudaMemcpy(attr, out.d, sizeof(float2) * n, cudaMemcpyDeviceToHost));
+  });
+}
+
+// part[b]: the blocks' sums of p log((p + 1e-9) / (q / z + 1e-9)); bounds: n + 1 row bounds.
+extern "C" int edge_kl(const int* bounds, int n, const int* col, const float* val, long long tail, const float* y, double z,
+                       double* sum) {
+  return fe::guarded([&] {
+    Array<int> b(bounds, n + 1);
+    Array<float2> p((const float2*)y, n);
+    Array<double> dz(&z, 1), out(&z, 1);
+    Tail<int> c(col, tail);
+    Tail<float> v(val, tail);
+    fe::kl_rows_kernel<<<1, 256>>>(b.d, c.d, v.d, p.d, p.d, nullptr, n, dz.d, out.d);
+    FE_LAUNCH("kl_rows_kernel");
+    FE_CUDA(cudaMemcpy(sum, out.d, sizeof(double), cudaMemcpyDeviceToHost));
+  });
+}
+
+// w: normalised in place by the degrees; out = W x, n x columns (column-major).
+extern "C" int edge_spectral(const int* bounds, int n, const int* col, float* w, long long tail, const float* degree,
+                             const double* x, int columns, double* out) {
+  return fe::guarded([&] {
+    Array<int> b(bounds, n + 1);
+    Array<float> dg(degree, n);
+    Array<double> dx(x, (long long)n * columns), dy(out, (long long)n * columns);
+    Tail<int> c(col, tail);
+    Tail<float> v(w, tail), nw(w, tail);
+    fe::sp_adjacency_kernel<<<1, fe::kSpThreads>>>(b.d, c.d, v.d, dg.d, n, nw.d);
+    FE_LAUNCH("sp_adjacency_kernel");
+    fe::sp_multiply_kernel<<<1, fe::kSpThreads>>>(b.d, c.d, nw.d, n, columns, dx.d, dy.d);
+    FE_LAUNCH("sp_multiply_kernel");
+    FE_CUDA(cudaMemcpy(w, nw.d + kEntries - tail, sizeof(float) * tail, cudaMemcpyDeviceToHost));
+    FE_CUDA(cudaMemcpy(out, dy.d, sizeof(double) * n * columns, cudaMemcpyDeviceToHost));
   });
 }

@@ -1,8 +1,10 @@
-"""Rows of P that end within a round of 128 entries of 2^31, the largest number of entries that is accepted: the
-relabelling and the attractive pass, launched alone on arrays of 2^31 entries whose tail alone is filled.
+"""Rows of P, or of a UMAP graph, that end within a round of 2^31, the largest number of entries that is accepted: the
+kernels that step over a row's entries, launched alone on arrays of 2^31 entries whose tail alone is filled.
 
-Relabelling: exact. Attraction: FP64 restatement; each lane sums at most two entries a row in FP32 and the warp's sum has
-five levels, each term's factors and products are within 6 units of 2^-24: 2^-20 of the sum of magnitudes.
+Relabelling: exact. The others against FP64. Attraction: each lane sums at most two entries a row in FP32 and the warp's
+sum has five levels, each term's factors and products are within 6 units of 2^-24: 2^-20 of the sum of magnitudes. KL:
+the differences and d^2 are rounded to float, 2^-22 of log(1 + d^2) at most. Spectral: the weights are rounded to float once, 2^-23 allowed
+for a tie; the products are FP64 sums of at most 300 terms, 2^-44.
 """
 import ctypes as C
 import os
@@ -66,3 +68,47 @@ def test_attractive(lib):
         d = y64[i] - y64[col[a:b]]
         t = (val[a:b] / (1 + (d * d).sum(1)))[:, None] * d
         assert (np.abs(got[i] - t.sum(0)) <= 2.0 ** -20 * np.abs(t).sum(0)).all()
+
+
+# contiguous rows up to the last entry: longer and shorter than a round of 32, a single entry, none
+CONTIGUOUS = np.array([300, 140, 33, 33, 1, 0])
+
+
+def _graph(seed):
+    rng = np.random.default_rng(seed)
+    bounds = (LAST - CONTIGUOUS).astype(np.int32)
+    n = len(bounds) - 1
+    return rng, bounds, n, rng.integers(0, n, TAIL).astype(np.int32), rng.uniform(0.01, 1.0, TAIL).astype(np.float32)
+
+
+def test_kl(lib):
+    rng, bounds, n, col, val = _graph(3)
+    y = rng.normal(size=(n, 2)).astype(np.float32)
+    z, got = 20.0, np.zeros(1)
+    assert lib.edge_kl(bounds.ctypes.data_as(C.c_void_p), n, col.ctypes.data_as(C.c_void_p),
+                       val.ctypes.data_as(C.c_void_p), C.c_longlong(TAIL), y.ctypes.data_as(C.c_void_p), C.c_double(z),
+                       got.ctypes.data_as(C.c_void_p)) == 0
+    want = size = 0.0
+    for i in range(n):
+        s = slice(bounds[i] - (ENTRIES - TAIL), bounds[i + 1] - (ENTRIES - TAIL))
+        d = y[i].astype(np.float64) - y[col[s]]
+        p = val[s].astype(np.float64)
+        want += (p * np.log((p + 1e-9) / (1 / (1 + (d * d).sum(1)) / z + 1e-9))).sum()
+        size += (p * np.log1p((d * d).sum(1))).sum()
+    assert abs(got[0] - want) <= 2.0 ** -22 * size
+
+
+def test_spectral(lib):
+    rng, bounds, n, col, val = _graph(4)
+    degree = rng.uniform(0.5, 2.0, n).astype(np.float32)
+    x = rng.normal(size=(8, n))
+    w, got = val.copy(), np.zeros((8, n))
+    assert lib.edge_spectral(bounds.ctypes.data_as(C.c_void_p), n, col.ctypes.data_as(C.c_void_p),
+                             w.ctypes.data_as(C.c_void_p), C.c_longlong(TAIL), degree.ctypes.data_as(C.c_void_p),
+                             x.ctypes.data_as(C.c_void_p), 8, got.ctypes.data_as(C.c_void_p)) == 0
+    for i in range(n):
+        s = slice(bounds[i] - (ENTRIES - TAIL), bounds[i + 1] - (ENTRIES - TAIL))
+        want = val[s] / np.sqrt(degree[i].astype(np.float64) * degree[col[s]].astype(np.float64))
+        np.testing.assert_allclose(w[s], want, rtol=2.0 ** -23)
+        t = w[s].astype(np.float64) * x[:, col[s]]
+        assert (np.abs(got[:, i] - t.sum(1)) <= 2.0 ** -44 * np.abs(t).sum(1)).all()
