@@ -196,7 +196,8 @@ kl_rows_kernel(const int* __restrict__ row_ptr, const int* __restrict__ col, con
   fill_log_table(table);
   __syncthreads();
   const int lane = threadIdx.x & 31, warps = gridDim.x * 8;
-  const Float2Sum inv_z = split(1.0 / (double)(float)fmax(*zsum, (double)FLT_MIN));
+  const double over_z = 1.0 / (double)(float)fmax(*zsum, (double)FLT_MIN);
+  const Float2Sum inv_z = split(over_z);
   const Float2Sum tiny = split(1e-9);
   Float2Sum acc{0.0f, 0.0f};
   for (int i = blockIdx.x * 8 + (threadIdx.x >> 5); i < n; i += warps) {
@@ -207,8 +208,9 @@ kl_rows_kernel(const int* __restrict__ row_ptr, const int* __restrict__ col, con
       const float pv = val[p];
       const float dx = yi.x - yj.x, dy = yi.y - yj.y;
       const float d2 = __fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy));
-      Float2Sum den = tiny;
+      Float2Sum den;
       if (!(d2 > 1.0e30f)) den = add(mul(divide(Float2Sum{1.0f, 0.0f}, two_sum(1.0f, d2)), inv_z), tiny);
+      else den = split(1.0 / (1.0 + (double)d2) * over_z + 1e-9);  // q is small, but Z may be as well
       const Float2Sum l = log_two(divide(add(tiny, pv), den), table);
       acc = add(acc, mul(l, pv));
     }
