@@ -412,16 +412,6 @@ __device__ __forceinline__ void two_sum_add(float& hi, float& lo, float u) {
 
 __device__ __forceinline__ float sign_f(float v) { return v == 0.0f ? 0.0f : (v < 0.0f ? -1.0f : 1.0f); }
 
-// Correctly rounded 1 / x for x in [1, 2^126): one Newton step by fused multiply-add on an approximation
-// within one unit in the last place rounds correctly (Markstein 1990); larger x, where the result is
-// below 1.2e-38, give 0. Free of the branch to a slow path, so that several pairs are in flight.
-__device__ __forceinline__ float reciprocal(float x) {
-  float r;
-  const float c = fminf(x, 3.4e38f);
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(c));
-  return __fmaf_rn(r, __fmaf_rn(-c, r, 1.0f), r);
-}
-
 // One repulsion pair: q, q^2 (y - r) with the compensated query position.
 __device__ __forceinline__ void repulse(float2 rr, float yhx, float yhy, float ylx, float yly, float& fz, float& fx,
                                         float& fy) {
