@@ -1,4 +1,5 @@
-// Exponential and logarithm in two floats (relative / absolute error about 1e-12), for the per-row searches
+// Exponential and logarithm in two floats (exp x: within 3e-12 of itself where its low part is a normal float; log x:
+// within 1e-12 (1 + |log2 x|)), for the per-row searches
 // and sums whose decisions FP32 is too short for: the FP64 pipe of this part issues one warp
 // instruction every 19 cycles of an SM, and an FP64 exp or log takes 40 to 50 of them (about 900
 // cycles) where these take 35 to 45 FP32 instructions (about 10).
@@ -65,14 +66,15 @@ __device__ __forceinline__ Float2Sum log_two(Float2Sum x, const float4* __restri
   const float p = __fmul_rn(m, t.x);
   const float z = __fsub_rn(p, 1.0f);  // exact
   const float zl = __fadd_rn(__fmaf_rn(m, t.x, -p), __fmul_rn(ml, t.x));
-  // log1p(z + zl) = z + zl - z^2 / 2 - z zl + z^3 / 3 - ...
+  // log1p(z + zl) = z + zl - z^2 / 2 - z zl + z^3 / 3 + z^2 zl - ...
   const float w = __fmul_rn(z, z), wl = __fmaf_rn(z, z, -w);
   const float poly = __fmul_rn(__fmul_rn(w, z), __fmaf_rn(z, __fmaf_rn(z, __fmaf_rn(z, -1.0f / 6.0f, 0.2f), -0.25f),
                                                           1.0f / 3.0f));
   // log 2 = 0.693145751953125 (16 bits: e times it is exact) + 1.42860682030941723e-6
   const Float2Sum s = two_sum((float)e * 0.693145751953125f, t.y);
   const Float2Sum u = two_sum(s.hi, z), v = two_sum(u.hi, -0.5f * w);
-  const float lo = s.lo + u.lo + v.lo + t.z + zl - 0.5f * wl - z * zl + poly + (float)e * 1.42860682030941723e-6f;
+  const float zz = __fmul_rn(z, zl), cross = __fmaf_rn(-z, zz, zz);
+  const float lo = s.lo + u.lo + v.lo + t.z + zl - 0.5f * wl - cross + poly + (float)e * 1.42860682030941723e-6f;
   return two_sum(v.hi, lo);
 }
 

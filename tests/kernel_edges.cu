@@ -1,4 +1,5 @@
-// Kernels of the library launched alone, on inputs that its entry points reach at sizes too large for a test.
+// Kernels and device functions of the library launched alone: on inputs that its entry points reach at sizes too large
+// for a test, and over the whole range of an argument.
 #include "../fastembedr_gb300/csrc/tsne_exact.cu"
 #include "../fastembedr_gb300/csrc/tsne_grid.cu"
 #include "../fastembedr_gb300/csrc/umap_spectral.cu"
@@ -84,5 +85,55 @@ extern "C" int edge_spectral(const int* bounds, int n, const int* col, float* w,
     FE_LAUNCH("sp_multiply_kernel");
     FE_CUDA(cudaMemcpy(w, nw.d + kEntries - tail, sizeof(float) * tail, cudaMemcpyDeviceToHost));
     FE_CUDA(cudaMemcpy(out, dy.d, sizeof(double) * n * columns, cudaMemcpyDeviceToHost));
+  });
+}
+
+namespace {
+__global__ void exp_kernel(const float2* x, int n, double* relative) {
+  __shared__ float2 table[fe::kExpEntries];
+  fe::fill_exp_table(table);
+  __syncthreads();
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const fe::Float2Sum v{x[i].x, x[i].y};
+    const double want = exp(fe::value(v));
+    relative[i] = (fe::value(fe::exp_two(v, table)) - want) / want;
+  }
+}
+__global__ void log_kernel(const float2* x, int n, double* absolute) {
+  __shared__ float4 table[fe::kLogEntries];
+  fe::fill_log_table(table);
+  __syncthreads();
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const fe::Float2Sum v{x[i].x, x[i].y};
+    absolute[i] = fe::value(fe::log_two(v, table)) - log(fe::value(v));
+  }
+}
+__global__ void reciprocal_kernel(int exponent, unsigned long long* differ) {
+  const unsigned m = blockIdx.x * blockDim.x + threadIdx.x;
+  const float x = __uint_as_float((unsigned)(127 + exponent) << 23 | m);
+  if (m < (1u << 23) && __float_as_uint(fe::reciprocal(x)) != __float_as_uint(__frcp_rn(x))) atomicAdd(differ, 1ull);
+}
+}  // namespace
+
+// error[i]: of exp(x[i]) relative to CUDA's FP64 function, or of log(x[i]) absolute; x: high and low parts.
+extern "C" int edge_two_float(int logarithm, const float* x, int n, double* error) {
+  return fe::guarded([&] {
+    Array<float2> dx((const float2*)x, n);
+    Array<double> e(error, n);
+    if (logarithm) log_kernel<<<64, 256>>>(dx.d, n, e.d);
+    else exp_kernel<<<64, 256>>>(dx.d, n, e.d);
+    FE_LAUNCH("two-float function");
+    FE_CUDA(cudaMemcpy(error, e.d, sizeof(double) * n, cudaMemcpyDeviceToHost));
+  });
+}
+
+// How many of the 2^23 floats in [2^exponent, 2^(exponent + 1)) have a reciprocal other than the correctly rounded one.
+extern "C" int edge_reciprocal(int exponent, unsigned long long* differ) {
+  return fe::guarded([&] {
+    *differ = 0;
+    Array<unsigned long long> d(differ, 1);
+    reciprocal_kernel<<<(1 << 23) / 256, 256>>>(exponent, d.d);
+    FE_LAUNCH("reciprocal_kernel");
+    FE_CUDA(cudaMemcpy(differ, d.d, sizeof(*differ), cudaMemcpyDeviceToHost));
   });
 }

@@ -1,4 +1,4 @@
-"""Rows of P, or of a UMAP graph, that end within a round of 2^31, the largest number of entries that is accepted: the
+"""Kernels and device functions launched alone. Rows of P, or of a UMAP graph, that end within a round of 2^31, the largest number of entries that is accepted: the
 kernels that step over a row's entries, launched alone on arrays of 2^31 entries whose tail alone is filled.
 
 Relabelling: exact. The others against FP64. Attraction: each lane sums at most two entries a row in FP32 and the warp's
@@ -112,3 +112,34 @@ def test_spectral(lib):
         np.testing.assert_allclose(w[s], want, rtol=2.0 ** -23)
         t = w[s].astype(np.float64) * x[:, col[s]]
         assert (np.abs(got[:, i] - t.sum(1)) <= 2.0 ** -44 * np.abs(t).sum(1)).all()
+
+
+# Bounds of the two-float functions, from their steps. exp: the polynomial, at most 1.5e-5, is rounded about five times in
+# FP32 (2.2e-12), the table and the products to 2^-47. log: eight FP32 additions of low parts of at most 1.5e-6 |log2 x| +
+# 3e-7 (7e-13 |log2 x| + 2e-13) and the rounding of |log2 x| 1.4e-6 (1.3e-13 |log2 x|).
+def test_exp_two(lib):
+    rng = np.random.default_rng(6)
+    x = np.r_[-np.geomspace(1e-9, 50.0, 200001), -np.arange(0, 50, 0.0108304247, dtype=np.float64), 0.0]
+    x = np.c_[x.astype(np.float32), np.zeros(len(x), np.float32)]
+    x[:, 1] = x[:, 0] * rng.uniform(-2.0 ** -25, 2.0 ** -25, len(x))
+    err = np.zeros(len(x))
+    assert lib.edge_two_float(0, x.ctypes.data_as(C.c_void_p), len(x), err.ctypes.data_as(C.c_void_p)) == 0
+    assert np.abs(err).max() <= 3e-12, (np.abs(err).max(), x[np.abs(err).argmax()])
+
+
+def test_log_two(lib):
+    rng = np.random.default_rng(7)
+    x = np.r_[np.geomspace(1e-30, 1e30, 200001), np.linspace(0.5, 2.0, 100001), 2.0 ** np.arange(-100, 100)]
+    x = np.c_[x.astype(np.float32), np.zeros(len(x), np.float32)]
+    x[:, 1] = x[:, 0] * rng.uniform(-2.0 ** -25, 2.0 ** -25, len(x))
+    err = np.zeros(len(x))
+    assert lib.edge_two_float(1, x.ctypes.data_as(C.c_void_p), len(x), err.ctypes.data_as(C.c_void_p)) == 0
+    bound = 1e-12 * (1.0 + np.abs(np.log2(x[:, 0].astype(np.float64))))
+    assert (np.abs(err) <= bound).all(), (np.abs(err) / bound).max()
+
+
+@pytest.mark.parametrize("exponent", [0, 1, 2, 7, 63, 124, 125])
+def test_reciprocal_is_correctly_rounded(lib, exponent):
+    differ = C.c_ulonglong(1)
+    assert lib.edge_reciprocal(exponent, C.byref(differ)) == 0
+    assert differ.value == 0
