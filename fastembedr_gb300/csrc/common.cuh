@@ -153,10 +153,10 @@ __device__ __forceinline__ Float2Sum divide(Float2Sum a, Float2Sum b) {
 // Correctly rounded 1 / x for x in [1, 2^126): one Newton step by fused multiply-add on an approximation
 // within one unit in the last place (Markstein 1990, whose theorem leaves out significands of all ones; with this
 // part's approximation the step rounds correctly for them too: compared for all 2^23 significands). Larger x, where the
-// result is below 1.2e-38, give 0. Free of the branch to a slow path, so that several pairs are in flight.
+// result is below 1.2e-38, give 0, and NaN gives NaN. Free of the branch to a slow path, so that several pairs are in flight.
 __device__ __forceinline__ float reciprocal(float x) {
-  float r;
-  const float c = fminf(x, 3.4e38f);
+  float r, c;
+  asm("min.NaN.f32 %0, %1, 0f7F7FC99E;" : "=f"(c) : "f"(x));  // 3.4e38: an infinite x must not make the step NaN
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(c));
   return __fmaf_rn(r, __fmaf_rn(-c, r, 1.0f), r);
 }

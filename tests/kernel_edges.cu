@@ -111,7 +111,8 @@ __global__ void log_kernel(const float2* x, int n, double* absolute) {
 __global__ void reciprocal_kernel(int exponent, unsigned long long* differ) {
   const unsigned m = blockIdx.x * blockDim.x + threadIdx.x;
   const float x = __uint_as_float((unsigned)(127 + exponent) << 23 | m);
-  if (m < (1u << 23) && __float_as_uint(fe::reciprocal(x)) != __float_as_uint(__frcp_rn(x))) atomicAdd(differ, 1ull);
+  const float got = fe::reciprocal(x), want = __frcp_rn(x);
+  if (m < (1u << 23) && !(got == want || (isnan(got) && isnan(want)))) atomicAdd(differ, 1ull);
 }
 }  // namespace
 
@@ -127,7 +128,7 @@ extern "C" int edge_two_float(int logarithm, const float* x, int n, double* erro
   });
 }
 
-// How many of the 2^23 floats in [2^exponent, 2^(exponent + 1)) have a reciprocal other than the correctly rounded one.
+// How many of the 2^23 floats in [2^exponent, 2^(exponent + 1)) (128: infinity and the NaNs) have a reciprocal other than the correctly rounded one.
 extern "C" int edge_reciprocal(int exponent, unsigned long long* differ) {
   return fe::guarded([&] {
     *differ = 0;
@@ -135,5 +136,20 @@ extern "C" int edge_reciprocal(int exponent, unsigned long long* differ) {
     reciprocal_kernel<<<(1 << 23) / 256, 256>>>(exponent, d.d);
     FE_LAUNCH("reciprocal_kernel");
     FE_CUDA(cudaMemcpy(differ, d.d, sizeof(*differ), cudaMemcpyDeviceToHost));
+  });
+}
+
+// Z, the sum of q over all pairs of different points.
+extern "C" int edge_z(const float* y, int n, double* z) {
+  return fe::guarded([&] {
+    const int tiles = (n + fe::kPairTile - 1) / fe::kPairTile, blocks = 256;
+    std::vector<double> part(blocks);
+    Array<float2> p((const float2*)y, n);
+    Array<double> out(part.data(), blocks);
+    fe::sum_q_tiles_kernel<<<blocks, 256>>>(p.d, n, tiles, out.d);
+    FE_LAUNCH("sum_q_tiles_kernel");
+    FE_CUDA(cudaMemcpy(part.data(), out.d, sizeof(double) * blocks, cudaMemcpyDeviceToHost));
+    *z = 0.0;
+    for (double v : part) *z += v;
   });
 }

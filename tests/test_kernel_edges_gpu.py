@@ -138,8 +138,22 @@ def test_log_two(lib):
     assert (np.abs(err) <= bound).all(), (np.abs(err) / bound).max()
 
 
-@pytest.mark.parametrize("exponent", [0, 1, 2, 7, 63, 124, 125])
+@pytest.mark.parametrize("exponent", [0, 1, 2, 7, 63, 124, 125, 128])
 def test_reciprocal_is_correctly_rounded(lib, exponent):
     differ = C.c_ulonglong(1)
     assert lib.edge_reciprocal(exponent, C.byref(differ)) == 0
     assert differ.value == 0
+
+
+# The sum over all pairs keeps FP64's digits though its terms are floats: they are correctly rounded, so their errors (a
+# few 2^-25) have no common sign and average out over 10^8 pairs, as do those of the FP32 sums of 128 terms (rms
+# 2e-7): 2e-7 / sqrt(4e5 sums) = 3e-10, three times that allowed.
+@pytest.mark.parametrize("spread", [0.1, 30.0])
+def test_normaliser(lib, spread):
+    n = 10000
+    y = (np.random.default_rng(8).standard_normal((n, 2)) * spread).astype(np.float32)
+    got = C.c_double()
+    assert lib.edge_z(y.ctypes.data_as(C.c_void_p), n, C.byref(got)) == 0
+    y64 = y.astype(np.float64)
+    want = sum((1 / (1 + ((y64[s:s + 500, None] - y64[None]) ** 2).sum(2))).sum() for s in range(0, n, 500)) - n
+    assert got.value == pytest.approx(want, rel=1e-9)
