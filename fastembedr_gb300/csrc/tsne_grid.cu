@@ -415,8 +415,10 @@ scatter_kernel(const float2* __restrict__ y, const TsneInstance* __restrict__ in
 // of columns and values bypasses L1. A warp whose SM has no chunk left takes chunks from the
 // SM with the most left, so uneven row lengths, or an SM shared with the grid stage, cost nothing.
 //
-// With three quarters of the gathers served by L1 the pass is bound by instruction issue (75 % of
-// the issue slots at 400,000 points), so the rest of the kernel is about instructions. A row is read
+// How many gathers L1 serves depends on the layout: 75 to 77 % where neighbours in the data lie close together in the
+// layout (discs drawn from the data's own coordinates), and the pass is then bound by instruction issue (75 % of the
+// issue slots at 400,000 points); 54 % on an optimised layout of 30 large clusters, where it is half issue, half
+// waiting (50 % of the slots at 200,000 points). So the rest of the kernel is about instructions. A row is read
 // in rounds of 128 entries from c0, its first entry rounded down to a multiple of 4, with 128-bit
 // loads (lane l takes entries 4 l .. + 3); entries outside the row are masked only in the rounds that
 // can hold some. Two rows share one reduction, and the two rows after them are prefetched into L2
@@ -568,9 +570,10 @@ __device__ __forceinline__ unsigned attr_left(unsigned* __restrict__ ctr, unsign
   return nchunks;
 }
 
-// Per iteration at 1M points (143 M entries, 90 neighbours): 0.508 -> 0.326 ms; 200,000: 98 -> 80 us.
-// The queues took the L1 hit rate from 27 to 77 % and the time to 0.35 ms; the rest came from the
-// masks, the shared reductions and the prefetch. Six blocks per SM with a few spilled registers are
+// Per iteration on discs (see above) of 1M points (143 M entries, 90 neighbours): 0.508 -> 0.326 ms; 200,000: 98 -> 80
+// us. The queues took the L1 hit rate from 27 to 77 % there and the time to 0.35 ms; the rest came from the
+// masks, the shared reductions and the prefetch. On an optimised layout of 1M points in 30 clusters: 0.582 -> 0.495 ms
+// (hits 22 -> 54 % at 200,000 points). Six blocks per SM with a few spilled registers are
 // faster than five without (0.360 ms at 1M). Rounds narrower than 128 entries at a row's end would
 // save instructions but sum a row in another order; they measured 0.317 ms and are not used.
 __global__ void __launch_bounds__(kAttrThreads, 6)
@@ -847,9 +850,9 @@ __global__ void scatter_points_kernel(const float2* __restrict__ scratch, const 
 // col[t] = delta[col[t]] for every entry, row by row in storage order. A block takes consecutive slots, whose
 // rows name points near one another: most gathers then hit L1, where a pass over the entries in the order of the CSR (rows in
 // the caller's order) is bound by the rate of random sectors from L2. Two rows of a warp are in flight, 128
-// entries each. 1M points x 90 neighbours (115M entries): 575 -> 326 us (540 the first time, out of the caller's
-// order), of 135 for moving the columns once. Shares of some 70 rows even out the row lengths: with 8 blocks
-// per SM the pass took 425 us, a third of it waiting for the longest shares.
+// entries each. 1M points x 90 neighbours (115M entries): 575 -> 326 us on discs, 484 on an optimised
+// layout (540 the first time, out of the caller's order), of 135 for moving the columns once. Shares of some 70 rows even out the row lengths: with 8 blocks
+// per SM the pass took 425 us (discs), a third of it waiting for the longest shares.
 // (positions are unsigned, as in attr_row)
 __device__ __forceinline__ int4 relabel_load(const int* __restrict__ col, uint2 se, unsigned i) {
   int4 v = make_int4(0, 0, 0, 0);

@@ -13,9 +13,13 @@
 //
 // The random draws are made in the reference's order (on the host, or the start block of a large layout on
 // the GPU; the column redraw of a vanishing Gram-Schmidt column included); every arithmetic step runs on the GPU in
-// FP64 with the reference's operation order and no contraction (__d*_rn). Sums over points are
-// reduced in a fixed block order, so results are deterministic and differ from the sequential
-// CPU sums by rounding only.
+// FP64, in a fixed order, so that results are deterministic; they differ from the CPU's by rounding. Degrees, the
+// normalisation and the steps after the rounds follow the reference's operations without contraction (__d*_rn) but for
+// sums over points, which go by blocks. The rounds do not: a row's products are fused into its sum and split over lanes, a
+// pass orthonormalises by Cholesky QR (Gram-Schmidt where a column vanishes, with its products not fused), and a Ritz
+// rotation takes its angle with one division and a reciprocal root. Against a restatement in long double on graphs of 600
+// and 1,500 points (well mixed, clustered, with eigenvalues next to 1) the start is as close as with Gram-Schmidt in the
+// reference's order, 1e-13 to 1e-6 of a layout of 10 for either.
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
