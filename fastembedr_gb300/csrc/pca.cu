@@ -33,6 +33,7 @@ constexpr int kMeanSlices = 32;
 constexpr int kJacobiThreads = 1024;
 constexpr int kJacobiSweeps = 30;
 constexpr int kPcaMaxFeatures = 1024;
+constexpr float kCloseGap = 1.0e-4f;
 constexpr int kJacobiSharedFeatures = 152;  // 152 x 152 two-float values: 185 KB of shared memory
 
 // Exponent of the power of two the centred data are divided by (`bits`: their largest magnitude's).
@@ -235,11 +236,12 @@ __device__ __forceinline__ void jacobi_rotate(Float2Sum& x, Float2Sum& y, Float2
 // (`tangents`, kJacobiSweeps (m - 1) m / 2 floats) for the kernel below, instead of carrying all of V along. A tangent
 // is FP32: an angle a little off leaves a little of the entry to the next sweep. Stops when the off-diagonal mass is
 // below 1e-26 of the diagonal mass (entries below 2^-43 of the spectrum), or after kJacobiSweeps sweeps.
-// lambda: the eigenvalues; info: the indices of the two largest, and the number of steps.
+// lambda: the eigenvalues; info: the indices of the two largest, the number of steps, and whether an eigenvalue lies within
+// kCloseGap of one of the two (of the largest).
 //
-// p = 50: 1907 us with A and V in FP64 in global memory, 480 us now, bound by the latency of the two
-// dependent phases of a step; the whole start of 5,000 x 150: 90.8 ms, 6.4 now; x 300, with A in global
-// memory: 1,516 ms, 140 now.
+// p = 50 (200,000 rows): 1916 us with A and V in FP64 in global memory, 194 us now and 37 for the vectors, bound by the
+// latency of the two dependent phases of a step; the whole start of 5,000 x 150: 90.8 ms, 6.2 now; x 300, with A in
+// global memory: 1,516 ms, 131 now.
 template <bool kShared>
 __global__ void __launch_bounds__(kJacobiThreads)
 pca_jacobi_kernel(const double* __restrict__ C, int p, Float2Sum* __restrict__ work, float* __restrict__ tangents,
@@ -249,6 +251,7 @@ pca_jacobi_kernel(const double* __restrict__ C, int p, Float2Sum* __restrict__ w
   __shared__ float4 s_rot[kJacobiThreads];  // c, s
   __shared__ float s_red[2][kJacobiThreads / 32];
   __shared__ bool s_done;
+  __shared__ int s_lead[2];
   Float2Sum* A = kShared ? s_a : work;
   const int m = p + (p & 1), half = m / 2;
   double top = 0.0;  // scaled by a power of two to a largest diagonal entry near 1
@@ -348,13 +351,22 @@ pca_jacobi_kernel(const double* __restrict__ C, int p, Float2Sum* __restrict__ w
     info[0] = b0;
     info[1] = b1;
     info[2] = steps;
+    s_lead[0] = b0;
+    s_lead[1] = b1;
   }
+  __syncthreads();
+  const float l0 = A[s_lead[0] * m + s_lead[0]].hi, l1 = A[s_lead[1] * m + s_lead[1]].hi, near = kCloseGap * l0;
+  bool close = l0 - l1 < near;
+  for (int i = threadIdx.x; i < p; i += blockDim.x)
+    if (i != s_lead[0] && i != s_lead[1]) close |= l1 - A[i * m + i].hi < near;
+  close = __syncthreads_or(close);
+  if (threadIdx.x == 0) info[3] = close;
   for (int i = threadIdx.x; i < p; i += blockDim.x) lambda[i] = value(A[i * m + i]) / unit;
 }
 
 // All eigenvectors, vectors[v * p + i]: the rotations applied in reverse to the unit vectors, a warp for each of a
 // block's two. x <- J x for each step's J, (x_i, x_j) <- (c x_i + s x_j, -s x_i + c x_j); the block computes the
-// rotations of as many steps as it has threads for.
+// rotations of as many steps as it has threads for. 50 vectors: 37 us, as the two leading ones alone took.
 __global__ void __launch_bounds__(kJacobiThreads)
 pca_vectors_kernel(const float* __restrict__ tangents, int p, const int* __restrict__ info,
                    Float2Sum* __restrict__ vectors) {
@@ -401,13 +413,14 @@ pca_vectors_kernel(const float* __restrict__ tangents, int p, const int* __restr
 // R = I - X^T X in FP64, x_c gains sum over i of e_ic x_i, e_ic = (S_ic + lambda_c R_ic) / (lambda_c - lambda_i), or
 // R_ic / 2 for an eigenvalue that cannot be told from lambda_c. It squares the error, which in two floats is some 1e-13
 // over the gap of the eigenvalues: with a gap of 1e-7 of the largest, a start of 151 features was off by 5e-7 of its
-// largest coordinate, 7e-8 now (6e-8 is the rounding to float).
+// largest coordinate, 7e-8 now (6e-8 is the rounding to float). Where no eigenvalue is that close (info[3]) the vectors
+// are good to 1e-9 as they are, and the kernels have nothing to do.
 // y[c * p + r] = (C x_c)_r, a warp per r.
 __global__ void __launch_bounds__(256)
 pca_product_kernel(const double* __restrict__ C, const Float2Sum* __restrict__ X, int p, const int* __restrict__ info,
                    double* __restrict__ y) {
   const int r = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  if (r >= p) return;
+  if (r >= p || !info[3]) return;
   for (int c = 0; c < 2; ++c) {
     const Float2Sum* x = X + (long long)info[c] * p;
     double t = 0.0;
@@ -421,7 +434,7 @@ __global__ void __launch_bounds__(256)
 pca_correction_kernel(const Float2Sum* __restrict__ X, const double* __restrict__ y, int p,
                       const double* __restrict__ lambda, const int* __restrict__ info, double* __restrict__ e) {
   const int i = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  if (i >= p) return;
+  if (i >= p || !info[3]) return;
   const Float2Sum* x = X + (long long)i * p;
   for (int c = 0; c < 2; ++c) {
     const Float2Sum* xc = X + (long long)info[c] * p;
@@ -445,7 +458,7 @@ pca_refine_kernel(const Float2Sum* __restrict__ X, const double* __restrict__ e,
   __shared__ double s_sum[8][2][32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, i = blockIdx.x * 32 + lane;
   double t[2] = {0.0, 0.0};
-  if (i < p)
+  if (i < p && info[3])
     for (int j = warp; j < p; j += 8) {
       const double v = value(X[(long long)j * p + i]);
       t[0] += e[j] * v;
@@ -639,7 +652,7 @@ void pca_tsne_start(const float* X, int n, int p, float2* init, cudaStream_t s) 
   w.reserve(&work, shared ? 1 : m * m);
   w.reserve(&tangents, kJacobiSweeps * (m - 1) * (m / 2));
   w.reserve(&lambda, p);
-  w.reserve(&info, 3);
+  w.reserve(&info, 4);
   w.reserve(&all, (std::size_t)p * p);
   w.reserve(&y, 2 * (std::size_t)p);
   w.reserve(&e, 2 * (std::size_t)p);
