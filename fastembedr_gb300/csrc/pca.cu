@@ -239,7 +239,7 @@ __device__ __forceinline__ void jacobi_rotate(Float2Sum& x, Float2Sum& y, Float2
 // lambda: the eigenvalues; info: the indices of the two largest, the number of steps, and whether an eigenvalue lies within
 // kCloseGap of one of the two (of the largest).
 //
-// p = 50 (200,000 rows): 1916 us with A and V in FP64 in global memory, 194 us now and 37 for the vectors, bound by the
+// p = 50 (200,000 rows): 1916 us with A and V in FP64 in global memory, 194 us now and 41 for the vectors, bound by the
 // latency of the two dependent phases of a step; the whole start of 5,000 x 150: 90.8 ms, 6.2 now; x 300, with A in
 // global memory: 1,516 ms, 131 now.
 template <bool kShared>
@@ -366,10 +366,11 @@ pca_jacobi_kernel(const double* __restrict__ C, int p, Float2Sum* __restrict__ w
 
 // All eigenvectors, vectors[v * p + i]: the rotations applied in reverse to the unit vectors, a warp for each of a
 // block's two. x <- J x for each step's J, (x_i, x_j) <- (c x_i + s x_j, -s x_i + c x_j); the block computes the
-// rotations of as many steps as it has threads for. 50 vectors: 37 us, as the two leading ones alone took.
+// rotations of as many steps as it has threads for. Where they are to be refined, the block of a leading vector x_c also
+// computes y[c * p + r] = (C x_c)_r. 50 vectors: 41 us, little more than the two leading ones alone took (36).
 __global__ void __launch_bounds__(kJacobiThreads)
 pca_vectors_kernel(const float* __restrict__ tangents, int p, const int* __restrict__ info,
-                   Float2Sum* __restrict__ vectors) {
+                   const double* __restrict__ C, Float2Sum* __restrict__ vectors, double* __restrict__ y) {
   __shared__ int2 s_pair[kJacobiThreads];
   __shared__ float4 s_rot[kJacobiThreads];
   __shared__ Float2Sum s_vec[2][kPcaMaxFeatures];
@@ -407,6 +408,17 @@ pca_vectors_kernel(const float* __restrict__ tangents, int p, const int* __restr
     const int v = i / p;
     if (first + v < p) vectors[(long long)(first + v) * p + i % p] = s_vec[v][i % p];
   }
+  if (!info[3]) return;
+  for (int c = 0; c < 2; ++c) {
+    const int v = info[c] - first;
+    if (v < 0 || v > 1) continue;
+    for (int r = comp; r < p; r += kJacobiThreads / 32) {
+      double t = 0.0;
+      for (int i = lane; i < p; i += 32) t += C[(long long)r * p + i] * value(s_vec[v][i]);
+      t = warp_sum(t);
+      if (lane == 0) y[c * p + r] = t;
+    }
+  }
 }
 
 // One step of Ogita and Aishima's refinement (2018) for the two leading eigenvectors x_c: with S = X^T C X and
@@ -414,63 +426,47 @@ pca_vectors_kernel(const float* __restrict__ tangents, int p, const int* __restr
 // R_ic / 2 for an eigenvalue that cannot be told from lambda_c. It squares the error, which in two floats is some 1e-13
 // over the gap of the eigenvalues: with a gap of 1e-7 of the largest, a start of 151 features was off by 5e-7 of its
 // largest coordinate, 7e-8 now (6e-8 is the rounding to float). Where no eigenvalue is that close (info[3]) the vectors
-// are good to 1e-9 as they are, and the kernels have nothing to do.
-// y[c * p + r] = (C x_c)_r, a warp per r.
-__global__ void __launch_bounds__(256)
-pca_product_kernel(const double* __restrict__ C, const Float2Sum* __restrict__ X, int p, const int* __restrict__ info,
-                   double* __restrict__ y) {
-  const int r = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  if (r >= p || !info[3]) return;
-  for (int c = 0; c < 2; ++c) {
-    const Float2Sum* x = X + (long long)info[c] * p;
-    double t = 0.0;
-    for (int i = lane; i < p; i += 32) t += C[(long long)r * p + i] * value(x[i]);
-    t = warp_sum(t);
-    if (lane == 0) y[c * p + r] = t;
-  }
-}
-// e[c * p + i] = e_ic, a warp per i.
-__global__ void __launch_bounds__(256)
-pca_correction_kernel(const Float2Sum* __restrict__ X, const double* __restrict__ y, int p,
-                      const double* __restrict__ lambda, const int* __restrict__ info, double* __restrict__ e) {
-  const int i = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  if (i >= p || !info[3]) return;
-  const Float2Sum* x = X + (long long)i * p;
-  for (int c = 0; c < 2; ++c) {
-    const Float2Sum* xc = X + (long long)info[c] * p;
-    double s = 0.0, r = 0.0;
-    for (int j = lane; j < p; j += 32) {
-      const double v = value(x[j]);
-      s += v * y[c * p + j];
-      r += v * value(xc[j]);
-    }
-    s = warp_sum(s);
-    r = (i == info[c] ? 1.0 : 0.0) - warp_sum(r);
-    const double gap = lambda[info[c]] - lambda[i];
-    if (lane == 0)
-      e[c * p + i] = fabs(gap) > 1e-12 * fabs(lambda[info[0]]) ? (s + lambda[info[c]] * r) / gap : 0.5 * r;
-  }
-}
-// vectors[c * p + i] = component c; block: 32 coordinates, eight warps share the sum.
-__global__ void __launch_bounds__(256)
-pca_refine_kernel(const Float2Sum* __restrict__ X, const double* __restrict__ e, int p, const int* __restrict__ info,
-                  Float2Sum* __restrict__ vectors) {
-  __shared__ double s_sum[8][2][32];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, i = blockIdx.x * 32 + lane;
+// are good to 1e-9 as they are. vectors[c * p + i] = component c; a block takes 32 coordinates, for which its warps form
+// every e_ic and share the sums.
+__global__ void __launch_bounds__(kJacobiThreads)
+pca_refine_kernel(const Float2Sum* __restrict__ X, const double* __restrict__ y, int p,
+                  const double* __restrict__ lambda, const int* __restrict__ info, Float2Sum* __restrict__ vectors) {
+  constexpr int kWarps = kJacobiThreads / 32;
+  __shared__ double s_e[2][kPcaMaxFeatures], s_sum[kWarps][2][32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, at = blockIdx.x * 32 + lane;
+  const int lead[2] = {info[0], info[1]};
   double t[2] = {0.0, 0.0};
-  if (i < p && info[3])
-    for (int j = warp; j < p; j += 8) {
-      const double v = value(X[(long long)j * p + i]);
-      t[0] += e[j] * v;
-      t[1] += e[p + j] * v;
+  if (info[3]) {
+    for (int q = warp; q < 2 * p; q += kWarps) {
+      const int c = q / p, i = q - c * p;
+      const Float2Sum *x = X + (long long)i * p, *xc = X + (long long)lead[c] * p;
+      double s = 0.0, r = 0.0;
+      for (int j = lane; j < p; j += 32) {
+        const double v = value(x[j]);
+        s += v * y[c * p + j];
+        r += v * value(xc[j]);
+      }
+      s = warp_sum(s);
+      r = (i == lead[c] ? 1.0 : 0.0) - warp_sum(r);
+      const double gap = lambda[lead[c]] - lambda[i];
+      if (lane == 0)
+        s_e[c][i] = fabs(gap) > 1e-12 * fabs(lambda[lead[0]]) ? (s + lambda[lead[c]] * r) / gap : 0.5 * r;
     }
+    __syncthreads();
+    if (at < p)
+      for (int j = warp; j < p; j += kWarps) {
+        const double v = value(X[(long long)j * p + at]);
+        t[0] += s_e[0][j] * v;
+        t[1] += s_e[1][j] * v;
+      }
+  }
   s_sum[warp][0][lane] = t[0];
   s_sum[warp][1][lane] = t[1];
   __syncthreads();
-  if (warp >= 2 || i >= p) return;
+  if (warp >= 2 || at >= p) return;
   double sum = 0.0;
-  for (int w = 0; w < 8; ++w) sum += s_sum[w][warp][lane];
-  vectors[warp * p + i] = split(value(X[(long long)info[warp] * p + i]) + sum);
+  for (int w = 0; w < kWarps; ++w) sum += s_sum[w][warp][lane];
+  vectors[warp * p + at] = split(value(X[(long long)lead[warp] * p + at]) + sum);
 }
 
 struct ArgMax {
@@ -531,34 +527,31 @@ pca_scores_kernel(const float* __restrict__ X, const float* __restrict__ mean, c
   }
 }
 
-// Signs from the largest-magnitude scores (one block; s_sign: two doubles).
-__global__ void pca_sign_kernel(const double2* __restrict__ sc, const ArgMax* __restrict__ part, int nparts,
-                                double* __restrict__ sign) {
-  const int c = threadIdx.x >> 5, lane = threadIdx.x & 31;  // a warp per component
-  ArgMax best{-1.0, 0};
-  for (int b = lane; b < nparts; b += 32) {
-    const ArgMax q = part[b * 2 + c];
-    if (q.v > best.v || (q.v == best.v && q.i < best.i)) best = q;
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    const double v = __shfl_xor_sync(0xffffffffu, best.v, o);
-    const long long i = __shfl_xor_sync(0xffffffffu, best.i, o);
-    if (v > best.v || (v == best.v && i < best.i)) best = ArgMax{v, i};
-  }
-  if (lane == 0) {
-    const double v = c == 0 ? sc[best.i].x : sc[best.i].y;
-    sign[c] = v < 0.0 ? -1.0 : 1.0;
-  }
-}
-
-// Signed float scores (non-finite -> 0) and the blocks' partial moments (sums of x, y, x^2, y^2 of the
+// Signed float scores (each component's largest in magnitude positive; non-finite -> 0) and the blocks' partial moments (sums of x, y, x^2, y^2 of the
 // scores over the data's power of two). One block of FP64 sums and the scaling took 1144 us for 200,000
-// rows; the three kernels take 29 us.
+// rows; the two kernels take 26 us.
 __global__ void __launch_bounds__(256)
 pca_moments_kernel(const double2* __restrict__ sc, const int* __restrict__ status, int n,
-                   const double* __restrict__ sign, float2* __restrict__ init, double* __restrict__ part) {
+                   const ArgMax* __restrict__ largest, int nlargest, float2* __restrict__ init,
+                   double* __restrict__ part) {
   __shared__ Float2Sum s_red[4][8];
-  const float sx = (float)sign[0], sy = (float)sign[1];
+  __shared__ float s_sign[2];
+  if (threadIdx.x < 64) {  // a warp per component
+    const int c = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    ArgMax best{-1.0, 0};
+    for (int b = lane; b < nlargest; b += 32) {
+      const ArgMax q = largest[b * 2 + c];
+      if (q.v > best.v || (q.v == best.v && q.i < best.i)) best = q;
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+      const double v = __shfl_xor_sync(0xffffffffu, best.v, o);
+      const long long i = __shfl_xor_sync(0xffffffffu, best.i, o);
+      if (v > best.v || (v == best.v && i < best.i)) best = ArgMax{v, i};
+    }
+    if (lane == 0) s_sign[c] = (c == 0 ? sc[best.i].x : sc[best.i].y) < 0.0 ? -1.0f : 1.0f;
+  }
+  __syncthreads();
+  const float sx = s_sign[0], sy = s_sign[1];
   const float unit = scalbnf(1.0f, -data_exponent(status[1]));
   Float2Sum m[4];
 #pragma unroll
@@ -634,8 +627,8 @@ void pca_tsne_start(const float* X, int n, int p, float2* init, cudaStream_t s) 
   const int mslices = std::max(1, std::min(kMeanSlices, ceil_div(n, 1024)));
   const std::size_t m = p + (p & 1);
   const bool shared = p <= kJacobiSharedFeatures;
-  double *sums = nullptr, *partial = nullptr, *C = nullptr, *sign = nullptr, *moments = nullptr;
-  double *lambda = nullptr, *y = nullptr, *e = nullptr;
+  double *sums = nullptr, *partial = nullptr, *C = nullptr, *moments = nullptr;
+  double *lambda = nullptr, *y = nullptr;
   float *mean = nullptr, *tangents = nullptr;
   float2* range = nullptr;
   Float2Sum *work = nullptr, *all = nullptr, *V = nullptr;
@@ -655,12 +648,10 @@ void pca_tsne_start(const float* X, int n, int p, float2* init, cudaStream_t s) 
   w.reserve(&info, 4);
   w.reserve(&all, (std::size_t)p * p);
   w.reserve(&y, 2 * (std::size_t)p);
-  w.reserve(&e, 2 * (std::size_t)p);
   w.reserve(&V, 2 * (std::size_t)p);
   w.reserve(&sc, n);
   w.reserve(&am, 2 * (std::size_t)sblocks);
   w.reserve(&status, 2);
-  w.reserve(&sign, 2);
   w.reserve(&moments, 4 * (std::size_t)mblocks);
   w.commit("device PCA initialization");
   FE_CUDA(cudaMemsetAsync(status, 0, 2 * sizeof(int), s));
@@ -679,25 +670,19 @@ void pca_tsne_start(const float* X, int n, int p, float2* init, cudaStream_t s) 
   FE_LAUNCH("pca_gram_sum_kernel");
   if (shared) {
     const int smem = (int)(m * m * sizeof(Float2Sum));
-    allow_dynamic_shared((const void*)pca_jacobi_kernel<true>);
+    if (smem > 16 * 1024) allow_dynamic_shared((const void*)pca_jacobi_kernel<true>);  // beside its static 24 KB
     pca_jacobi_kernel<true><<<1, kJacobiThreads, smem, s>>>(C, p, work, tangents, lambda, info);
   } else {
     pca_jacobi_kernel<false><<<1, kJacobiThreads, 0, s>>>(C, p, work, tangents, lambda, info);
   }
   FE_LAUNCH("pca_jacobi_kernel");
-  pca_vectors_kernel<<<ceil_div(p, 2), kJacobiThreads, 0, s>>>(tangents, p, info, all);
+  pca_vectors_kernel<<<ceil_div(p, 2), kJacobiThreads, 0, s>>>(tangents, p, info, C, all, y);
   FE_LAUNCH("pca_vectors_kernel");
-  pca_product_kernel<<<ceil_div(p, 8), 256, 0, s>>>(C, all, p, info, y);
-  FE_LAUNCH("pca_product_kernel");
-  pca_correction_kernel<<<ceil_div(p, 8), 256, 0, s>>>(all, y, p, lambda, info, e);
-  FE_LAUNCH("pca_correction_kernel");
-  pca_refine_kernel<<<ceil_div(p, 32), 256, 0, s>>>(all, e, p, info, V);
+  pca_refine_kernel<<<ceil_div(p, 32), kJacobiThreads, 0, s>>>(all, y, p, lambda, info, V);
   FE_LAUNCH("pca_refine_kernel");
   pca_scores_kernel<<<sblocks, 256, 0, s>>>(X, mean, status, n, p, V, sc, am);
   FE_LAUNCH("pca_scores_kernel");
-  pca_sign_kernel<<<1, 64, 0, s>>>(sc, am, sblocks, sign);
-  FE_LAUNCH("pca_sign_kernel");
-  pca_moments_kernel<<<mblocks, 256, 0, s>>>(sc, status, n, sign, init, moments);
+  pca_moments_kernel<<<mblocks, 256, 0, s>>>(sc, status, n, am, sblocks, init, moments);
   FE_LAUNCH("pca_moments_kernel");
   pca_scale_kernel<<<mblocks, 256, 0, s>>>(init, status, n, moments, mblocks);
   FE_LAUNCH("pca_scale_kernel");
