@@ -670,7 +670,7 @@ void pca_tsne_start(const float* X, int n, int p, float2* init, cudaStream_t s) 
   FE_LAUNCH("pca_gram_sum_kernel");
   if (shared) {
     const int smem = (int)(m * m * sizeof(Float2Sum));
-    if (smem > 16 * 1024) allow_dynamic_shared((const void*)pca_jacobi_kernel<true>);  // beside its static 24 KB
+    allow_dynamic_shared((const void*)pca_jacobi_kernel<true>, smem);
     pca_jacobi_kernel<true><<<1, kJacobiThreads, smem, s>>>(C, p, work, tangents, lambda, info);
   } else {
     pca_jacobi_kernel<false><<<1, kJacobiThreads, 0, s>>>(C, p, work, tangents, lambda, info);
