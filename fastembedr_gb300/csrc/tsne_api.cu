@@ -178,7 +178,7 @@ struct TsneJob {
       row_probabilities(d_idx, d_dist, n, k, perplexity, d_p, nullptr, s);
       symmetrise(d_idx, d_p, n, k, offset, P, s);
     }
-    tsne_device_alloc(D, n, grid, mode);
+    tsne_device_alloc(D, n, grid, mode, s);
     reorder = reorder_enabled();
     float2* d_init = nullptr;
     Arena tmp;
@@ -242,7 +242,7 @@ struct TsneJob {
       lr[t] = (float)sz[t];
       max_n = std::max(max_n, sz[t]);
     }
-    tsne_batch_alloc(D, sz, gr, lr, mode);
+    tsne_batch_alloc(D, sz, gr, lr, mode, s);
     const int n = D.n;
     std::vector<int> first(ninst + 1, 0);
     for (int t = 0; t < ninst; ++t) first[t + 1] = first[t] + sz[t];

@@ -935,14 +935,15 @@ TsneDevice::~TsneDevice() {
 
 int default_grid_size(int n, int /*mode*/) { return cuda_fft_grid_size(n); }
 
-void tsne_device_alloc(TsneDevice& d, int n, int grid, int mode) {
-  tsne_batch_alloc(d, std::vector<int>{n}, std::vector<int>{grid}, std::vector<float>{1.0f}, mode);
+void tsne_device_alloc(TsneDevice& d, int n, int grid, int mode, cudaStream_t s) {
+  tsne_batch_alloc(d, std::vector<int>{n}, std::vector<int>{grid}, std::vector<float>{1.0f}, mode, s);
 }
 
 namespace {
 // Group instances by grid size, allocate the class workspaces in d.grid_arena and point the
-// instance table at them (host copy; the caller uploads it).
-void build_grid_classes(TsneDevice& d, const std::vector<int>& grids) {
+// instance table at them (host copy; the caller uploads it). The set-up runs on s and waits for s alone: waiting for the
+// device, or on the legacy stream, while another thread captures its graph is not allowed (the driver crashed there).
+void build_grid_classes(TsneDevice& d, const std::vector<int>& grids, cudaStream_t s) {
   const int ninst = (int)d.inst.size();
   std::vector<int> distinct(grids.begin(), grids.end());
   std::sort(distinct.begin(), distinct.end());
@@ -978,6 +979,7 @@ void build_grid_classes(TsneDevice& d, const std::vector<int>& grids) {
   }
   d.grid_arena.commit("t-SNE grid workspaces");
   std::vector<int> flat;
+  std::vector<std::vector<float2>> tables(distinct.size());
   int max_grid = 0;
   for (std::size_t c = 0; c < distinct.size(); ++c) {
     GridClass& k = d.classes[c];
@@ -992,22 +994,23 @@ void build_grid_classes(TsneDevice& d, const std::vector<int>& grids) {
       I.charges = k.charges + (std::size_t)j * k.grid * k.grid * kChargeStride;
       I.potential = k.potential + (std::size_t)j * k.grid * k.grid;
     }
-    const std::vector<float2> tw = fft_class_twiddles(k);
-    FE_CUDA(cudaMemcpy(k.twiddle, tw.data(), sizeof(float2) * tw.size(), cudaMemcpyHostToDevice));
-    FE_CUDA(cudaMemset(k.charges, 0, sizeof(long long) * kChargeStride * (std::size_t)k.count * k.grid * k.grid));
-    FE_CUDA(cudaMemset(k.potential, 0, sizeof(float4) * (std::size_t)k.count * k.grid * k.grid));
+    const std::vector<float2>& tw = tables[c] = fft_class_twiddles(k);
+    FE_CUDA(cudaMemcpyAsync(k.twiddle, tw.data(), sizeof(float2) * tw.size(), cudaMemcpyHostToDevice, s));
+    FE_CUDA(cudaMemsetAsync(k.charges, 0, sizeof(long long) * kChargeStride * (std::size_t)k.count * k.grid * k.grid, s));
+    FE_CUDA(cudaMemsetAsync(k.potential, 0, sizeof(float4) * (std::size_t)k.count * k.grid * k.grid, s));
   }
-  FE_CUDA(cudaMemcpy(d_members, flat.data(), sizeof(int) * ninst, cudaMemcpyHostToDevice));
+  FE_CUDA(cudaMemcpyAsync(d_members, flat.data(), sizeof(int) * ninst, cudaMemcpyHostToDevice, s));
   d.grid = d.inst[0].grid;
   d.nodes = d.inst[0].nodes;
   d.key_bits = 2 * log2_ceil(max_grid);
   d.sort_bits = d.key_bits + log2_ceil(ninst);
   if (d.sort_bits > 32) throw Error("t-SNE batch: too many instances for the spatial sort key");
+  FE_CUDA(cudaStreamSynchronize(s));  // the tables go out of scope
 }
 }  // namespace
 
 void tsne_batch_alloc(TsneDevice& d, const std::vector<int>& sizes, const std::vector<int>& grids,
-                      const std::vector<float>& lr_mult, int mode) {
+                      const std::vector<float>& lr_mult, int mode, cudaStream_t s) {
   const int ninst = (int)sizes.size();
   if (ninst < 1 || grids.size() != sizes.size() || lr_mult.size() != sizes.size())
     throw Error("t-SNE batch: one size, grid and learning-rate multiplier per instance");
@@ -1065,30 +1068,27 @@ void tsne_batch_alloc(TsneDevice& d, const std::vector<int>& sizes, const std::v
   d.arena.reserve(&d.radix.scan_tmp, ceil_div(256LL * nb, 1024));
   d.arena.commit("t-SNE optimizer state");
   d.reordered = false;
-  build_grid_classes(d, grids);
+  build_grid_classes(d, grids, s);
   std::vector<int2> blk(nblocks);
   for (int b = 0; b < ninst; ++b)
     for (int t = 0; t < d.inst[b].blocks; ++t)
       blk[d.inst[b].block_begin + t] = make_int2(b, d.inst[b].pt_begin + t * kPointBlock);
-  FE_CUDA(cudaMemcpy(d.d_inst, d.inst.data(), sizeof(TsneInstance) * ninst, cudaMemcpyHostToDevice));
-  FE_CUDA(cudaMemcpy(d.blocks, blk.data(), sizeof(int2) * nblocks, cudaMemcpyHostToDevice));
-  FE_CUDA(cudaMemset(d.counter, 0, sizeof(unsigned) * ninst));
-  FE_CUDA(cudaMemset(d.attr_ctr, 0, sizeof(unsigned) * (1 + (std::size_t)d.attr_queues) * kAttrCtrStride));
-  FE_CUDA(cudaMemset(d.cur, 0, sizeof(GridState) * ninst));
+  FE_CUDA(cudaMemcpyAsync(d.d_inst, d.inst.data(), sizeof(TsneInstance) * ninst, cudaMemcpyHostToDevice, s));
+  FE_CUDA(cudaMemcpyAsync(d.blocks, blk.data(), sizeof(int2) * nblocks, cudaMemcpyHostToDevice, s));
+  FE_CUDA(cudaMemsetAsync(d.counter, 0, sizeof(unsigned) * ninst, s));
+  FE_CUDA(cudaMemsetAsync(d.attr_ctr, 0, sizeof(unsigned) * (1 + (std::size_t)d.attr_queues) * kAttrCtrStride, s));
+  FE_CUDA(cudaMemsetAsync(d.cur, 0, sizeof(GridState) * ninst, s));
   if (!d.side) FE_CUDA(cudaStreamCreateWithFlags(&d.side, cudaStreamNonBlocking));
   if (!d.fork) FE_CUDA(cudaEventCreateWithFlags(&d.fork, cudaEventDisableTiming));
   if (!d.join) FE_CUDA(cudaEventCreateWithFlags(&d.join, cudaEventDisableTiming));
-  // the synchronous setup above ran on the legacy stream, which the job's non-blocking streams
-  // do not wait for
-  FE_CUDA(cudaDeviceSynchronize());
+  FE_CUDA(cudaStreamSynchronize(s));  // blk goes out of scope
 }
 
 void tsne_regrid(TsneDevice& d, const std::vector<int>& grids, cudaStream_t s) {
   if (grids.size() != d.inst.size()) throw Error("t-SNE regrid: one grid size per instance");
   FE_CUDA(cudaStreamSynchronize(s));
-  build_grid_classes(d, grids);
-  FE_CUDA(cudaMemcpy(d.d_inst, d.inst.data(), sizeof(TsneInstance) * d.inst.size(), cudaMemcpyHostToDevice));
-  FE_CUDA(cudaDeviceSynchronize());
+  build_grid_classes(d, grids, s);
+  FE_CUDA(cudaMemcpyAsync(d.d_inst, d.inst.data(), sizeof(TsneInstance) * d.inst.size(), cudaMemcpyHostToDevice, s));
   // `next` of every instance was laid out for its old grid: recompute it from the layout
   layout_stats_kernel<<<d.nblocks, kStepThreads, 0, s>>>(d.y, d.d_inst, d.blocks, d.mode, d.partial, d.counter,
                                                           d.next);

@@ -134,11 +134,11 @@ struct TsneDevice {
 // Nodes per side used for a given size (the reference CUDA policy for either stencil).
 int default_grid_size(int n, int mode);
 
-void tsne_device_alloc(TsneDevice& d, int n, int grid, int mode);
+void tsne_device_alloc(TsneDevice& d, int n, int grid, int mode, cudaStream_t s);
 // Batch of instances: sizes[b] points on a grids[b] x grids[b] grid, learning rate multipliers
 // lr_mult[b].
 void tsne_batch_alloc(TsneDevice& d, const std::vector<int>& sizes, const std::vector<int>& grids,
-                      const std::vector<float>& lr_mult, int mode);
+                      const std::vector<float>& lr_mult, int mode, cudaStream_t s);
 // Change the instances' grid sizes: rebuild the grid classes and their workspaces, then
 // recompute every instance's next grid from the current layout (stream-ordered on s).
 void tsne_regrid(TsneDevice& d, const std::vector<int>& grids, cudaStream_t s);

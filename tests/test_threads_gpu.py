@@ -1,6 +1,6 @@
-"""Calls of different sizes on several threads: a kernel's limit of dynamic shared memory belongs to the process, so one
-thread's launch must not depend on the size of another's. Every call's result is compared with its result alone, bit
-for bit."""
+"""Calls of different sizes on several threads. A kernel's limit of dynamic shared memory belongs to the process, so one
+thread's launch must not depend on the size of another's; and no thread may wait for the device, or on the legacy stream,
+while another captures its iterations in a graph. Every call's result is compared with its result alone, bit for bit."""
 import threading
 
 import numpy as np
@@ -39,9 +39,19 @@ def _graph(k):
     return lambda: api.umap_graph(idx, dist, index_offset=0)["weights"]
 
 
+def _tsne(n):
+    k = 15
+    idx = ((np.arange(n)[:, None] + 1 + np.arange(k)) % n).astype(np.int32)
+    rng = np.random.default_rng(n)
+    dist = np.sort(rng.uniform(0.2, 3.0, (n, k)), 1).astype(np.float32)
+    init = rng.normal(size=(n, 2)).astype(np.float32)
+    return lambda: api.tsne_knn(idx, dist, perplexity=5.0, n_iter=5, early_exaggeration_iter=5, Y_init=init).layout
+
+
 @pytest.mark.parametrize("make,large,small,reps", [(_spectral, 300000, (40, 100, 300, 900), 60), (_pca, 120, (3, 5, 9, 17), 120),
                                                    (_affinities, 100, (50, 55, 60, 70), 400),
-                                                   (_graph, 100, (50, 55, 60, 70), 400)])
+                                                   (_graph, 100, (50, 55, 60, 70), 400),
+                                                   (_tsne, 30000, (100, 300, 900, 2000), 60)])
 def test_sizes_side_by_side(make, large, small, reps):
     faults, stop = [], threading.Event()
 
