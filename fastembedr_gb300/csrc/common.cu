@@ -135,14 +135,9 @@ int sm_count() {
   return sms;
 }
 
-void allow_dynamic_shared(const void* kernel, std::size_t bytes) {
-  cudaFuncAttributes a{};
-  FE_CUDA(cudaFuncGetAttributes(&a, kernel));
-  if (bytes + a.sharedSizeBytes <= 48 * 1024) return;
-  int dev = 0, most = 0;
-  FE_CUDA(cudaGetDevice(&dev));
-  FE_CUDA(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-  FE_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)a.sharedSizeBytes));
+void allow_dynamic_shared(const void* kernel, std::size_t bytes, std::size_t most) {
+  if (bytes <= 16 * 1024) return;
+  FE_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
 }
 
 }  // namespace fe

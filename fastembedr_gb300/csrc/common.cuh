@@ -96,10 +96,11 @@ inline int ceil_div(long long a, long long b) { return static_cast<int>((a + b -
 // writes to those buffers are complete.
 void order_after_legacy_stream(cudaStream_t s);
 int sm_count();
-// Lets `kernel` be launched with `bytes` of dynamic shared memory: beyond 48 KB in all, its static share included, a
-// kernel has to be allowed more. It is then allowed all that its static share leaves: the limit is a state of the whole
-// process, and set to what one call needs, a smaller call on another thread would lower it before the larger one's launch.
-void allow_dynamic_shared(const void* kernel, std::size_t bytes);
+// Lets `kernel` be launched with `bytes` of dynamic shared memory. Beyond 48 KB in all, its static share included (up to
+// 25 KB here), a kernel has to be allowed more; it is then allowed `most`, the most that any call uses: the limit is a state
+// of the whole process, and set to what one call needs, a smaller call on another thread would lower it before the larger
+// one's launch.
+void allow_dynamic_shared(const void* kernel, std::size_t bytes, std::size_t most);
 
 // ---------------------------------------------------------------- host uploads
 // Host -> device copy of caller memory (pageable or not), ordered on stream s. Copies of at

@@ -670,7 +670,8 @@ void pca_tsne_start(const float* X, int n, int p, float2* init, cudaStream_t s) 
   FE_LAUNCH("pca_gram_sum_kernel");
   if (shared) {
     const int smem = (int)(m * m * sizeof(Float2Sum));
-    allow_dynamic_shared((const void*)pca_jacobi_kernel<true>, smem);
+    allow_dynamic_shared((const void*)pca_jacobi_kernel<true>, smem,
+                         kJacobiSharedFeatures * kJacobiSharedFeatures * sizeof(Float2Sum));
     pca_jacobi_kernel<true><<<1, kJacobiThreads, smem, s>>>(C, p, work, tangents, lambda, info);
   } else {
     pca_jacobi_kernel<false><<<1, kJacobiThreads, 0, s>>>(C, p, work, tangents, lambda, info);

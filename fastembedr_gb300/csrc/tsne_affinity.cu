@@ -321,7 +321,7 @@ void row_probabilities(const int* /*d_idx*/, const float* d_dist, int n, int k, 
   int rows = kBisectRows;
   while (rows > 1 && (std::size_t)rows * (k + 1) * 2 * sizeof(float) > 112 * 1024) rows >>= 1;
   const std::size_t smem = (std::size_t)rows * (k + 1) * 2 * sizeof(float);
-  allow_dynamic_shared((const void*)row_probabilities_kernel, smem);
+  allow_dynamic_shared((const void*)row_probabilities_kernel, smem, 224 * 1024);
   row_probabilities_kernel<<<ceil_div(n, rows), rows, smem, s>>>(d_dist, n, k, std::log((double)perplexity), d_p,
                                                                  d_entropy);
   FE_LAUNCH("row_probabilities_kernel");

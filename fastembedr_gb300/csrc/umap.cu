@@ -233,7 +233,7 @@ void smooth_knn(const float* d_dist, int n, int k, const double* acc, float* sig
   while (rows > 1 && (std::size_t)rows * (k + 1) * 2 * sizeof(float) > 96 * 1024) rows >>= 1;
   const std::size_t smem = (std::size_t)rows * (k + 1) * 2 * sizeof(float);
   if (smem > 200 * 1024) throw Error("k is too large for the UMAP smooth-kNN search (at most 25,000 neighbours)");
-  allow_dynamic_shared((const void*)umap_smooth_knn_kernel, smem);
+  allow_dynamic_shared((const void*)umap_smooth_knn_kernel, smem, 200 * 1024);
   umap_smooth_knn_kernel<<<ceil_div(n, rows), rows, smem, s>>>(d_dist, n, k, std::log2((double)k), acc, sig, rho);
   FE_LAUNCH("umap_smooth_knn_kernel");
 }

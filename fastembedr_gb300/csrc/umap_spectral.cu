@@ -995,7 +995,7 @@ void umap_spectral_start(const int* offsets, const int* neighbors, const float* 
     const bool shared = (long long)tiles * points <= kSpSharedRows;
     const int smem = shared ? kSpBlock * tiles * points * (int)sizeof(double) : 0;
     const void* rounds = shared ? (const void*)sp_rounds_kernel<true> : (const void*)sp_rounds_kernel<false>;
-    allow_dynamic_shared(rounds, smem);
+    allow_dynamic_shared(rounds, smem, kSpBlock * kSpSharedRows * sizeof(double));
     int per_sm = 0;
     FE_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, rounds, kSpRoundThreads, smem));
     if (per_sm * sm_count() < parts) throw Error("the spectral start's subspace iteration cannot be made resident");
